@@ -49,7 +49,9 @@ enum { O1D_NCHW = 0, O1D_NHWC = 1 };
 /* Bits of the `add_identity` / `flags` argument of the operators. */
 enum {
     O1D_FLAG_IDENTITY = 1,    /* w' = w + (k == pad): the reference's `resid`                     */
-    O1D_FLAG_GELU_INPUT = 2   /* the input tensor is a pre-activation: exact GELU is applied as it is loaded */
+    O1D_FLAG_GELU_INPUT = 2,  /* the input tensor is a pre-activation: exact GELU is applied as it is loaded */
+    O1D_FLAG_PARAMS_BF16 = 4  /* w and bias (o1d_wgrad_act: dw and db) are bf16, not fp32; requests whose kernels
+                                 read fp32 parameters only are refused with O1D_ERR_UNSUPPORTED               */
 };
 enum { O1D_F32 = 0, O1D_BF16 = 1 };
 
@@ -77,7 +79,8 @@ enum {
     O1D_ROUTE_NONE = -1,
     O1D_ROUTE_GENERAL = 0,   /* gather kernels: any stride, layout, angle                      */
     O1D_ROUTE_TILED = 1,     /* restaged channel planes with register windows                  */
-    O1D_ROUTE_DIRECT = 2,    /* TMA halo tiles, one tap list per thread                        */
+    O1D_ROUTE_DIRECT = 2,    /* NHWC tiles as TMA brings them: one tap list per thread, or packed
+                                segments of a line per channel pair                            */
     O1D_ROUTE_PLANE7 = 3,    /* 7x7 maps, one channel plane per thread                         */
     O1D_ROUTE_LINES = 4,     /* whole lines per thread (round-robin angle assignment)          */
     O1D_ROUTE_WALK = 5       /* items computed in place in their NHWC layout (square fp32 maps) */

@@ -1,0 +1,266 @@
+// Segment kernels: configuration and launches (see o1d_seg.cuh).
+#include <string.h>
+
+#include <memory>
+#include <vector>
+
+#include "o1d_seg.cuh"
+
+namespace o1d {
+
+namespace {
+
+int round_up(int v, int m) { return (v + m - 1) / m * m; }
+
+// Lines of one chunk: pairs of channels per canonical line, and the reach that a tile needs.
+struct Chunk {
+    int pairs[8];
+    int reach_h, reach_w;
+};
+Chunk chunk_of(const int8_t *chan, int c0, int c1, int K) {
+    Chunk k{};
+    for (int c = c0; c < c1; c += 2) {
+        k.pairs[chan[c]]++;
+        if (c + 1 < c1 && chan[c + 1] != chan[c]) k.pairs[chan[c + 1]]++;
+    }
+    for (int o = 0; o < 8; o++)
+        if (k.pairs[o]) {
+            // the bodies run all taps of their reach, missing ones with weight zero
+            const int rh = kCanonDh[o][kHalf - (K <= 15 ? 7 : 15)], rw = kCanonDw[o][kHalf - (K <= 15 ? 7 : 15)];
+            if (abs(rh) > k.reach_h) k.reach_h = abs(rh);
+            if (abs(rw) > k.reach_w) k.reach_w = abs(rw);
+        }
+    return k;
+}
+
+// Cycles of one task on a scheduler with three warps (measured at 56x56x96, batch 128).
+constexpr double kAxis28 = 3600, kAxis14 = 1950, kSlantTask = 4600, kDiagTask = 2050;
+constexpr double kPieceCycles = 2.4;         // TMA, per pixel of a tile
+
+double compute_cycles(const Chunk &k, int imgs, int lenh, int lenw, int LT) {
+    double sum = 0;
+    for (int o = 0; o < 8; o++) {
+        const int n = k.pairs[o], per = n ? seg::class_pairs(n) : 1, split = ceil_div(n, per);
+        if (!n) continue;
+        const int lpg = 32 / per, fr = seg::frame_of(o), kind = seg::kind_of(o);
+        const int plen = fr == seg::FR_H ? lenw : lenh, llen = fr == seg::FR_H ? lenh : lenw;
+        const int lines = kind == KIND_AXIS ? llen : kind == KIND_DIAG ? lenw + seg::kTD - 1 : ceil_div(llen, seg::kSR);
+        const int bl = kind == KIND_SLANT ? seg::kST : kind == KIND_AXIS ? LT : seg::kTD;
+        const double cyc = kind == KIND_SLANT ? kSlantTask : kind == KIND_DIAG ? kDiagTask : LT == 28 ? kAxis28 : kAxis14;
+        sum += split * (double)ceil_div(imgs * lines, lpg) * ceil_div(plen, bl) * cyc;
+    }
+    return sum / 4;                          // schedulers
+}
+
+// Best way to cut the maps for these lines.  Whole maps need no halo (a border of one pixel of zeros is
+// enough); maps that do not fit twice are cut along the axis the lines reach least.
+bool choose_geo(const Chunk &k, const SegParams &p, int room, int LT, SegGeo *out, double *cycles) {
+    double best = 0;
+    for (int nth = 1; nth <= 64; nth++) {
+        const int TH = ceil_div(p.H, nth);
+        if (nth > 1 && (TH < 6 || ceil_div(p.H, TH) != nth)) continue;
+        for (int ntw = 1; ntw <= 64; ntw++) {
+            const int TW = ceil_div(p.W, ntw);
+            if (ntw > 1 && (TW < 6 || ceil_div(p.W, TW) != ntw)) continue;
+            SegGeo g{};
+            g.nth = nth; g.ntw = ntw; g.TH = TH; g.TW = TW;
+            g.halo_h = nth > 1; g.halo_w = ntw > 1;
+            g.oh = g.halo_h ? k.reach_h : 1;
+            g.ow = g.halo_w ? k.reach_w : 0;
+            g.RT = g.halo_h ? TH + 2 * k.reach_h : TH + 2;
+            g.P = (g.halo_w ? TW + 2 * k.reach_w : TW + 1) | 1;
+            if (g.P > 256 || g.RT > 256) continue;
+            g.plo_h = g.halo_h ? -g.oh : -1;
+            g.phi_h = g.halo_h ? g.RT - g.oh - 1 : TH;
+            g.plo_w = g.halo_w ? -g.ow : -1;
+            g.phi_w = g.halo_w ? g.P - g.ow - 1 : TW;
+            g.img_bytes = g.RT * g.P * p.px;
+            if (round_up(g.img_bytes + p.px, 128) > room) continue;
+            g.G = 1;
+            if (nth * ntw == 1)              // small maps: enough lines to fill the lanes of twelve warps
+                while (g.G < 64 && g.G < p.N && g.G * p.H * p.W < 1024 && 2 * round_up((g.G + 1) * g.img_bytes + p.px, 128) <= room) g.G++;
+            g.tile_bytes = g.G * g.img_bytes;
+            g.buf_bytes = round_up(g.tile_bytes + p.px, 128);     // ends in a pixel of zeros
+            g.nbuf = room / g.buf_bytes;
+            if (g.nbuf > seg::kMaxBuf) g.nbuf = seg::kMaxBuf;
+            g.items = ceil_div(p.N, g.G) * nth * ntw;
+            const double load = kPieceCycles * g.G * g.RT * g.P * (p.px == 64 ? 1.5 : p.px == 48 ? 1.25 : 1.0);
+            const double comp = compute_cycles(k, g.G, TH, TW, LT);
+            // one buffer: every load is exposed
+            const double cyc = (g.nbuf == 1 ? comp + load : comp > load ? comp : load) + 300;
+            if (best == 0 || cyc * g.items < best) { best = cyc * g.items; *out = g; *cycles = cyc; }
+        }
+        if (best != 0 && nth > 4 && TH < 16) break;
+    }
+    return best != 0;
+}
+
+bool same_geo(const SegGeo &a, const SegGeo &b) { return memcmp(&a, &b, sizeof(SegGeo)) == 0; }
+
+// Plan for chunks of `px` bytes and line blocks of LT outputs; the estimated time in *cycles.
+bool plan_chunks(const int8_t *chan, SegParams &p, int px, int esize, int LT, int room, int *ngeos, double *cycles) {
+    p.px = px;
+    p.CC = px / esize;
+    p.nruns = 0;
+    const int nch = ceil_div(p.C, p.CC);
+    int geos = 0;
+    double total = 0;
+    Chunk prev{};
+    std::vector<double> cyc;
+    for (int i = 0; i < nch; i++) {
+        const int c0 = i * p.CC, c1 = c0 + p.CC < p.C ? c0 + p.CC : p.C;
+        const Chunk k = chunk_of(chan, c0, c1, p.K);
+        if (p.nruns && memcmp(&k, &prev, sizeof(k)) == 0) {
+            p.run[p.nruns - 1].nchunks++;
+        } else {
+            if (p.nruns == kSegRuns) return false;
+            SegGeo g;
+            double c;
+            if (!choose_geo(k, p, room, LT, &g, &c)) return false;
+            int at = 0;
+            while (at < geos && !same_geo(p.geo[at], g)) at++;
+            if (at == geos) {
+                if (geos == kSegGeos) return false;
+                p.geo[geos++] = g;
+            }
+            p.run[p.nruns++] = SegRun{i, 1, at, 0, 0};
+            cyc.push_back(c);
+            prev = k;
+        }
+        total += cyc.back() * p.geo[p.run[p.nruns - 1].geo].items;
+    }
+    p.total_cost = 0;
+    for (int r = 0; r < p.nruns; r++) {
+        p.run[r].cost = (int)(cyc[r] / 16) + 1;
+        p.total_cost += (long long)p.run[r].cost * p.geo[p.run[r].geo].items * seg::kParts * p.run[r].nchunks;
+    }
+    *ngeos = geos;
+    *cycles = total;
+    return true;
+}
+
+bool make_config(const int8_t *chan, int N, int H, int W, int C, int K, int esize, int smem_optin, int sms, bool wgrad, SegConfig *cfg) {
+    if (C % 8 != 0 || K > kMaxTaps) return false;
+    // pairs of channels on different lines are computed twice and stored by halves
+    int mixed = 0;
+    for (int c = 0; c + 1 < C; c += 2) mixed += chan[c] != chan[c + 1];
+    if (mixed * 8 > C) return false;
+    const int tail = round_up((int)sizeof(seg::Tables), 16) + 12 * seg::kMaxBuf + 128;
+    const int room = smem_optin - round_up(seg::kPadBytes, 128) - tail;
+    double best = 0;
+    for (int px = 32; px <= 64; px += 16)
+        for (int LT = 14; LT <= 28; LT += 14) {
+            SegConfig t{};
+            t.p.N = N; t.p.H = H; t.p.W = W; t.p.C = C; t.p.K = K;
+            double cyc;
+            if (!plan_chunks(chan, t.p, px, esize, LT, room, &t.ngeos, &cyc)) continue;
+            if (best == 0 || cyc < best) { best = cyc; t.line_block = LT; *cfg = t; }
+        }
+    if (best == 0) return false;
+    SegParams &p = cfg->p;
+    int bytes = 0;
+    long long items = 0;
+    for (int i = 0; i < cfg->ngeos; i++)
+        if (p.geo[i].nbuf * p.geo[i].buf_bytes > bytes) bytes = p.geo[i].nbuf * p.geo[i].buf_bytes;
+    for (int r = 0; r < p.nruns; r++) items += (long long)p.run[r].nchunks * p.geo[p.run[r].geo].items;
+    p.off_tile = round_up(seg::kPadBytes, 128);
+    p.off_tab = p.off_tile + bytes;
+    p.off_bar = p.off_tab + round_up((int)sizeof(seg::Tables), 16);
+    cfg->esize = esize;
+    cfg->short_reach = K <= 15;
+    cfg->smem_bytes = p.off_bar + 12 * seg::kMaxBuf;
+    cfg->grid = items * 4 < sms ? (int)items * 4 : sms;          // no CTA with less than a quarter item
+    // CTAs per chunk in proportion to cost, where that comes out even enough
+    const int nch = ceil_div(C, p.CC);
+    p.per_chunk = nch * 3 <= cfg->grid;
+    if (p.per_chunk) {
+        int left = cfg->grid;
+        double worst = 0;
+        auto load = [&](int r) { return (double)p.run[r].cost * p.geo[p.run[r].geo].items; };
+        for (int r = 0; r < p.nruns; r++) {
+            p.run[r].ctas = (int)(load(r) * seg::kParts * cfg->grid / p.total_cost);
+            if (p.run[r].ctas < 1) p.run[r].ctas = 1;
+            left -= p.run[r].ctas * p.run[r].nchunks;
+        }
+        while (left > 0) {               // the rest to the slowest runs
+            int at = -1;
+            for (int r = 0; r < p.nruns; r++)
+                if (p.run[r].nchunks <= left && (at < 0 || load(r) / p.run[r].ctas > load(at) / p.run[at].ctas)) at = r;
+            if (at < 0) break;
+            p.run[at].ctas++;
+            left -= p.run[at].nchunks;
+        }
+        for (int r = 0; r < p.nruns; r++)
+            if (load(r) / p.run[r].ctas > worst) worst = load(r) / p.run[r].ctas;
+        const double even = (double)p.total_cost / seg::kParts / cfg->grid;
+        if (left < 0 || worst > 1.3 * even) p.per_chunk = 0;
+        else cfg->grid -= left;
+    }
+    return cfg->smem_bytes <= smem_optin;
+}
+
+// Configurations of the last requests of this thread (they depend on the shape and the lines only).
+struct Entry {
+    int N, H, W, C, K, esize, smem, sms;
+    bool wgrad, taken;
+    std::vector<int8_t> chan;
+    SegConfig cfg;
+};
+constexpr size_t kKept = 64;
+
+}  // namespace
+
+bool seg_configure(const int8_t *chan, int N, int H, int W, int C, int K, int esize, int smem_optin, int sms, bool wgrad,
+                   const SegConfig **cfg) {
+    thread_local std::vector<std::unique_ptr<Entry>> kept;
+    thread_local size_t oldest = 0;
+    for (const auto &e : kept)
+        if (e->N == N && e->H == H && e->W == W && e->C == C && e->K == K && e->esize == esize && e->smem == smem_optin && e->sms == sms &&
+            e->wgrad == wgrad && memcmp(e->chan.data(), chan, C) == 0) {
+            *cfg = &e->cfg;
+            return e->taken;
+        }
+    auto e = std::make_unique<Entry>();
+    e->N = N; e->H = H; e->W = W; e->C = C; e->K = K; e->esize = esize; e->smem = smem_optin; e->sms = sms; e->wgrad = wgrad;
+    e->chan.assign(chan, chan + C);
+    e->taken = make_config(chan, N, H, W, C, K, esize, smem_optin, sms, wgrad, &e->cfg);
+    *cfg = &e->cfg;
+    const bool taken = e->taken;
+    if (kept.size() < kKept) kept.push_back(std::move(e));
+    else { kept[oldest] = std::move(e); oldest = (oldest + 1) % kKept; }
+    return taken;
+}
+
+namespace {
+struct ConvArgs {
+    const SegMaps *maps;
+    const void *w, *bias;
+    int wbf16;
+    const int8_t *chan;
+    void *y;
+    int *err_flag;
+    SegParams p;
+    cudaStream_t st;
+};
+template <typename T, int R, int LT> cudaError_t conv(const SegConfig &cfg, const ConvArgs &a) {
+    auto kern = seg::seg_conv_kernel<T, R, LT>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg.smem_bytes);
+    if (e != cudaSuccess) return e;
+    kern<<<cfg.grid, seg::kThreads, cfg.smem_bytes, a.st>>>(*a.maps, a.w, a.bias, a.wbf16, a.chan, (T *)a.y, a.err_flag, a.p);
+    return cudaGetLastError();
+}
+template <typename T> cudaError_t conv_any(const SegConfig &cfg, const ConvArgs &a) {
+    if (cfg.short_reach) return cfg.line_block == 28 ? conv<T, 7, 28>(cfg, a) : conv<T, 7, 14>(cfg, a);
+    return cfg.line_block == 28 ? conv<T, 15, 28>(cfg, a) : conv<T, 15, 14>(cfg, a);
+}
+}  // namespace
+
+cudaError_t seg_launch_conv(const SegConfig &cfg, const SegMaps &maps, const void *w, const void *bias, int wbf16,
+                            const int8_t *chan, void *y, int flip, int identity, int *err_flag, cudaStream_t st) {
+    ConvArgs a{&maps, w, bias, wbf16, chan, y, err_flag, cfg.p, st};
+    a.p.flip = flip;
+    a.p.identity = identity;
+    return cfg.esize == 4 ? conv_any<float>(cfg, a) : conv_any<__nv_bfloat16>(cfg, a);
+}
+
+}  // namespace o1d

@@ -1,0 +1,594 @@
+// Segment kernels: the oriented convolution straight from NHWC tiles, on pairs of channels with packed
+// fp32 arithmetic (fma.rn.f32x2).
+//
+// A tile (32 bytes of channels: 8 pairs of bf16 or 4 pairs of fp32 channels, 32 bytes being one DRAM
+// sector) is brought into shared memory by TMA in its global layout and is never rearranged.  A thread
+// owns one channel pair and a block of outputs, and streams the inputs that the block can see, each
+// loaded once and used for every output it reaches:
+//   rows, columns   28 positions of one line (14 on short lines): 58 loads for 868 packed FMAs (31 taps)
+//   diagonals       14 positions along the diagonal:              34 loads for 294 (21 distinct taps)
+//   slanted lines   3 lines x 8 positions:                       174 loads for 696 (29 taps on 11 lines)
+// The line is a stride (pixel, row, or row +- pixel), so the eight orientations are three bodies.
+// Weights sit in registers, one pair of floats per tap.
+//
+// Bound: the FMA pipe.  A packed FMA occupies it for two issue slots, which leaves every other slot for
+// the loads, the bf16 -> fp32 widening and the address arithmetic (1.5-2 instructions per input).
+// That is why the kernels take arbitrary positions inside the tile without special cases: inputs past
+// the end of a line are clamped onto a pixel of zeros (TMA fills coordinates outside the tensor), which
+// costs nothing while the pipe is busy; whole left / right halves of a line's halo are skipped at the
+// borders of the map.  One CTA of twelve warps per SM; the tile after next is loaded while the warps,
+// each at its own pace, walk through the tasks of the current one.
+//
+// Lanes are ordered pair first, so that the lanes of a load cover whole 32-byte pixels of neighbouring
+// lines (an odd pixel pitch keeps those in different banks) and the lanes of a store whole sectors.
+// Channels of a chunk that lie on different lines form classes with tasks of their own; a pair whose two
+// channels differ is computed once for each.
+#pragma once
+
+#include <cuda.h>
+
+#include <type_traits>
+
+#include "o1d_common.cuh"
+#include "o1d_lines.cuh"
+#include "o1d_seg.h"
+
+namespace o1d {
+namespace seg {
+
+constexpr int kWarps = 12, kThreads = 32 * kWarps;
+constexpr int kTD = 14;                  // outputs of a thread along a diagonal
+// lines x positions of a thread on slanted lines: an odd number of lines keeps neighbouring blocks in
+// different banks (4 x 7: 6 wavefronts a load)
+constexpr int kSR = 3, kST = 8;
+constexpr int kMaxBuf = 4;
+constexpr int kMaxCC = 32;               // channels of a chunk
+constexpr int kPadBytes = 256;           // zeros in front of the tile
+constexpr uint32_t kSpinLimit = 1u << 22;
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(f32x2 &d, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Bounded wait; on expiry raises the device flag and reports false.
+__device__ __noinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err_flag) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < kSpinLimit; i++)
+        if (mbar_try_wait(bar, parity)) return true;
+    *err_flag = 1;
+    return false;
+}
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+template <int I, int N, class F> __device__ __forceinline__ void static_for(F &&f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        static_for<I + 1, N>(f);
+    }
+}
+
+extern __shared__ __align__(1024) char g_smem[];
+
+// One pixel's channel pair, as two floats (from a byte offset in shared memory), and back.
+template <typename T> struct Pair;
+template <> struct Pair<float> {
+    static constexpr int kBytes = 8;
+    static __device__ __forceinline__ f32x2 lds(int a) { return *reinterpret_cast<const f32x2 *>(g_smem + a); }
+    static __device__ __forceinline__ f32x2 ldg(const float *p) { return __ldg(reinterpret_cast<const f32x2 *>(p)); }
+    static __device__ __forceinline__ void st(float *p, f32x2 v) { *reinterpret_cast<f32x2 *>(p) = v; }
+};
+template <> struct Pair<__nv_bfloat16> {
+    static constexpr int kBytes = 4;
+    static __device__ __forceinline__ f32x2 widen(uint32_t v) {
+        return pack2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+    }
+    static __device__ __forceinline__ f32x2 lds(int a) { return widen(*reinterpret_cast<const uint32_t *>(g_smem + a)); }
+    static __device__ __forceinline__ f32x2 ldg(const __nv_bfloat16 *p) { return widen(__ldg(reinterpret_cast<const uint32_t *>(p))); }
+    static __device__ __forceinline__ void st(__nv_bfloat16 *p, f32x2 v) {
+        const float2 f = unpack2(v);
+        uint32_t r;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(f.y), "f"(f.x));
+        *reinterpret_cast<uint32_t *>(p) = r;
+    }
+};
+
+// Frame of canonical line o: positions run along image columns (H), rows (V) or both (diagonals, from
+// row to row); stored tap t of the base line has weight t, or 30 - t when rev is set, and line offset
+// sgn * dh (o1d_lines.cuh).
+enum : int { FR_H = 0, FR_V = 1, FR_D = 2 };
+__host__ __device__ constexpr int frame_of(int o) { return (o == 0 || o == 1 || o == 7) ? FR_H : (o == 2 || o == 6) ? FR_D : FR_V; }
+__host__ __device__ constexpr int kind_of(int o) { return (o == 0 || o == 4) ? KIND_AXIS : (o == 2 || o == 6) ? KIND_DIAG : KIND_SLANT; }
+__host__ __device__ constexpr int sgn_of(int o) { return (o == 5 || o == 7) ? -1 : 1; }
+__host__ __device__ constexpr int rev_of(int o) { return (o == 0 || o == 1) ? 0 : 1; }
+constexpr bool frames_consistent() {
+    for (int o = 0; o < 8; o++)
+        for (int t = 0; t < kMaxTaps; t++) {
+            const int k = rev_of(o) ? kMaxTaps - 1 - t : t;
+            const int dh = kCanonDh[o][k], dw = kCanonDw[o][k], b = kind_of(o), fr = frame_of(o);
+            const int pos = fr == FR_H ? dw : dh;
+            const int line = fr == FR_H ? dh : fr == FR_V ? dw : o == 2 ? dw + dh : dw - dh;
+            if (pos != kCanonDw[b][t]) return false;
+            if (line != (b == KIND_SLANT ? sgn_of(o) * kCanonDh[1][t] : 0)) return false;
+        }
+    return true;
+}
+static_assert(frames_consistent(), "every canonical line must be a line (or a staircase of lines) of its frame");
+
+// Tap number of a slanted line at (line offset, position offset); the three centre taps share 15.
+constexpr int slant_tap(int dr, int dp, int half) {
+    for (int t = kHalf - half; t <= kHalf + half; t++)
+        if (kCanonDh[1][t] == dr && kCanonDw[1][t] == dp) return (t == 14 || t == 16) ? 15 : t;
+    return -1;
+}
+// Does input (rho, pi) reach any output of a slanted block?
+constexpr bool slant_used(int rho, int pi, int half) {
+    for (int r = 0; r < kSR; r++)
+        for (int t = 0; t < kST; t++)
+            if (slant_tap(rho - r, pi - t, half) >= 0) return true;
+    return false;
+}
+constexpr int slant_first(int rho, int half) {
+    for (int pi = -13; pi < kST + 13; pi++) if (slant_used(rho, pi, half)) return pi;
+    return 99;
+}
+constexpr int slant_last(int rho, int half) {
+    for (int pi = kST + 13; pi >= -13; pi--) if (slant_used(rho, pi, half)) return pi;
+    return -99;
+}
+
+// ---- bodies ----------------------------------------------------------------------------------------
+// O: the block's outputs (or, for the weight gradient, the values of dy there); Wt: the weights (or the
+// accumulators of their gradient), by stored tap.  Addresses are byte offsets in shared memory, of the
+// lane's channel pair.  Inputs are visited outwards from the block's first position, so that one add-and-clamp
+// per input keeps the address inside the line.
+template <bool WG> __device__ __forceinline__ void use(f32x2 &o, f32x2 &w, f32x2 x) {
+    if (WG) fma2(w, o, x); else fma2(o, w, x);
+}
+
+// Line: a = address of the block's first position, step between positions, lo / hi = addresses the line is
+// clamped to.  OUTSIDE: the first position itself may lie before lo (diagonals).  left / right: run the
+// inputs before / behind the block.
+template <typename T, int R, int NO, bool OUTSIDE, bool WG>
+__device__ __forceinline__ void line_body(int a, int step, int lo, int hi, bool left, bool right, f32x2 (&O)[NO],
+                                          f32x2 (&Wt)[kMaxTaps]) {
+    auto input = [&](auto i_, f32x2 x) {            // position i relative to the first output
+        constexpr int i = decltype(i_)::value;
+        static_for<0, NO>([&](auto o_) {
+            constexpr int o = decltype(o_)::value, j = i - o;
+            if constexpr (j >= -R && j <= R) use<WG>(O[o], Wt[kHalf + j], x);
+        });
+    };
+    if (left) {
+        int b = OUTSIDE ? max(a, lo) : a;
+        static_for<0, R>([&](auto i_) {
+            b = max(b - step, lo);
+            input(std::integral_constant<int, -1 - decltype(i_)::value>{}, Pair<T>::lds(b));
+        });
+    }
+    static_for<0, NO>([&](auto i_) {
+        input(i_, Pair<T>::lds(OUTSIDE ? max(a, lo) : a));
+        a = min(a + step, hi);
+    });
+    if (right)
+        static_for<NO, NO + R>([&](auto i_) {
+            input(i_, Pair<T>::lds(OUTSIDE ? max(a, lo) : a));
+            a = min(a + step, hi);
+        });
+}
+
+// Slanted line: 3 lines (l0.., in direction sgn) x 8 positions.  base = address of line 0, first position of
+// the block; lines outside [llo, lhi] read line lzero.  lo, hi: the clamps relative to the first position.
+template <typename T, int HALF, bool WG>
+__device__ __forceinline__ void slant_body(int base, int lstep, int pstep, int l0, int sgn, int llo, int lhi, int lzero, int lo,
+                                           int hi, f32x2 (&O)[kSR * kST], f32x2 (&Wt)[kMaxTaps]) {
+    constexpr int D = kCanonDh[1][kHalf - HALF];     // reach in lines
+    static_for<0, kSR + 2 * D>([&](auto r_) {
+        constexpr int rho = decltype(r_)::value - D, first = slant_first(rho, HALF), last = slant_last(rho, HALF);
+        int l = sgn > 0 ? l0 + rho : l0 + kSR - 1 - rho;
+        l = l < llo || l > lhi ? lzero : l;
+        const int la = base + l * lstep, alo = la + lo, ahi = la + hi;
+        auto input = [&](auto pi_, f32x2 x) {
+            constexpr int pi = decltype(pi_)::value;
+            static_for<0, kSR * kST>([&](auto o_) {
+                constexpr int o = decltype(o_)::value, t = slant_tap(rho - o / kST, pi - o % kST, HALF);
+                if constexpr (t >= 0) use<WG>(O[o], Wt[t], x);
+            });
+        };
+        if constexpr (first < 0) {
+            constexpr int s = last < 0 ? last : -1;
+            int b = max(la + s * pstep, alo);
+            static_for<0, s - first + 1>([&](auto i_) {
+                constexpr int pi = s - decltype(i_)::value;
+                if constexpr (slant_used(rho, pi, HALF)) input(std::integral_constant<int, pi>{}, Pair<T>::lds(b));
+                b = max(b - pstep, alo);
+            });
+        }
+        if constexpr (last >= 0) {
+            constexpr int s = first < 0 ? 0 : first;
+            int b = min(la + s * pstep, ahi);
+            static_for<0, last + 1 - s>([&](auto i_) {
+                constexpr int pi = decltype(i_)::value + s;
+                if constexpr (slant_used(rho, pi, HALF)) input(std::integral_constant<int, pi>{}, Pair<T>::lds(b));
+                b = min(b + pstep, ahi);
+            });
+        }
+    });
+}
+
+// ---- tables ----------------------------------------------------------------------------------------
+constexpr int kMaxPairs = kMaxCC / 2;
+// Pairs of one line that share a group of lanes: all of them, or half where that leaves fewer lanes idle.
+__host__ __device__ constexpr int class_pairs(int m) { return 32 / m * m < 27 ? (m + 1) / 2 : m; }
+struct Class { int canon, n, full, entry[kMaxPairs]; };        // entry: pair | channels of it (1 low, 2 high) << 4; full: all are 3
+struct Tables {
+    f32x2 w[32][kMaxPairs];                  // by stored tap (colliding taps summed) and pair
+    f32x2 bias[kMaxPairs];
+    int ncls, ids[kMaxCC];
+    Class cls[12];
+};
+// Taps summed into stored tap i of a line kind (three 5-bit numbers, 31 = none).
+struct MergeTable { uint16_t src[3][32]; };
+constexpr MergeTable make_merge() {
+    MergeTable m{};
+    for (int kind = 0; kind < 3; kind++)
+        for (int i = 0; i < 32; i++) {
+            int found[3] = {31, 31, 31}, n = 0;
+            for (int t = 0; t < kMaxTaps; t++) {
+                const int at = kind == KIND_SLANT ? (t == 14 || t == 16 ? 15 : t) : kCanonDw[kind][t] + kHalf;
+                if (at == i) found[n++] = t;
+            }
+            for (int e = 0; e < 3; e++) m.src[kind][i] |= (uint16_t)(found[e] << (5 * e));
+        }
+    return m;
+}
+static __device__ const MergeTable g_merge = make_merge();
+
+// Weight of base tap t of channel c on canonical line id (0 when the kernel is shorter than the line).
+__device__ __forceinline__ float base_weight(const void *w, int wbf16, int c, int id, int t, const SegParams &p) {
+    if (t >= kMaxTaps) return 0.f;
+    const int k = ((rev_of(id) ^ p.flip) ? kMaxTaps - 1 - t : t) - kHalf + p.K / 2;
+    if (k < 0 || k >= p.K) return 0.f;
+    const size_t at = (size_t)c * p.K + k;
+    return wbf16 ? __bfloat162float(((const __nv_bfloat16 *)w)[at]) : __ldg((const float *)w + at);
+}
+// Tables of the chunk that starts at channel c0; ends in a barrier.
+__device__ __noinline__ void build_tables(Tables *tab, const SegParams &p, const void *w, const void *bias, int wbf16,
+                                          const int8_t *chan, int c0) {
+    const int tid = threadIdx.x;
+    if (tid < p.CC) tab->ids[tid] = c0 + tid < p.C ? (int)__ldg(chan + c0 + tid) : -1;
+    if (tid < p.CC)
+        reinterpret_cast<float *>(tab->bias)[tid] =
+            !bias || c0 + tid >= p.C ? 0.f
+            : wbf16 ? __bfloat162float(((const __nv_bfloat16 *)bias)[c0 + tid]) : __ldg((const float *)bias + c0 + tid);
+    __syncthreads();
+    if (w)
+#pragma unroll 1
+        for (int i = tid; i < p.CC * 32; i += kThreads) {
+            const int c = i >> 5, t = i & 31, id = tab->ids[c];
+            float v = 0.f;
+            if (id >= 0) {
+                const uint32_t src = g_merge.src[kind_of(id)][t];
+                v = base_weight(w, wbf16, c0 + c, id, src & 31, p) + base_weight(w, wbf16, c0 + c, id, src >> 5 & 31, p) +
+                    base_weight(w, wbf16, c0 + c, id, src >> 10 & 31, p);
+                if (t == kHalf && p.identity) v += 1.f;
+            }
+            reinterpret_cast<float *>(&tab->w[t][c >> 1])[c & 1] = v;
+        }
+    if (tid == kThreads - 1) {
+        int n = 0;
+#pragma unroll 1
+        for (int o = 0; o < 8; o++) {
+            int m = 0;
+#pragma unroll 1
+            for (int q = 0; q < p.CC / 2; q++) m += tab->ids[2 * q] == o || tab->ids[2 * q + 1] == o;
+            const int most = m ? class_pairs(m) : 0;
+            int q = 0;
+#pragma unroll 1
+            while (m > 0) {
+                Class *cl = &tab->cls[n++];
+                cl->canon = o;
+                cl->full = 1;
+                cl->n = 0;
+#pragma unroll 1
+                for (; cl->n < most && m > 0; q++) {
+                    const int mask = (tab->ids[2 * q] == o ? 1 : 0) | (tab->ids[2 * q + 1] == o ? 2 : 0);
+                    if (!mask) continue;
+                    cl->entry[cl->n++] = q | mask << 4;
+                    m--;
+                    if (mask != 3) cl->full = 0;
+                }
+            }
+        }
+        tab->ncls = n;
+    }
+    __syncthreads();
+}
+
+// Either channel of a pair, or both: predicated stores (branches would triple the code).
+template <typename T> __device__ __forceinline__ void store_pair(T *p, f32x2 v, int mask) {
+    const float2 f = unpack2(v);
+    if constexpr (sizeof(T) == 4)
+        asm volatile("{.reg .pred l, h;\n setp.ne.u32 l, %3, 0;\n setp.ne.u32 h, %4, 0;\n @l st.global.f32 [%0], %1;\n @h st.global.f32 [%0+4], %2;}"
+                     ::"l"(p), "f"(f.x), "f"(f.y), "r"(mask & 1), "r"(mask & 2) : "memory");
+    else
+        asm volatile("{.reg .pred l, h;\n .reg .b16 a, b;\n setp.ne.u32 l, %3, 0;\n setp.ne.u32 h, %4, 0;\n cvt.rn.bf16.f32 a, %1;\n"
+                     " cvt.rn.bf16.f32 b, %2;\n @l st.global.b16 [%0], a;\n @h st.global.b16 [%0+2], b;}"
+                     ::"l"(p), "f"(f.x), "f"(f.y), "r"(mask & 1), "r"(mask & 2) : "memory");
+}
+
+// `left` outputs of a line (at most NO), ps elements apart.
+template <typename T, int NO>
+__device__ __forceinline__ void store_line(T *q, ptrdiff_t ps, const f32x2 *O, int left, bool all, int mask) {
+    if (all) {
+#pragma unroll
+        for (int o = 0; o < NO; o++) {
+            if (o < left) Pair<T>::st(q, O[o]);
+            q += ps;
+        }
+    } else {
+#pragma unroll
+        for (int o = 0; o < NO; o++) {
+            if (o < left) store_pair(q, O[o], mask);
+            q += ps;
+        }
+    }
+}
+
+// ---- kernel ----------------------------------------------------------------------------------------
+// Division of the work.  A part is 1 / kParts of an item's tasks.
+//   CTAs per chunk (p.per_chunk): every chunk has a number of CTAs in proportion to its cost; they take its
+//   items in turn, and the last, incomplete round by parts.  All chunks advance through the images at one
+//   pace, so the chunks that share a pixel's DRAM bursts and L2 lines meet there.
+//   Otherwise (too many chunks for that): the sequence runs, chunks, items, parts is cut into shares of
+//   equal cost, one per CTA.
+constexpr int kParts = 8;
+struct Segment {                             // work of a CTA on one chunk
+    int run, chunk;                          // chunk within the run
+    int full, first, step;                   // items first, first + step, ...: `full` whole ones,
+    int begin, end;                          // then the parts [begin, end) of the chunk
+    __device__ __forceinline__ int count() const { return full + (end > begin ? (end + kParts - 1) / kParts - begin / kParts : 0); }
+    __device__ __forceinline__ int item(int s) const { return s < full ? first + s * step : begin / kParts + s - full; }
+};
+struct Spot { int run, chunk, part; };
+__device__ __forceinline__ Spot spot_of(const SegParams &p, long long at) {
+    Spot s{0, 0, 0};
+#pragma unroll 1
+    for (; s.run < p.nruns; s.run++) {
+        const SegRun &r = p.run[s.run];
+        const long long chunk = (long long)r.cost * p.geo[r.geo].items * kParts, all = chunk * r.nchunks;
+        if (at < all) {
+            s.chunk = (int)(at / chunk);
+            s.part = (int)((at - s.chunk * chunk) / r.cost);
+            return s;
+        }
+        at -= all;
+    }
+    return s;                                // one past the end
+}
+__device__ __forceinline__ bool first_segment(const SegParams &p, Segment &g, Spot &at, const Spot &end) {
+    if (p.per_chunk) {
+        int b = blockIdx.x;
+        g.run = 0;
+#pragma unroll 1
+        while (b >= p.run[g.run].nchunks * p.run[g.run].ctas) { b -= p.run[g.run].nchunks * p.run[g.run].ctas; g.run++; }
+        const int kc = p.run[g.run].ctas, items = p.geo[p.run[g.run].geo].items;
+        g.chunk = b / kc;
+        g.first = b - g.chunk * kc;
+        g.step = kc;
+        g.full = items / kc;
+        const int base = g.full * kc * kParts, tail = items * kParts - base;
+        g.begin = base + tail * g.first / kc;
+        g.end = base + tail * (g.first + 1) / kc;
+        return g.count() > 0;
+    }
+    g.full = g.first = g.step = 0;
+    if (at.run > end.run || (at.run == end.run && (at.chunk > end.chunk || (at.chunk == end.chunk && at.part >= end.part)))) return false;
+    g.run = at.run;
+    g.chunk = at.chunk;
+    g.begin = at.part;
+    const bool here = at.run == end.run && at.chunk == end.chunk;
+    g.end = here ? end.part : p.geo[p.run[at.run].geo].items * kParts;
+    // where the next segment starts
+    at.part = 0;
+    if (here) at = end;
+    else if (++at.chunk == p.run[at.run].nchunks) { at.chunk = 0; at.run++; }
+    return at.run < p.nruns || g.run < p.nruns;
+}
+
+// R: reach of the taps (15, or 7 for kernels of up to 15 taps); LT: outputs of a thread along a line.
+template <typename T, int R, int LT>
+__global__ void __launch_bounds__(kThreads, 1)
+seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ wv, const void *__restrict__ biasv, int wbf16,
+                const int8_t *__restrict__ chan, T *__restrict__ y, int *__restrict__ err_flag,
+                const __grid_constant__ SegParams p) {
+    char *sm = g_smem;
+    constexpr int PB = Pair<T>::kBytes, RD = kCanonDh[2][kHalf - R];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    Tables *tab = reinterpret_cast<Tables *>(sm + p.off_tab);
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + p.off_bar);
+    int *cnt = reinterpret_cast<int *>(full + kMaxBuf);
+
+    Segment g;
+    Spot at{0, 0, 0}, end{0, 0, 0};
+    if (!p.per_chunk) {
+        at = spot_of(p, p.total_cost * blockIdx.x / gridDim.x);
+        end = spot_of(p, p.total_cost * (blockIdx.x + 1) / gridDim.x);
+    }
+    bool more = first_segment(p, g, at, end);
+    auto issue = [&](const Segment &g, int s, int buf) {          // item number s of the segment
+        const SegGeo &ge = p.geo[p.run[g.run].geo];
+        const int it = g.item(s), tiles = ge.nth * ge.ntw;
+        int n0 = it * ge.G, th = 0, tw = 0;
+        if (tiles > 1) {
+            n0 = it / tiles;
+            const int r = it - n0 * tiles;
+            th = r / ge.ntw;
+            tw = r - th * ge.ntw;
+        }
+        mbar_expect_tx(&full[buf], ge.tile_bytes);
+        tma_load_4d(sm + p.off_tile + buf * ge.buf_bytes, &maps.m[p.run[g.run].geo], &full[buf],
+                    (p.run[g.run].chunk0 + g.chunk) * p.CC, tw * ge.TW - ge.ow, th * ge.TH - ge.oh, n0);
+    };
+    if (tid == 0) {
+#pragma unroll 1
+        for (int b = 0; b < kMaxBuf; b++) { mbar_init(&full[b], 1); cnt[b] = 0; }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = tid; i < kPadBytes / 4; i += kThreads) reinterpret_cast<float *>(sm + p.off_tile - kPadBytes)[i] = 0.f;
+
+    int turn = warp;                             // tasks until this warp's next one
+    bool ok = true;
+    uint32_t phase = 0;                          // parity of each buffer's barrier
+#pragma unroll 1
+    for (; more; more = !p.per_chunk && first_segment(p, g, at, end)) {
+        const SegGeo &ge = p.geo[p.run[g.run].geo];
+        const int c0 = (p.run[g.run].chunk0 + g.chunk) * p.CC, tiles = ge.nth * ge.ntw, row_bytes = ge.P * p.px, px = p.px;
+        const int nitems = g.count();
+        __syncthreads();                         // the previous segment is done with tables and buffers
+        if (tid == 0) {
+#pragma unroll 1
+            for (int b = 0; b < ge.nbuf && b < nitems; b++) issue(g, b, b);
+        }
+        // the pixel in front of a buffer's tile is the previous buffer's last one: zeros
+        for (int i = tid; i < ge.nbuf * 16; i += kThreads)
+            if ((i & 15) * 4 < px)
+                *reinterpret_cast<float *>(sm + p.off_tile + ((i >> 4) + 1) * ge.buf_bytes - px + (i & 15) * 4) = 0.f;
+        build_tables(tab, p, wv, biasv, wbf16, chan, c0);
+        int buf = 0;
+#pragma unroll 1
+        for (int s = 0; s < nitems; s++) {
+            const int it = g.item(s);
+            const int part0 = s < g.full ? 0 : max(g.begin - it * kParts, 0), part1 = s < g.full ? kParts : min(g.end - it * kParts, kParts);
+            int n0 = it * ge.G, h0 = 0, w0 = 0, imgs = min(ge.G, p.N - n0);
+            if (tiles > 1) {
+                n0 = it / tiles;
+                imgs = 1;
+                const int r = it - n0 * tiles;
+                h0 = r / ge.ntw;
+                w0 = (r - h0 * ge.ntw) * ge.TW;
+                h0 *= ge.TH;
+            }
+            const int lenh = min(ge.TH, p.H - h0), lenw = min(ge.TW, p.W - w0);       // outputs of this tile
+            const int tbuf = p.off_tile + buf * ge.buf_bytes + ge.oh * row_bytes + ge.ow * px;
+            if (ok) ok = mbar_wait(&full[buf], phase >> buf & 1, err_flag);
+            phase ^= 1u << buf;
+#pragma unroll 1
+            for (int ci = 0; ci < tab->ncls; ci++) {
+                const Class *cl = &tab->cls[ci];
+                const int id = cl->canon, np = cl->n, kind = kind_of(id), fr = frame_of(id);
+                const int lpg = 32 / np;                                            // lines per group of lanes
+                const int plen = fr == FR_H ? lenw : lenh, llen = fr == FR_H ? lenh : lenw;
+                const int nlines = kind == KIND_AXIS ? llen : kind == KIND_DIAG ? lenw + kTD - 1 : (llen + kSR - 1) / kSR;
+                const int bl = kind == KIND_SLANT ? kST : kind == KIND_AXIS ? LT : kTD, npb = (plen + bl - 1) / bl;
+                const int nt = (imgs * nlines + lpg - 1) / lpg * npb, t0 = nt * part0 / kParts, t1 = nt * part1 / kParts;
+                const int ln = lane / np, entry = cl->entry[lane - ln * np], pair = entry & 15, mask = entry >> 4;
+                const bool all = cl->full;
+                int t = t0 + turn, ug = t / npb, pb = t - ug * npb;
+                const int dug = kWarps / npb, dpb = kWarps - dug * npb;
+                turn -= t1 - t0;
+#pragma unroll 1
+                for (; t < t1; t += kWarps, turn += kWarps) {
+                    const int li = ug * lpg + ln, gi = ge.G == 1 ? (li >= nlines) : li / nlines, line = li - gi * nlines;
+                    const bool act = ln < lpg && gi < imgs;
+                    const int gt = tbuf + pair * PB + (act ? gi : 0) * ge.img_bytes;         // first output of the image
+                    f32x2 Wt[kMaxTaps];
+#pragma unroll
+                    for (int i = 0; i < kMaxTaps; i++) Wt[i] = tab->w[i][pair];
+                    const f32x2 bias = tab->bias[pair];
+                    T *yi = y + ((size_t)(n0 + gi) * p.H + h0) * p.W * p.C + (size_t)w0 * p.C + c0 + 2 * pair;
+                    const int p0 = pb * bl;
+                    if (kind == KIND_SLANT) {
+                        f32x2 O[kSR * kST];
+#pragma unroll
+                        for (int o = 0; o < kSR * kST; o++) O[o] = bias;
+                        const int l0 = line * kSR;
+                        const bool hf = fr == FR_H;
+                        const int lstep = hf ? row_bytes : px, pstep = hf ? px : row_bytes;
+                        const int plo = hf ? ge.plo_w : ge.plo_h, phi = hf ? ge.phi_w : ge.phi_h;
+                        const int cut = hf ? ge.halo_h : ge.halo_w;
+                        const int llo = (hf ? ge.plo_h : ge.plo_w) + 1 - cut, lhi = (hf ? ge.phi_h : ge.phi_w) - 1 + cut;
+                        const int lzero = cut ? 0 : hf ? ge.plo_h : ge.phi_w;
+                        slant_body<T, R, false>(gt + p0 * pstep, lstep, pstep, l0, sgn_of(id), llo, lhi, lzero, (plo - p0) * pstep,
+                                                (phi - p0) * pstep, O, Wt);
+                        const ptrdiff_t ls = hf ? (ptrdiff_t)p.W * p.C : p.C, ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
+#pragma unroll
+                        for (int r = 0; r < kSR; r++) {
+                            const int l = sgn_of(id) > 0 ? l0 + r : l0 + kSR - 1 - r;
+                            store_line<T, kST>(yi + l * ls + p0 * ps, ps, &O[r * kST], act && l < llen ? plen - p0 : 0, all, mask);
+                        }
+                    } else if (kind == KIND_AXIS) {
+                        f32x2 O[LT];
+#pragma unroll
+                        for (int o = 0; o < LT; o++) O[o] = bias;
+                        const bool hf = fr == FR_H;
+                        const int step = hf ? px : row_bytes, base = gt + line * (hf ? row_bytes : px);
+                        const bool cut = hf ? ge.halo_w : ge.halo_h;
+                        line_body<T, R, LT, false, false>(base + p0 * step, step, base + (hf ? ge.plo_w : ge.plo_h) * step,
+                                                          base + (hf ? ge.phi_w : ge.phi_h) * step, p0 > 0 || cut, p0 + LT < plen || cut,
+                                                          O, Wt);
+                        const ptrdiff_t ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
+                        store_line<T, LT>(yi + line * (hf ? (ptrdiff_t)p.W * p.C : p.C) + p0 * ps, ps, O, act ? plen - p0 : 0, all, mask);
+                    } else {
+                        f32x2 O[kTD];
+#pragma unroll
+                        for (int o = 0; o < kTD; o++) O[o] = bias;
+                        const int dw = id == 2 ? -1 : 1, w = dw > 0 ? line - (kTD - 1) : line;
+                        // where the diagonal enters and leaves the tile (at the zeros around a whole map), from the block's first position
+                        const int f = max(dw > 0 ? ge.plo_w - w : w - ge.phi_w, ge.plo_h - p0);
+                        const int l = min(dw > 0 ? ge.phi_w - w : w - ge.plo_w, ge.phi_h - p0);
+                        const int step = row_bytes + dw * px, a0 = gt + p0 * row_bytes + w * px;
+                        line_body<T, RD, kTD, true, false>(a0, step, a0 + f * step, a0 + l * step, p0 > 0 || ge.halo_h,
+                                                           p0 + kTD < plen || ge.halo_h, O, Wt);
+                        T *yl = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
+                        const ptrdiff_t ps = ((ptrdiff_t)p.W + dw) * p.C;
+#pragma unroll
+                        for (int o = 0; o < kTD; o++) {
+                            if (act && p0 + o < plen && (unsigned)(w + o * dw) < (unsigned)lenw) {
+                                if (all) Pair<T>::st(yl, O[o]); else store_pair(yl, O[o], mask);
+                            }
+                            yl += ps;
+                        }
+                    }
+                    ug += dug;
+                    pb += dpb;
+                    if (pb >= npb) { pb -= npb; ug++; }
+                }
+            }
+            __syncwarp();
+            if (lane == 0 && atomicAdd(&cnt[buf], 1) == kWarps - 1) {       // last warp through: refill
+                cnt[buf] = 0;
+                if (s + ge.nbuf < nitems) issue(g, s + ge.nbuf, buf);
+            }
+            if (++buf == ge.nbuf) buf = 0;
+        }
+    }
+}
+
+}  // namespace seg
+}  // namespace o1d

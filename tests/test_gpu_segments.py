@@ -1,0 +1,60 @@
+"""Segment kernels (csrc/o1d_seg.cuh): sizes around the edges of their blocks, lanes and tiles, against
+the general kernels on the same device inputs."""
+import math
+
+import pytest
+import torch
+
+import oriented1d_b200 as o1d
+from tests.util import angle_list
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _plan(mode, C, K):
+    return o1d.Plan([math.pi * int(mode[3:]) / 8] * C if mode.startswith("one") else angle_list(mode, C), K)
+
+
+# N, H, W, C, K, angles: one pixel, one row, blocks of 14 / 28 positions and 3 x 8 / 14 x diagonal blocks with and
+# without remainder, several images per item, a last item with fewer, channels that do not fill a chunk, pairs of
+# channels on two lines, maps cut along either axis
+SHAPES = [(1, 1, 1, 16, 31, "one2"), (3, 1, 29, 16, 31, "one1"), (2, 30, 1, 8, 15, "one6"), (5, 13, 15, 64, 31, "model"),
+          (4, 14, 28, 24, 27, "one7"), (2, 29, 27, 64, 31, "model+"), (17, 10, 9, 40, 7, "model"), (2, 57, 56, 32, 31, "one5"),
+          (1, 56, 57, 96, 31, "model"), (2, 61, 120, 48, 31, "model+"), (1, 130, 35, 64, 13, "model"), (1, 210, 333, 16, 31, "one3"),
+          (1, 99, 301, 16, 31, "one6"), (1, 300, 301, 8, 31, "one4")]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_segments_equal_general(shape, dtype):
+    N, H, W, C, K, mode = shape
+    g = torch.Generator(device=DEV).manual_seed(H * W + C)
+    x = torch.randn((N, H, W, C), generator=g, device=DEV).to(dtype)
+    dy = torch.randn((N, H, W, C), generator=g, device=DEV).to(dtype)
+    w = 0.1 * torch.randn((C, 1, 1, K), generator=g, device=DEV)
+    bias = torch.randn((C,), generator=g, device=DEV)
+    plan = _plan(mode, C, K)
+
+    def run(route):
+        try:
+            o1d.ops.set_route(route)
+            out = (o1d.fprop(x, w, bias, plan, 1, True, True), o1d.dgrad(dy, w, plan, H, W, 1, True))
+            name = o1d.ops.last_route()
+            return out + o1d.wgrad(dy, x, plan, 1, True, True), name
+        finally:
+            o1d.ops.set_route(0)
+
+    ref, _ = run(1)
+    got, name = run(0)
+    assert name == "direct" and o1d.ops.device_status() == 0
+    for a, b in zip(got[:2], ref[:2]):
+        a, b = a.float(), b.float()
+        if dtype == torch.float32:
+            assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+        else:                                    # both round an fp32 sum: at most one bf16 ulp apart
+            assert float(((a - b).abs() / b.abs().clamp_min(1e-2)).max()) <= 2 ** -7
+    for a, b in zip(got[2:], ref[2:]):
+        assert float((a - b).abs().max()) <= 1e-4 * float(b.abs().max())
+    again = run(0)[0]
+    assert all(torch.equal(a, b) for a, b in zip(got, again))        # same bits again
