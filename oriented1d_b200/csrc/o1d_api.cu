@@ -310,15 +310,15 @@ int device_flag_ptr(int **out) {
     return O1D_OK;
 }
 
-// Tensor maps of `t` for every way the configuration cuts it.
-int seg_maps(const SegConfig &cfg, const void *t, SegMaps *maps, const char *what) {
+// Tensor maps of `t` for every way the configuration cuts it: the tiles with their halo, or the outputs alone.
+int seg_maps(const SegConfig &cfg, const void *t, bool with_halo, SegMaps *maps, const char *what) {
     const SegParams &p = cfg.p;
     const size_t e = cfg.esize;
     const cuuint64_t dims[4] = {(cuuint64_t)p.C, (cuuint64_t)p.W, (cuuint64_t)p.H, (cuuint64_t)p.N};
     const cuuint64_t strides[3] = {p.C * e, (cuuint64_t)p.W * p.C * e, (cuuint64_t)p.H * p.W * p.C * e};
     for (int i = 0; i < cfg.ngeos; i++) {
         const SegGeo &g = p.geo[i];
-        const cuuint32_t box[4] = {(cuuint32_t)p.CC, (cuuint32_t)g.P, (cuuint32_t)g.RT, (cuuint32_t)g.G};
+        const cuuint32_t box[4] = {(cuuint32_t)p.CC, (cuuint32_t)(with_halo ? g.P : g.TW), (cuuint32_t)(with_halo ? g.RT : g.TH), (cuuint32_t)g.G};
         O1D_MAP(encode_map4(&maps->m[i], t, cfg.esize, dims, strides, box), what);
     }
     return O1D_OK;
@@ -336,7 +336,7 @@ int try_seg(const void *x, const void *w, const void *bias, int wbf16, const Pla
     if (!seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, false, &cfg)) return kNotTiled;
     if (((uintptr_t)y & 15) != 0) return kNotTiled;
     SegMaps maps;
-    int rc = seg_maps(*cfg, x, &maps, "segment fprop");
+    int rc = seg_maps(*cfg, x, true, &maps, "segment fprop");
     if (rc) return rc;
     int *flag = nullptr;
     if ((rc = device_flag_ptr(&flag))) return rc;
@@ -546,6 +546,30 @@ int try_direct_wgrad(const void *dy, const void *x, const PlanHeader &ph, const 
     const int tot = C * (K + 1);
     direct_wgrad_final_kernel<<<ceil_div(tot, 128), 128, 0, st>>>(mp, partial, pv.cls, pv.taps, dw, db, C, K);
     O1D_CUDA(cudaGetLastError());
+    g_last_route = O1D_ROUTE_DIRECT;
+    return O1D_OK;
+}
+
+// Weight gradient through the segment kernels; dw and db bf16 when `out_bf16` is set.
+int try_seg_wgrad(const void *dy, const void *x, const PlanHeader &ph, const void *plan_host, const void *plan_dev, void *dw,
+                  void *db, int out_bf16, void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K,
+                  int stride, int layout, int dtype, cudaStream_t st, const DeviceInfo &d) {
+    if (g_force_generic || !ph.all_canon || ph.chan_off == 0 || stride != 1 || layout != O1D_NHWC) return kNotTiled;
+    const int esize = dtype == O1D_F32 ? 4 : 2;
+    const int8_t *chan_host = reinterpret_cast<const int8_t *>(static_cast<const char *>(plan_host) + ph.chan_off);
+    const SegConfig *cfg = nullptr;
+    if (!seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, true, &cfg)) return kNotTiled;
+    if (((uintptr_t)dy & 15) != 0 || ((uintptr_t)workspace & 15) != 0) return kNotTiled;
+    if (workspace_bytes < seg_wgrad_bytes(*cfg)) return O1D_ERR_WORKSPACE;
+    SegMaps maps, dy_maps;
+    int rc = seg_maps(*cfg, x, true, &maps, "segment wgrad (x)");
+    if (rc) return rc;
+    if ((rc = seg_maps(*cfg, dy, false, &dy_maps, "segment wgrad (dy)"))) return rc;
+    int *flag = nullptr;
+    if ((rc = device_flag_ptr(&flag))) return rc;
+    PlanView pv = plan_view(plan_dev, ph);
+    const cudaError_t e = seg_launch_wgrad(*cfg, maps, dy_maps, pv.chan, dy, dw, db, out_bf16, (float *)workspace, flag, st);
+    if (e != cudaSuccess) return cuda_fail(e, "segment wgrad launch");
     g_last_route = O1D_ROUTE_DIRECT;
     return O1D_OK;
 }
@@ -808,8 +832,14 @@ namespace {
 // (stems, dense-prediction maps, arbitrary angles), then general.
 int wgrad_dispatch(const void *dy, const void *x, const PlanHeader &ph, const void *plan_host, const void *plan_dev,
                    float *dw, float *db, void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K,
-                   int stride, int layout, int dtype, int act, cudaStream_t st, const DeviceInfo &d) {
+                   int stride, int layout, int dtype, int act, int out_bf16, cudaStream_t st, const DeviceInfo &d) {
     int rc;
+    if (g_prefer == 0 && !act && !(H == 7 && W == 7)) {       // see route_forward
+        rc = try_seg_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, out_bf16, workspace, workspace_bytes, N, H, W, C, K, stride,
+                           layout, dtype, st, d);
+        if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
+    }
+    if (out_bf16) return O1D_ERR_UNSUPPORTED;                 // the other families write fp32 gradients
     if (act) {                 // x is GELU(pre), applied on load: tiled kernels, else general
         rc = try_tiled_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, workspace, workspace_bytes, N, H, W, C, K, stride,
                              layout, dtype, act, st, d, nullptr);
@@ -877,7 +907,8 @@ int o1d_wgrad_act(const void *dy, const void *x, const void *plan_host, const vo
     DeviceInfo d;
     if ((rc = device_info(&d))) return rc;
     return wgrad_dispatch(dy, x, ph, plan_host, plan_dev, dw, db, workspace, workspace_bytes, N, H, W, C, K, stride,
-                          layout, dtype, (flags & O1D_FLAG_GELU_INPUT) ? 1 : 0, (cudaStream_t)stream, d);
+                          layout, dtype, (flags & O1D_FLAG_GELU_INPUT) ? 1 : 0, (flags & O1D_FLAG_PARAMS_BF16) ? 1 : 0,
+                          (cudaStream_t)stream, d);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -934,7 +965,7 @@ int o1d_wgrad_static(const void *dy, const void *x, const void *plan_host, const
     // Same order of kernel families as o1d_wgrad(); a family whose partial sums exceed the array
     // is skipped, and when even the general kernels' do not fit the request is refused.
     rc = wgrad_dispatch(dy, x, ph, plan_host, plan_dev, dw, db, scratch, O1D_STATIC_SCRATCH_BYTES, N, H, W, C, K,
-                        stride, layout, dtype, 0, (cudaStream_t)stream, d);
+                        stride, layout, dtype, 0, 0, (cudaStream_t)stream, d);
     if (rc == O1D_ERR_WORKSPACE) {
         snprintf(g_err, sizeof(g_err), "o1d_wgrad_static: the partial sums of this shape do not fit the built-in "
                  "array of %d bytes; use o1d_wgrad() with a workspace", O1D_STATIC_SCRATCH_BYTES);

@@ -163,6 +163,7 @@ bool make_config(const int8_t *chan, int N, int H, int W, int C, int K, int esiz
     for (int i = 0; i < cfg->ngeos; i++)
         if (p.geo[i].nbuf * p.geo[i].buf_bytes > bytes) bytes = p.geo[i].nbuf * p.geo[i].buf_bytes;
     for (int r = 0; r < p.nruns; r++) items += (long long)p.run[r].nchunks * p.geo[p.run[r].geo].items;
+    if (wgrad && bytes < seg::kWarps * 32 * seg::kMaxPairs * 8) bytes = seg::kWarps * 32 * seg::kMaxPairs * 8;   // sums over warps
     p.off_tile = round_up(seg::kPadBytes, 128);
     p.off_tab = p.off_tile + bytes;
     p.off_bar = p.off_tab + round_up((int)sizeof(seg::Tables), 16);
@@ -232,35 +233,51 @@ bool seg_configure(const int8_t *chan, int N, int H, int W, int C, int K, int es
 }
 
 namespace {
-struct ConvArgs {
-    const SegMaps *maps;
+struct Args {
+    const SegMaps *maps, *dy_maps;
     const void *w, *bias;
     int wbf16;
     const int8_t *chan;
     void *y;
+    float *partial;
     int *err_flag;
     SegParams p;
     cudaStream_t st;
 };
-template <typename T, int R, int LT> cudaError_t conv(const SegConfig &cfg, const ConvArgs &a) {
-    auto kern = seg::seg_conv_kernel<T, R, LT>;
+template <typename T, int R, int LT, bool WG> cudaError_t launch(const SegConfig &cfg, const Args &a) {
+    auto kern = seg::seg_kernel<T, R, LT, WG>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg.smem_bytes);
     if (e != cudaSuccess) return e;
-    kern<<<cfg.grid, seg::kThreads, cfg.smem_bytes, a.st>>>(*a.maps, a.w, a.bias, a.wbf16, a.chan, (T *)a.y, a.err_flag, a.p);
+    kern<<<cfg.grid, seg::kThreads, cfg.smem_bytes, a.st>>>(*a.maps, *a.dy_maps, a.w, a.bias, a.wbf16, a.chan, (T *)a.y, a.partial,
+                                                            a.err_flag, a.p);
     return cudaGetLastError();
 }
-template <typename T> cudaError_t conv_any(const SegConfig &cfg, const ConvArgs &a) {
-    if (cfg.short_reach) return cfg.line_block == 28 ? conv<T, 7, 28>(cfg, a) : conv<T, 7, 14>(cfg, a);
-    return cfg.line_block == 28 ? conv<T, 15, 28>(cfg, a) : conv<T, 15, 14>(cfg, a);
+template <typename T, bool WG> cudaError_t launch_any(const SegConfig &cfg, const Args &a) {
+    if (cfg.short_reach) return cfg.line_block == 28 ? launch<T, 7, 28, WG>(cfg, a) : launch<T, 7, 14, WG>(cfg, a);
+    return cfg.line_block == 28 ? launch<T, 15, 28, WG>(cfg, a) : launch<T, 15, 14, WG>(cfg, a);
 }
 }  // namespace
 
 cudaError_t seg_launch_conv(const SegConfig &cfg, const SegMaps &maps, const void *w, const void *bias, int wbf16,
                             const int8_t *chan, void *y, int flip, int identity, int *err_flag, cudaStream_t st) {
-    ConvArgs a{&maps, w, bias, wbf16, chan, y, err_flag, cfg.p, st};
+    Args a{&maps, &maps, w, bias, wbf16, chan, y, nullptr, err_flag, cfg.p, st};
     a.p.flip = flip;
     a.p.identity = identity;
-    return cfg.esize == 4 ? conv_any<float>(cfg, a) : conv_any<__nv_bfloat16>(cfg, a);
+    return cfg.esize == 4 ? launch_any<float, false>(cfg, a) : launch_any<__nv_bfloat16, false>(cfg, a);
+}
+
+size_t seg_wgrad_bytes(const SegConfig &cfg) {
+    const int slots = cfg.grid + (cfg.p.per_chunk ? 0 : ceil_div(cfg.p.C, cfg.p.CC));
+    return (size_t)slots * cfg.p.CC * 32 * sizeof(float);
+}
+
+cudaError_t seg_launch_wgrad(const SegConfig &cfg, const SegMaps &maps, const SegMaps &dy_maps, const int8_t *chan, const void *dy,
+                             void *dw, void *db, int out_bf16, float *partial, int *err_flag, cudaStream_t st) {
+    Args a{&maps, &dy_maps, nullptr, nullptr, 0, chan, const_cast<void *>(dy), partial, err_flag, cfg.p, st};
+    const cudaError_t e = cfg.esize == 4 ? launch_any<float, true>(cfg, a) : launch_any<__nv_bfloat16, true>(cfg, a);
+    if (e != cudaSuccess) return e;
+    seg::seg_wgrad_final_kernel<<<ceil_div(cfg.p.C, cfg.p.CC), 256, 0, st>>>(partial, chan, dw, db, out_bf16, cfg.grid, cfg.p);
+    return cudaGetLastError();
 }
 
 }  // namespace o1d

@@ -57,6 +57,7 @@ __device__ __forceinline__ float2 unpack2(f32x2 v) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
     return r;
 }
+__device__ __forceinline__ void add2(f32x2 &d, f32x2 a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(a)); }
 __device__ __forceinline__ void fma2(f32x2 &d, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -86,6 +87,9 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, u
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
         ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap *map, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
 template <int I, int N, class F> __device__ __forceinline__ void static_for(F &&f) {
     if constexpr (I < N) {
         f(std::integral_constant<int, I>{});
@@ -100,7 +104,11 @@ template <typename T> struct Pair;
 template <> struct Pair<float> {
     static constexpr int kBytes = 8;
     static __device__ __forceinline__ f32x2 lds(int a) { return *reinterpret_cast<const f32x2 *>(g_smem + a); }
-    static __device__ __forceinline__ f32x2 ldg(const float *p) { return __ldg(reinterpret_cast<const f32x2 *>(p)); }
+    static __device__ __forceinline__ f32x2 ldg_if(bool c, const float *p) {         // zero when !c
+        f32x2 r;
+        asm volatile("{.reg .pred q;\n setp.ne.u32 q, %2, 0;\n mov.b64 %0, 0;\n @q ld.global.nc.b64 %0, [%1];}" : "=l"(r) : "l"(p), "r"((uint32_t)c));
+        return r;
+    }
     static __device__ __forceinline__ void st(float *p, f32x2 v) { *reinterpret_cast<f32x2 *>(p) = v; }
 };
 template <> struct Pair<__nv_bfloat16> {
@@ -109,7 +117,11 @@ template <> struct Pair<__nv_bfloat16> {
         return pack2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
     }
     static __device__ __forceinline__ f32x2 lds(int a) { return widen(*reinterpret_cast<const uint32_t *>(g_smem + a)); }
-    static __device__ __forceinline__ f32x2 ldg(const __nv_bfloat16 *p) { return widen(__ldg(reinterpret_cast<const uint32_t *>(p))); }
+    static __device__ __forceinline__ f32x2 ldg_if(bool c, const __nv_bfloat16 *p) {
+        uint32_t r;
+        asm volatile("{.reg .pred q;\n setp.ne.u32 q, %2, 0;\n mov.b32 %0, 0;\n @q ld.global.nc.b32 %0, [%1];}" : "=r"(r) : "l"(p), "r"((uint32_t)c));
+        return widen(r);
+    }
     static __device__ __forceinline__ void st(__nv_bfloat16 *p, f32x2 v) {
         const float2 f = unpack2(v);
         uint32_t r;
@@ -245,7 +257,11 @@ __device__ __forceinline__ void slant_body(int base, int lstep, int pstep, int l
 constexpr int kMaxPairs = kMaxCC / 2;
 // Pairs of one line that share a group of lanes: all of them, or half where that leaves fewer lanes idle.
 __host__ __device__ constexpr int class_pairs(int m) { return 32 / m * m < 27 ? (m + 1) / 2 : m; }
-struct Class { int canon, n, full, entry[kMaxPairs]; };        // entry: pair | channels of it (1 low, 2 high) << 4; full: all are 3
+struct Class {
+    int canon, n, full;
+    int warp0, warps;                        // weight gradient: warps that work on it
+    int entry[kMaxPairs];
+};        // entry: pair | channels of it (1 low, 2 high) << 4; full: all are 3
 struct Tables {
     f32x2 w[32][kMaxPairs];                  // by stored tap (colliding taps summed) and pair
     f32x2 bias[kMaxPairs];
@@ -268,6 +284,14 @@ constexpr MergeTable make_merge() {
     return m;
 }
 static __device__ const MergeTable g_merge = make_merge();
+// Stored tap of each tap of a diagonal.
+struct DiagTable { int8_t at[kMaxTaps]; __device__ int operator[](int t) const { return at[t]; } };
+constexpr DiagTable make_diag() {
+    DiagTable d{};
+    for (int t = 0; t < kMaxTaps; t++) d.at[t] = (int8_t)(kCanonDw[2][t] + kHalf);
+    return d;
+}
+static __device__ const DiagTable g_diag_at = make_diag();
 
 // Weight of base tap t of channel c on canonical line id (0 when the kernel is shorter than the line).
 __device__ __forceinline__ float base_weight(const void *w, int wbf16, int c, int id, int t, const SegParams &p) {
@@ -330,6 +354,43 @@ __device__ __noinline__ void build_tables(Tables *tab, const SegParams &p, const
     __syncthreads();
 }
 
+// Weight gradient: the warps are dealt to the classes in proportion to their tasks' cost, so that a warp
+// keeps its accumulators for all items of a segment.  One thread.
+__device__ __noinline__ void deal_warps(Tables *tab, int imgs, int lenh, int lenw, int lt) {
+    float cost[12], total = 0.f;
+    int left = kWarps;
+#pragma unroll 1
+    for (int i = 0; i < tab->ncls; i++) {
+        const Class &c = tab->cls[i];
+        const int kind = kind_of(c.canon), fr = frame_of(c.canon), lpg = 32 / c.n;
+        const int plen = fr == FR_H ? lenw : lenh, llen = fr == FR_H ? lenh : lenw;
+        const int lines = kind == KIND_AXIS ? llen : kind == KIND_DIAG ? lenw + kTD - 1 : (llen + kSR - 1) / kSR;
+        const int bl = kind == KIND_SLANT ? kST : kind == KIND_AXIS ? lt : kTD;
+        const float each = kind == KIND_SLANT ? 4.6f : kind == KIND_DIAG ? 2.05f : lt == 28 ? 3.6f : 1.95f;
+        cost[i] = each * ((imgs * lines + lpg - 1) / lpg) * ((plen + bl - 1) / bl);
+        total += cost[i];
+    }
+#pragma unroll 1
+    for (int i = 0; i < tab->ncls; i++) {
+        tab->cls[i].warps = max(1, (int)(kWarps * cost[i] / total));
+        left -= tab->cls[i].warps;
+    }
+#pragma unroll 1
+    while (left != 0) {                      // one more to the slowest class, or one less from the fastest
+        int at = -1;
+#pragma unroll 1
+        for (int i = 0; i < tab->ncls; i++) {
+            const float v = cost[i] / tab->cls[i].warps, w = at < 0 ? 0.f : cost[at] / tab->cls[at].warps;
+            if (left > 0 ? (at < 0 || v > w) : (tab->cls[i].warps > 1 && (at < 0 || v < w))) at = i;
+        }
+        tab->cls[at].warps += left > 0 ? 1 : -1;
+        left += left > 0 ? -1 : 1;
+    }
+    int w = 0;
+#pragma unroll 1
+    for (int i = 0; i < tab->ncls; i++) { tab->cls[i].warp0 = w; w += tab->cls[i].warps; }
+}
+
 // Either channel of a pair, or both: predicated stores (branches would triple the code).
 template <typename T> __device__ __forceinline__ void store_pair(T *p, f32x2 v, int mask) {
     const float2 f = unpack2(v);
@@ -342,6 +403,14 @@ template <typename T> __device__ __forceinline__ void store_pair(T *p, f32x2 v, 
                      ::"l"(p), "f"(f.x), "f"(f.y), "r"(mask & 1), "r"(mask & 2) : "memory");
 }
 
+// The block's dy, zero past the last `left` positions of the line.
+template <typename T, int NO> __device__ __forceinline__ void load_line(const T *q, ptrdiff_t ps, f32x2 *O, int left) {
+#pragma unroll
+    for (int o = 0; o < NO; o++) {
+        O[o] = Pair<T>::ldg_if(o < left, q);
+        q += ps;
+    }
+}
 // `left` outputs of a line (at most NO), ps elements apart.
 template <typename T, int NO>
 __device__ __forceinline__ void store_line(T *q, ptrdiff_t ps, const f32x2 *O, int left, bool all, int mask) {
@@ -391,9 +460,9 @@ __device__ __forceinline__ Spot spot_of(const SegParams &p, long long at) {
     }
     return s;                                // one past the end
 }
-__device__ __forceinline__ bool first_segment(const SegParams &p, Segment &g, Spot &at, const Spot &end) {
+__device__ __forceinline__ bool first_segment(const SegParams &p, Segment &g, Spot &at, const Spot &end, int cta) {
     if (p.per_chunk) {
-        int b = blockIdx.x;
+        int b = cta;
         g.run = 0;
 #pragma unroll 1
         while (b >= p.run[g.run].nchunks * p.run[g.run].ctas) { b -= p.run[g.run].nchunks * p.run[g.run].ctas; g.run++; }
@@ -422,11 +491,13 @@ __device__ __forceinline__ bool first_segment(const SegParams &p, Segment &g, Sp
 }
 
 // R: reach of the taps (15, or 7 for kernels of up to 15 taps); LT: outputs of a thread along a line.
-template <typename T, int R, int LT>
+// WG = false: y = conv(x) + bias.  WG = true: y is dy, and each CTA leaves its share of the weight and bias
+// gradients of its chunks in `partial` ([slot][channel of the chunk][32], by stored tap, the bias last).
+template <typename T, int R, int LT, bool WG>
 __global__ void __launch_bounds__(kThreads, 1)
-seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ wv, const void *__restrict__ biasv, int wbf16,
-                const int8_t *__restrict__ chan, T *__restrict__ y, int *__restrict__ err_flag,
-                const __grid_constant__ SegParams p) {
+seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps dy_maps, const void *__restrict__ wv,
+           const void *__restrict__ biasv, int wbf16, const int8_t *__restrict__ chan, T *__restrict__ y,
+           float *__restrict__ partial, int *__restrict__ err_flag, const __grid_constant__ SegParams p) {
     char *sm = g_smem;
     constexpr int PB = Pair<T>::kBytes, RD = kCanonDh[2][kHalf - R];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -440,7 +511,7 @@ seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ w
         at = spot_of(p, p.total_cost * blockIdx.x / gridDim.x);
         end = spot_of(p, p.total_cost * (blockIdx.x + 1) / gridDim.x);
     }
-    bool more = first_segment(p, g, at, end);
+    bool more = first_segment(p, g, at, end, blockIdx.x);
     auto issue = [&](const Segment &g, int s, int buf) {          // item number s of the segment
         const SegGeo &ge = p.geo[p.run[g.run].geo];
         const int it = g.item(s), tiles = ge.nth * ge.ntw;
@@ -454,6 +525,8 @@ seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ w
         mbar_expect_tx(&full[buf], ge.tile_bytes);
         tma_load_4d(sm + p.off_tile + buf * ge.buf_bytes, &maps.m[p.run[g.run].geo], &full[buf],
                     (p.run[g.run].chunk0 + g.chunk) * p.CC, tw * ge.TW - ge.ow, th * ge.TH - ge.oh, n0);
+        // dy is read straight from global memory, each value once: have it in L2 by then
+        if (WG) tma_prefetch_4d(&dy_maps.m[p.run[g.run].geo], (p.run[g.run].chunk0 + g.chunk) * p.CC, tw * ge.TW, th * ge.TH, n0);
     };
     if (tid == 0) {
 #pragma unroll 1
@@ -466,10 +539,11 @@ seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ w
     bool ok = true;
     uint32_t phase = 0;                          // parity of each buffer's barrier
 #pragma unroll 1
-    for (; more; more = !p.per_chunk && first_segment(p, g, at, end)) {
+    for (; more; more = !p.per_chunk && first_segment(p, g, at, end, blockIdx.x)) {
         const SegGeo &ge = p.geo[p.run[g.run].geo];
         const int c0 = (p.run[g.run].chunk0 + g.chunk) * p.CC, tiles = ge.nth * ge.ntw, row_bytes = ge.P * p.px, px = p.px;
         const int nitems = g.count();
+        if (WG) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();                         // the previous segment is done with tables and buffers
         if (tid == 0) {
 #pragma unroll 1
@@ -480,7 +554,17 @@ seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ w
             if ((i & 15) * 4 < px)
                 *reinterpret_cast<float *>(sm + p.off_tile + ((i >> 4) + 1) * ge.buf_bytes - px + (i & 15) * 4) = 0.f;
         build_tables(tab, p, wv, biasv, wbf16, chan, c0);
-        int buf = 0;
+        int buf = 0, my_class = 0, stride = kWarps;
+        f32x2 Wg[kMaxTaps], dbias = 0;           // weight gradient: the warp's accumulators
+        if constexpr (WG) {
+            if (tid == 0) deal_warps(tab, ge.G, ge.TH, ge.TW, LT);
+            __syncthreads();
+            while (warp >= tab->cls[my_class].warp0 + tab->cls[my_class].warps) my_class++;
+            stride = tab->cls[my_class].warps;
+            turn = warp - tab->cls[my_class].warp0;
+#pragma unroll
+            for (int i = 0; i < kMaxTaps; i++) Wg[i] = 0;
+        }
 #pragma unroll 1
         for (int s = 0; s < nitems; s++) {
             const int it = g.item(s);
@@ -499,7 +583,7 @@ seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ w
             if (ok) ok = mbar_wait(&full[buf], phase >> buf & 1, err_flag);
             phase ^= 1u << buf;
 #pragma unroll 1
-            for (int ci = 0; ci < tab->ncls; ci++) {
+            for (int ci = WG ? my_class : 0; ci < (WG ? my_class + 1 : tab->ncls); ci++) {
                 const Class *cl = &tab->cls[ci];
                 const int id = cl->canon, np = cl->n, kind = kind_of(id), fr = frame_of(id);
                 const int lpg = 32 / np;                                            // lines per group of lanes
@@ -510,23 +594,18 @@ seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ w
                 const int ln = lane / np, entry = cl->entry[lane - ln * np], pair = entry & 15, mask = entry >> 4;
                 const bool all = cl->full;
                 int t = t0 + turn, ug = t / npb, pb = t - ug * npb;
-                const int dug = kWarps / npb, dpb = kWarps - dug * npb;
+                const int dug = stride / npb, dpb = stride - dug * npb;
                 turn -= t1 - t0;
 #pragma unroll 1
-                for (; t < t1; t += kWarps, turn += kWarps) {
+                for (; t < t1; t += stride, turn += stride) {
                     const int li = ug * lpg + ln, gi = ge.G == 1 ? (li >= nlines) : li / nlines, line = li - gi * nlines;
                     const bool act = ln < lpg && gi < imgs;
                     const int gt = tbuf + pair * PB + (act ? gi : 0) * ge.img_bytes;         // first output of the image
-                    f32x2 Wt[kMaxTaps];
-#pragma unroll
-                    for (int i = 0; i < kMaxTaps; i++) Wt[i] = tab->w[i][pair];
-                    const f32x2 bias = tab->bias[pair];
                     T *yi = y + ((size_t)(n0 + gi) * p.H + h0) * p.W * p.C + (size_t)w0 * p.C + c0 + 2 * pair;
                     const int p0 = pb * bl;
+                    auto task = [&](f32x2 (&Wt)[kMaxTaps], f32x2 bias) {
                     if (kind == KIND_SLANT) {
                         f32x2 O[kSR * kST];
-#pragma unroll
-                        for (int o = 0; o < kSR * kST; o++) O[o] = bias;
                         const int l0 = line * kSR;
                         const bool hf = fr == FR_H;
                         const int lstep = hf ? row_bytes : px, pstep = hf ? px : row_bytes;
@@ -534,46 +613,87 @@ seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ w
                         const int cut = hf ? ge.halo_h : ge.halo_w;
                         const int llo = (hf ? ge.plo_h : ge.plo_w) + 1 - cut, lhi = (hf ? ge.phi_h : ge.phi_w) - 1 + cut;
                         const int lzero = cut ? 0 : hf ? ge.plo_h : ge.phi_w;
-                        slant_body<T, R, false>(gt + p0 * pstep, lstep, pstep, l0, sgn_of(id), llo, lhi, lzero, (plo - p0) * pstep,
-                                                (phi - p0) * pstep, O, Wt);
                         const ptrdiff_t ls = hf ? (ptrdiff_t)p.W * p.C : p.C, ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
+                        T *yb = yi + (sgn_of(id) > 0 ? l0 : l0 + kSR - 1) * ls + p0 * ps;       // first of the block's lines
+                        const ptrdiff_t dls = sgn_of(id) > 0 ? ls : -ls;
+                        int left[kSR];
 #pragma unroll
-                        for (int r = 0; r < kSR; r++) {
-                            const int l = sgn_of(id) > 0 ? l0 + r : l0 + kSR - 1 - r;
-                            store_line<T, kST>(yi + l * ls + p0 * ps, ps, &O[r * kST], act && l < llen ? plen - p0 : 0, all, mask);
+                        for (int r = 0; r < kSR; r++) left[r] = act && (sgn_of(id) > 0 ? l0 + r : l0 + kSR - 1 - r) < llen ? plen - p0 : 0;
+                        if constexpr (WG) {
+#pragma unroll
+                            for (int r = 0; r < kSR; r++) load_line<T, kST>(yb + r * dls, ps, &O[r * kST], left[r]);
+                        } else {
+#pragma unroll
+                            for (int o = 0; o < kSR * kST; o++) O[o] = bias;
+                        }
+                        slant_body<T, R, WG>(gt + p0 * pstep, lstep, pstep, l0, sgn_of(id), llo, lhi, lzero, (plo - p0) * pstep,
+                                             (phi - p0) * pstep, O, Wt);
+                        if constexpr (WG) {
+#pragma unroll
+                            for (int o = 0; o < kSR * kST; o++) add2(dbias, O[o]);
+                        } else {
+#pragma unroll
+                            for (int r = 0; r < kSR; r++) store_line<T, kST>(yb + r * dls, ps, &O[r * kST], left[r], all, mask);
                         }
                     } else if (kind == KIND_AXIS) {
                         f32x2 O[LT];
-#pragma unroll
-                        for (int o = 0; o < LT; o++) O[o] = bias;
                         const bool hf = fr == FR_H;
                         const int step = hf ? px : row_bytes, base = gt + line * (hf ? row_bytes : px);
                         const bool cut = hf ? ge.halo_w : ge.halo_h;
-                        line_body<T, R, LT, false, false>(base + p0 * step, step, base + (hf ? ge.plo_w : ge.plo_h) * step,
-                                                          base + (hf ? ge.phi_w : ge.phi_h) * step, p0 > 0 || cut, p0 + LT < plen || cut,
-                                                          O, Wt);
                         const ptrdiff_t ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
-                        store_line<T, LT>(yi + line * (hf ? (ptrdiff_t)p.W * p.C : p.C) + p0 * ps, ps, O, act ? plen - p0 : 0, all, mask);
+                        T *yl = yi + line * (hf ? (ptrdiff_t)p.W * p.C : p.C) + p0 * ps;
+                        if constexpr (WG) load_line<T, LT>(yl, ps, O, act ? plen - p0 : 0);
+                        else {
+#pragma unroll
+                            for (int o = 0; o < LT; o++) O[o] = bias;
+                        }
+                        line_body<T, R, LT, false, WG>(base + p0 * step, step, base + (hf ? ge.plo_w : ge.plo_h) * step,
+                                                       base + (hf ? ge.phi_w : ge.phi_h) * step, p0 > 0 || cut, p0 + LT < plen || cut, O, Wt);
+                        if constexpr (WG) {
+#pragma unroll
+                            for (int o = 0; o < LT; o++) add2(dbias, O[o]);
+                        } else
+                            store_line<T, LT>(yl, ps, O, act ? plen - p0 : 0, all, mask);
                     } else {
                         f32x2 O[kTD];
-#pragma unroll
-                        for (int o = 0; o < kTD; o++) O[o] = bias;
                         const int dw = id == 2 ? -1 : 1, w = dw > 0 ? line - (kTD - 1) : line;
+                        T *yl = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
+                        const ptrdiff_t ps = ((ptrdiff_t)p.W + dw) * p.C;
+                        auto in = [&](int o) { return act && p0 + o < plen && (unsigned)(w + o * dw) < (unsigned)lenw; };
+                        if constexpr (WG) {
+                            const T *q = yl;
+#pragma unroll
+                            for (int o = 0; o < kTD; o++) { O[o] = Pair<T>::ldg_if(in(o), q); q += ps; }
+                        } else {
+#pragma unroll
+                            for (int o = 0; o < kTD; o++) O[o] = bias;
+                        }
                         // where the diagonal enters and leaves the tile (at the zeros around a whole map), from the block's first position
                         const int f = max(dw > 0 ? ge.plo_w - w : w - ge.phi_w, ge.plo_h - p0);
                         const int l = min(dw > 0 ? ge.phi_w - w : w - ge.plo_w, ge.phi_h - p0);
                         const int step = row_bytes + dw * px, a0 = gt + p0 * row_bytes + w * px;
-                        line_body<T, RD, kTD, true, false>(a0, step, a0 + f * step, a0 + l * step, p0 > 0 || ge.halo_h,
-                                                           p0 + kTD < plen || ge.halo_h, O, Wt);
-                        T *yl = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
-                        const ptrdiff_t ps = ((ptrdiff_t)p.W + dw) * p.C;
+                        line_body<T, RD, kTD, true, WG>(a0, step, a0 + f * step, a0 + l * step, p0 > 0 || ge.halo_h,
+                                                        p0 + kTD < plen || ge.halo_h, O, Wt);
+                        if constexpr (WG) {
 #pragma unroll
-                        for (int o = 0; o < kTD; o++) {
-                            if (act && p0 + o < plen && (unsigned)(w + o * dw) < (unsigned)lenw) {
-                                if (all) Pair<T>::st(yl, O[o]); else store_pair(yl, O[o], mask);
+                            for (int o = 0; o < kTD; o++) add2(dbias, O[o]);
+                        } else {
+#pragma unroll
+                            for (int o = 0; o < kTD; o++) {
+                                if (in(o)) {
+                                    if (all) Pair<T>::st(yl, O[o]); else store_pair(yl, O[o], mask);
+                                }
+                                yl += ps;
                             }
-                            yl += ps;
                         }
+                    }
+                    };
+                    if constexpr (WG) task(Wg, 0);
+                    else {
+                        f32x2 Wt[kMaxTaps];
+#pragma unroll
+                        for (int i = 0; i < kMaxTaps; i++) Wt[i] = tab->w[i][pair];
+                        task(Wt, tab->bias[pair]);
                     }
                     ug += dug;
                     pb += dpb;
@@ -587,6 +707,94 @@ seg_conv_kernel(const __grid_constant__ SegMaps maps, const void *__restrict__ w
             }
             if (++buf == ge.nbuf) buf = 0;
         }
+        if constexpr (WG) {
+            // lanes of a pair, then the warps of a class, each in a fixed order
+            const int np = tab->cls[my_class].n, ln = lane / np;
+            __syncthreads();
+            f32x2 *red = reinterpret_cast<f32x2 *>(sm + p.off_tile);         // [warp][32][kMaxPairs]
+            auto lanes = [&](f32x2 v) {
+#pragma unroll 1
+                for (int n = 32 / np; n > 1;) {
+                    const int half = (n + 1) / 2;
+                    const f32x2 u = __shfl_down_sync(~0u, v, half * np);
+                    if (ln + half < n) add2(v, u);
+                    n = half;
+                }
+                return v;
+            };
+            static_for<0, kMaxTaps + 1>([&](auto i_) {
+                constexpr int i = decltype(i_)::value;
+                const f32x2 v = lanes(i < kMaxTaps ? Wg[i < kMaxTaps ? i : 0] : dbias);
+                if (lane < np) red[(warp * 32 + i) * kMaxPairs + lane] = v;
+            });
+            __syncthreads();
+            const int slot = p.per_chunk ? (int)blockIdx.x : (int)blockIdx.x + p.run[g.run].chunk0 + g.chunk;
+#pragma unroll 1
+            for (int ci = 0; ci < tab->ncls; ci++) {
+                const Class &cl = tab->cls[ci];
+#pragma unroll 1
+                for (int i = tid; i < cl.n * 64; i += kThreads) {
+                    const int e = i >> 6, half = i >> 5 & 1, t = i & 31, entry = cl.entry[e];
+                    if (!(entry >> 4 >> half & 1)) continue;
+                    float sum = 0.f;
+#pragma unroll 1
+                    for (int w = cl.warp0; w < cl.warp0 + cl.warps; w++)
+                        sum += reinterpret_cast<const float *>(&red[(w * 32 + t) * kMaxPairs + e])[half];
+                    partial[((size_t)slot * p.CC + 2 * (entry & 15) + half) * 32 + t] = sum;
+                }
+            }
+        }
+    }
+}
+
+// Adds the shares of a chunk (one CTA each) in the order of the CTAs and writes the weight and bias gradients.
+static __global__ void __launch_bounds__(256)
+seg_wgrad_final_kernel(const float *__restrict__ partial, const int8_t *__restrict__ chan, void *__restrict__ dw, void *__restrict__ db,
+                       int out_bf16, int ctas, const __grid_constant__ SegParams p) {
+    __shared__ int slots[256], nslots;
+    const int chunk = blockIdx.x, tid = threadIdx.x;
+    bool has = false;                            // does CTA `tid` have a segment of this chunk?
+    int slot = tid;
+    if (tid < ctas) {
+        Segment g;
+        Spot at{0, 0, 0}, end{0, 0, 0};
+        if (!p.per_chunk) {
+            at = spot_of(p, p.total_cost * tid / ctas);
+            end = spot_of(p, p.total_cost * (tid + 1) / ctas);
+            slot = tid + chunk;
+        }
+        bool more = first_segment(p, g, at, end, tid);
+#pragma unroll 1
+        while (more && !has) {
+            has = p.run[g.run].chunk0 + g.chunk == chunk;
+            more = !p.per_chunk && first_segment(p, g, at, end, tid);
+        }
+    }
+    slots[tid] = has ? slot : -1;
+    __syncthreads();
+    if (tid == 0) {
+        int n = 0;
+#pragma unroll 1
+        for (int i = 0; i < ctas; i++)
+            if (slots[i] >= 0) slots[n++] = slots[i];
+        nslots = n;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int i = tid; i < p.CC * 32; i += 256) {
+        const int cc = i >> 5, c = chunk * p.CC + cc, k = i & 31;      // k: tap of the kernel, 31: the bias
+        if (c >= p.C || (k < 31 ? k >= p.K : db == nullptr)) continue;
+        int at = 31;
+        if (k < 31) {
+            const int id = chan[c], j = k - p.K / 2 + kHalf, t = rev_of(id) ? kMaxTaps - 1 - j : j, kind = kind_of(id);
+            at = kind == KIND_SLANT ? (t == 14 || t == 16 ? 15 : t) : kind == KIND_DIAG ? g_diag_at[t] : t;
+        }
+        float sum = 0.f;
+#pragma unroll 1
+        for (int n = 0; n < nslots; n++) sum += partial[((size_t)slots[n] * p.CC + cc) * 32 + at];
+        const size_t o = k < 31 ? (size_t)c * p.K + k : c;
+        void *out = k < 31 ? dw : db;
+        if (out_bf16) ((__nv_bfloat16 *)out)[o] = __float2bfloat16_rn(sum); else ((float *)out)[o] = sum;
     }
 }
 

@@ -53,4 +53,10 @@ bool seg_configure(const int8_t *chan, int N, int H, int W, int C, int K, int es
 cudaError_t seg_launch_conv(const SegConfig &cfg, const SegMaps &maps, const void *w, const void *bias, int wbf16,
                             const int8_t *chan, void *y, int flip, int identity, int *err_flag, cudaStream_t st);
 
+// Weight gradient (and bias gradient when db is not null): dw, db fp32, or bf16 when out_bf16 is set.
+// `partial`: seg_wgrad_bytes() of scratch.
+size_t seg_wgrad_bytes(const SegConfig &cfg);
+cudaError_t seg_launch_wgrad(const SegConfig &cfg, const SegMaps &maps, const SegMaps &dy_maps, const int8_t *chan, const void *dy,
+                             void *dw, void *db, int out_bf16, float *partial, int *err_flag, cudaStream_t st);
+
 }  // namespace o1d
