@@ -276,7 +276,7 @@ cudaError_t seg_launch_wgrad(const SegConfig &cfg, const SegMaps &maps, const Se
     Args a{&maps, &dy_maps, nullptr, nullptr, 0, chan, const_cast<void *>(dy), partial, err_flag, cfg.p, st};
     const cudaError_t e = cfg.esize == 4 ? launch_any<float, true>(cfg, a) : launch_any<__nv_bfloat16, true>(cfg, a);
     if (e != cudaSuccess) return e;
-    seg::seg_wgrad_final_kernel<<<ceil_div(cfg.p.C, cfg.p.CC), 256, 0, st>>>(partial, chan, dw, db, out_bf16, cfg.grid, cfg.p);
+    seg::seg_wgrad_final_kernel<<<dim3(ceil_div(cfg.p.C, cfg.p.CC), ceil_div(cfg.p.CC * 32, 256)), 256, 0, st>>>(partial, chan, dw, db, out_bf16, cfg.grid, cfg.p);
     return cudaGetLastError();
 }
 

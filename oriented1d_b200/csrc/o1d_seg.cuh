@@ -613,16 +613,18 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                         const int cut = hf ? ge.halo_h : ge.halo_w;
                         const int llo = (hf ? ge.plo_h : ge.plo_w) + 1 - cut, lhi = (hf ? ge.phi_h : ge.phi_w) - 1 + cut;
                         const int lzero = cut ? 0 : hf ? ge.plo_h : ge.phi_w;
-                        const ptrdiff_t ls = hf ? (ptrdiff_t)p.W * p.C : p.C, ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
-                        T *yb = yi + (sgn_of(id) > 0 ? l0 : l0 + kSR - 1) * ls + p0 * ps;       // first of the block's lines
-                        const ptrdiff_t dls = sgn_of(id) > 0 ? ls : -ls;
-                        int left[kSR];
+                        // line r of the block, `left` positions of it (addresses are formed where they are used: kept
+                        // over the body they cost registers, 10 % of the time)
+                        auto each_line = [&](auto &&f) {
+                            const ptrdiff_t ls = hf ? (ptrdiff_t)p.W * p.C : p.C, ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
 #pragma unroll
-                        for (int r = 0; r < kSR; r++) left[r] = act && (sgn_of(id) > 0 ? l0 + r : l0 + kSR - 1 - r) < llen ? plen - p0 : 0;
-                        if constexpr (WG) {
-#pragma unroll
-                            for (int r = 0; r < kSR; r++) load_line<T, kST>(yb + r * dls, ps, &O[r * kST], left[r]);
-                        } else {
+                            for (int r = 0; r < kSR; r++) {
+                                const int l = sgn_of(id) > 0 ? l0 + r : l0 + kSR - 1 - r;
+                                f(r, yi + l * ls + p0 * ps, ps, act && l < llen ? plen - p0 : 0);
+                            }
+                        };
+                        if constexpr (WG) each_line([&](int r, T *q, ptrdiff_t ps, int left) { load_line<T, kST>(q, ps, &O[r * kST], left); });
+                        else {
 #pragma unroll
                             for (int o = 0; o < kSR * kST; o++) O[o] = bias;
                         }
@@ -631,18 +633,18 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                         if constexpr (WG) {
 #pragma unroll
                             for (int o = 0; o < kSR * kST; o++) add2(dbias, O[o]);
-                        } else {
-#pragma unroll
-                            for (int r = 0; r < kSR; r++) store_line<T, kST>(yb + r * dls, ps, &O[r * kST], left[r], all, mask);
-                        }
+                        } else
+                            each_line([&](int r, T *q, ptrdiff_t ps, int left) { store_line<T, kST>(q, ps, &O[r * kST], left, all, mask); });
                     } else if (kind == KIND_AXIS) {
                         f32x2 O[LT];
                         const bool hf = fr == FR_H;
                         const int step = hf ? px : row_bytes, base = gt + line * (hf ? row_bytes : px);
                         const bool cut = hf ? ge.halo_w : ge.halo_h;
-                        const ptrdiff_t ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
-                        T *yl = yi + line * (hf ? (ptrdiff_t)p.W * p.C : p.C) + p0 * ps;
-                        if constexpr (WG) load_line<T, LT>(yl, ps, O, act ? plen - p0 : 0);
+                        auto place = [&](auto &&f) {
+                            const ptrdiff_t ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
+                            f(yi + line * (hf ? (ptrdiff_t)p.W * p.C : p.C) + p0 * ps, ps);
+                        };
+                        if constexpr (WG) place([&](T *q, ptrdiff_t ps) { load_line<T, LT>(q, ps, O, act ? plen - p0 : 0); });
                         else {
 #pragma unroll
                             for (int o = 0; o < LT; o++) O[o] = bias;
@@ -653,15 +655,14 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
 #pragma unroll
                             for (int o = 0; o < LT; o++) add2(dbias, O[o]);
                         } else
-                            store_line<T, LT>(yl, ps, O, act ? plen - p0 : 0, all, mask);
+                            place([&](T *q, ptrdiff_t ps) { store_line<T, LT>(q, ps, O, act ? plen - p0 : 0, all, mask); });
                     } else {
                         f32x2 O[kTD];
                         const int dw = id == 2 ? -1 : 1, w = dw > 0 ? line - (kTD - 1) : line;
-                        T *yl = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
-                        const ptrdiff_t ps = ((ptrdiff_t)p.W + dw) * p.C;
                         auto in = [&](int o) { return act && p0 + o < plen && (unsigned)(w + o * dw) < (unsigned)lenw; };
                         if constexpr (WG) {
-                            const T *q = yl;
+                            const T *q = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
+                            const ptrdiff_t ps = ((ptrdiff_t)p.W + dw) * p.C;
 #pragma unroll
                             for (int o = 0; o < kTD; o++) { O[o] = Pair<T>::ldg_if(in(o), q); q += ps; }
                         } else {
@@ -678,6 +679,8 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
 #pragma unroll
                             for (int o = 0; o < kTD; o++) add2(dbias, O[o]);
                         } else {
+                            T *yl = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
+                            const ptrdiff_t ps = ((ptrdiff_t)p.W + dw) * p.C;
 #pragma unroll
                             for (int o = 0; o < kTD; o++) {
                                 if (in(o)) {
@@ -712,21 +715,23 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
             const int np = tab->cls[my_class].n, ln = lane / np;
             __syncthreads();
             f32x2 *red = reinterpret_cast<f32x2 *>(sm + p.off_tile);         // [warp][32][kMaxPairs]
-            auto lanes = [&](f32x2 v) {
 #pragma unroll 1
-                for (int n = 32 / np; n > 1;) {
-                    const int half = (n + 1) / 2;
+            for (int n = 32 / np; n > 1;) {
+                const int half = (n + 1) / 2;
+                const bool take = ln + half < n;
+                static_for<0, kMaxTaps + 1>([&](auto i_) {
+                    constexpr int i = decltype(i_)::value;
+                    f32x2 &v = i < kMaxTaps ? Wg[i < kMaxTaps ? i : 0] : dbias;
                     const f32x2 u = __shfl_down_sync(~0u, v, half * np);
-                    if (ln + half < n) add2(v, u);
-                    n = half;
-                }
-                return v;
-            };
-            static_for<0, kMaxTaps + 1>([&](auto i_) {
-                constexpr int i = decltype(i_)::value;
-                const f32x2 v = lanes(i < kMaxTaps ? Wg[i < kMaxTaps ? i : 0] : dbias);
-                if (lane < np) red[(warp * 32 + i) * kMaxPairs + lane] = v;
-            });
+                    if (take) add2(v, u);
+                });
+                n = half;
+            }
+            if (lane < np)
+                static_for<0, kMaxTaps + 1>([&](auto i_) {
+                    constexpr int i = decltype(i_)::value;
+                    red[(warp * 32 + i) * kMaxPairs + lane] = i < kMaxTaps ? Wg[i < kMaxTaps ? i : 0] : dbias;
+                });
             __syncthreads();
             const int slot = p.per_chunk ? (int)blockIdx.x : (int)blockIdx.x + p.run[g.run].chunk0 + g.chunk;
 #pragma unroll 1
@@ -781,7 +786,7 @@ seg_wgrad_final_kernel(const float *__restrict__ partial, const int8_t *__restri
     }
     __syncthreads();
 #pragma unroll 1
-    for (int i = tid; i < p.CC * 32; i += 256) {
+    for (int i = blockIdx.y * 256 + tid; i < p.CC * 32; i += gridDim.y * 256) {
         const int cc = i >> 5, c = chunk * p.CC + cc, k = i & 31;      // k: tap of the kernel, 31: the bias
         if (c >= p.C || (k < 31 ? k >= p.K : db == nullptr)) continue;
         int at = 31;
@@ -790,7 +795,7 @@ seg_wgrad_final_kernel(const float *__restrict__ partial, const int8_t *__restri
             at = kind == KIND_SLANT ? (t == 14 || t == 16 ? 15 : t) : kind == KIND_DIAG ? g_diag_at[t] : t;
         }
         float sum = 0.f;
-#pragma unroll 1
+#pragma unroll 8
         for (int n = 0; n < nslots; n++) sum += partial[((size_t)slots[n] * p.CC + cc) * 32 + at];
         const size_t o = k < 31 ? (size_t)c * p.K + k : c;
         void *out = k < 31 ? dw : db;
