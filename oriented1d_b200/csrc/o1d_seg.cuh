@@ -672,8 +672,10 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                         // where the diagonal enters and leaves the tile (at the zeros around a whole map), from the block's first position
                         const int f = max(dw > 0 ? ge.plo_w - w : w - ge.phi_w, ge.plo_h - p0);
                         const int l = min(dw > 0 ? ge.phi_w - w : w - ge.plo_w, ge.phi_h - p0);
-                        const int step = row_bytes + dw * px, a0 = gt + p0 * row_bytes + w * px;
-                        line_body<T, RD, kTD, true, WG>(a0, step, a0 + f * step, a0 + l * step, p0 > 0 || ge.halo_h,
+                        // (a diagonal that misses the tile reads its first row, zeros around a whole map)
+                        const bool miss = f > l;
+                        const int step = row_bytes + dw * px, a0 = miss ? gt + ge.plo_h * row_bytes : gt + p0 * row_bytes + w * px;
+                        line_body<T, RD, kTD, true, WG>(a0, step, miss ? a0 : a0 + f * step, miss ? a0 : a0 + l * step, p0 > 0 || ge.halo_h,
                                                         p0 + kTD < plen || ge.halo_h, O, Wt);
                         if constexpr (WG) {
 #pragma unroll
