@@ -204,7 +204,8 @@ int o1d_wgrad_static(const void *dy, const void *x,
  * (models/convnext.py:28-56 LayerNorm, :183-189 stem LayerNorm+GELU, :309 block norm; the
  * reference calls F.layer_norm / F.gelu).  x, y: [rows, C] fp32 or bf16; gamma, beta: [C]
  * fp32; statistics in fp32, biased variance.  C must be a multiple of 4 (fp32) / 8 (bf16)
- * and at most 1024 (fp32) / 2048 (bf16).  Forward only. */
+ * and at most 1024 (fp32) / 2048 (bf16).  Forward only.  `gelu` is a flag word here and in the
+ * backward: bit 0 = GELU, O1D_FLAG_PARAMS_BF16 = gamma, beta (and dgamma, dbeta) are bf16. */
 int o1d_layernorm_cl(const void *x, const float *gamma, const float *beta, void *y,
                      long long rows, int C, float eps, int dtype, int gelu, void *stream);
 
@@ -223,7 +224,8 @@ int o1d_layernorm_cl_bwd(const void *x, const void *dy, const float *gamma, cons
 /* Column sums of a channels-last matrix, out[c] = sum_r x[r, c] in fp32: the bias gradient that
  * autograd forms for the Linear layers on either side of the convolution in a block
  * (models/convnext.py:298-300,310,312).  x [rows, C] fp32 or bf16, C a multiple of 4 / 8; summed in
- * a fixed order.  workspace: o1d_colsum_workspace_bytes(rows, C, dtype) bytes, uninitialised. */
+ * a fixed order.  workspace: o1d_colsum_workspace_bytes(rows, C, dtype) bytes, uninitialised.
+ * dtype | O1D_FLAG_PARAMS_BF16: out is bf16. */
 size_t o1d_colsum_workspace_bytes(long long rows, int C, int dtype);
 int o1d_colsum(const void *x, float *out, void *workspace, size_t workspace_bytes, long long rows, int C,
                int dtype, void *stream);
@@ -232,7 +234,7 @@ int o1d_colsum(const void *x, float *out, void *workspace, size_t workspace_byte
  * tensor with Cin <= 4 channels, y channels-last with Cout (a multiple of 8) channels: the
  * `x.permute(0,2,3,1)` + `nn.Linear(in_chans, 64)` that opens the reference's 1D stem
  * (models/convnext.py:143,170-176), in one pass.  x, y fp32 or bf16; w [Cout,Cin], bias [Cout]
- * (or NULL) fp32.  Forward only. */
+ * (or NULL) fp32, or bf16 with dtype | O1D_FLAG_PARAMS_BF16.  Forward only. */
 int o1d_pointwise_in(const void *x, const float *w, const float *bias, void *y,
                      int N, int Cin, long long HW, int Cout, int dtype, void *stream);
 

@@ -78,7 +78,24 @@ def _load() -> ctypes.CDLL:
     return lib
 
 
+def _load_ext():
+    """The native tensor front end (csrc/o1d_torch.cpp), on the library loaded above."""
+    import importlib.util
+    import torch  # noqa: F401  (its libraries must be in the process first)
+    if _build.ext_stale():
+        try:
+            _build.build_ext()
+        except Exception as e:
+            raise RuntimeError(f"_o1d_torch.so is missing or stale and could not be rebuilt ({e}); "
+                               "run `python -m oriented1d_b200.build`") from e
+    spec = importlib.util.spec_from_file_location("_o1d_torch", _build.EXT)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
 lib = _load()
+ext = _load_ext()
 
 
 def check(status: int, what: str = "o1d") -> None:
@@ -92,3 +109,6 @@ def check(status: int, what: str = "o1d") -> None:
     if status == 1:
         raise ValueError(f"{what}: {msg}")
     raise O1dError(f"{what}: {msg}")
+
+
+ext.set_check(check)

@@ -978,12 +978,13 @@ int o1d_wgrad_static(const void *dy, const void *x, const void *plan_host, const
 
 namespace {
 template <typename T, int G, int VPL>
-int launch_ln(const void *x, const float *gamma, const float *beta, void *y, int64_t rows, int C, float eps, int gelu,
+int launch_ln(const void *x, const void *gamma, const void *beta, void *y, int64_t rows, int C, float eps, int flags,
               cudaStream_t st, const DeviceInfo &d) {
     const int64_t groups = (rows * G + kLnThreads - 1) / kLnThreads;
     const int64_t cap = (int64_t)d.sms * 16;
     const int grid = (int)(groups < cap ? (groups > 0 ? groups : 1) : cap);
-    layernorm_cl_kernel<T, G, VPL><<<grid, kLnThreads, 0, st>>>((const T *)x, gamma, beta, (T *)y, rows, C, eps, gelu);
+    layernorm_cl_kernel<T, G, VPL><<<grid, kLnThreads, 0, st>>>((const T *)x, gamma, beta, (flags & O1D_FLAG_PARAMS_BF16) != 0, (T *)y, rows, C, eps,
+                                                                flags & 1);
     O1D_CUDA(cudaGetLastError());
     return O1D_OK;
 }
@@ -994,28 +995,29 @@ inline int ln_bwd_grid(int64_t rows, int G, int sms) {
     return (int)(groups < cap ? (groups > 0 ? groups : 1) : cap);
 }
 template <typename T, int G, int VPL>
-int launch_ln_bwd(const void *x, const void *dy, const float *gamma, const float *beta, void *dx, float *dgamma,
-                  float *dbeta, float *partial, int64_t rows, int C, float eps, int gelu, cudaStream_t st,
+int launch_ln_bwd(const void *x, const void *dy, const void *gamma, const void *beta, void *dx, void *dgamma,
+                  void *dbeta, float *partial, int64_t rows, int C, float eps, int flags, cudaStream_t st,
                   const DeviceInfo &d) {
     const int grid = ln_bwd_grid(rows, G, d.sms);
     const int smem = (kLnThreads / 32) * 2 * C * (int)sizeof(float);
-    if (gelu) {
+    const int pbf16 = (flags & O1D_FLAG_PARAMS_BF16) != 0;
+    if (flags & 1) {
         auto kern = layernorm_cl_bwd_kernel<T, G, VPL, true>;
         if (smem > 48 * 1024) O1D_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kern<<<grid, kLnThreads, smem, st>>>((const T *)x, (const T *)dy, gamma, beta, (T *)dx, partial, rows, C, eps);
+        kern<<<grid, kLnThreads, smem, st>>>((const T *)x, (const T *)dy, gamma, beta, pbf16, (T *)dx, partial, rows, C, eps);
     } else {
         auto kern = layernorm_cl_bwd_kernel<T, G, VPL, false>;
         if (smem > 48 * 1024) O1D_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kern<<<grid, kLnThreads, smem, st>>>((const T *)x, (const T *)dy, gamma, beta, (T *)dx, partial, rows, C, eps);
+        kern<<<grid, kLnThreads, smem, st>>>((const T *)x, (const T *)dy, gamma, beta, pbf16, (T *)dx, partial, rows, C, eps);
     }
     O1D_CUDA(cudaGetLastError());
-    layernorm_cl_bwd_final_kernel<<<ceil_div(2 * C, 32), dim3(32, 8), 0, st>>>(partial, dgamma, dbeta, grid, C);
+    layernorm_cl_bwd_final_kernel<<<ceil_div(2 * C, 32), dim3(32, 8), 0, st>>>(partial, dgamma, dbeta, pbf16, grid, C);
     O1D_CUDA(cudaGetLastError());
     return O1D_OK;
 }
 template <typename T>
-int dispatch_ln_bwd(const void *x, const void *dy, const float *gamma, const float *beta, void *dx, float *dgamma,
-                    float *dbeta, float *partial, int64_t rows, int C, float eps, int gelu, cudaStream_t st,
+int dispatch_ln_bwd(const void *x, const void *dy, const void *gamma, const void *beta, void *dx, void *dgamma,
+                    void *dbeta, float *partial, int64_t rows, int C, float eps, int gelu, cudaStream_t st,
                     const DeviceInfo &d) {
     const int nvec = C / (16 / (int)sizeof(T));
 #define O1D_LNB(G, V) launch_ln_bwd<T, G, V>(x, dy, gamma, beta, dx, dgamma, dbeta, partial, rows, C, eps, gelu, st, d)
@@ -1028,7 +1030,7 @@ int dispatch_ln_bwd(const void *x, const void *dy, const float *gamma, const flo
     return O1D_ERR_UNSUPPORTED;
 }
 template <typename T>
-int dispatch_ln(const void *x, const float *gamma, const float *beta, void *y, int64_t rows, int C, float eps,
+int dispatch_ln(const void *x, const void *gamma, const void *beta, void *y, int64_t rows, int C, float eps,
                 int gelu, cudaStream_t st, const DeviceInfo &d) {
     const int nvec = C / (16 / (int)sizeof(T));
     if (nvec <= 8) return launch_ln<T, 8, 1>(x, gamma, beta, y, rows, C, eps, gelu, st, d);
@@ -1068,7 +1070,7 @@ size_t o1d_layernorm_cl_bwd_workspace_bytes(long long rows, int C) {
 int o1d_layernorm_cl_bwd(const void *x, const void *dy, const float *gamma, const float *beta, void *dx, float *dgamma,
                          float *dbeta, void *workspace, size_t workspace_bytes, long long rows, int C, float eps,
                          int dtype, int gelu, void *stream) {
-    if (!x || !dy || !gamma || !dx || !dgamma || !dbeta || (gelu && !beta) || rows <= 0 || C <= 0 ||
+    if (!x || !dy || !gamma || !dx || !dgamma || !dbeta || ((gelu & 1) && !beta) || rows <= 0 || C <= 0 ||
         (dtype != O1D_F32 && dtype != O1D_BF16))
         return O1D_ERR_INVALID;
     const int ve = dtype == O1D_F32 ? 4 : 8;
@@ -1128,6 +1130,8 @@ size_t o1d_colsum_workspace_bytes(long long rows, int C, int dtype) {
 
 int o1d_colsum(const void *x, float *out, void *workspace, size_t workspace_bytes, long long rows, int C, int dtype,
                void *stream) {
+    const int pbf16 = (dtype & O1D_FLAG_PARAMS_BF16) != 0;
+    dtype &= ~O1D_FLAG_PARAMS_BF16;
     if (!x || !out || rows <= 0 || C <= 0 || (dtype != O1D_F32 && dtype != O1D_BF16)) return O1D_ERR_INVALID;
     const int ve = dtype == O1D_F32 ? 4 : 8;
     if (C % ve != 0 || ((uintptr_t)x & 15)) return O1D_ERR_UNSUPPORTED;
@@ -1140,13 +1144,15 @@ int o1d_colsum(const void *x, float *out, void *workspace, size_t workspace_byte
     if (dtype == O1D_F32) launch_colsum<float>(x, (float *)workspace, rows, C, slices, st);
     else launch_colsum<__nv_bfloat16>(x, (float *)workspace, rows, C, slices, st);
     O1D_CUDA(cudaGetLastError());
-    colsum_final_kernel<<<ceil_div(C, 32), dim3(32, 8), 0, st>>>((const float *)workspace, out, slices, C);
+    colsum_final_kernel<<<ceil_div(C, 32), dim3(32, 8), 0, st>>>((const float *)workspace, out, pbf16, slices, C);
     O1D_CUDA(cudaGetLastError());
     return O1D_OK;
 }
 
 int o1d_pointwise_in(const void *x, const float *w, const float *bias, void *y, int N, int Cin, long long HW,
                      int Cout, int dtype, void *stream) {
+    const int pbf16 = (dtype & O1D_FLAG_PARAMS_BF16) != 0;
+    dtype &= ~O1D_FLAG_PARAMS_BF16;
     if (!x || !w || !y || N <= 0 || HW <= 0 || Cin <= 0 || Cout <= 0 || (dtype != O1D_F32 && dtype != O1D_BF16))
         return O1D_ERR_INVALID;
     if (Cin > 4 || Cout % 8 != 0 || HW > 0x7fffffffLL || ((uintptr_t)y & 15)) return O1D_ERR_UNSUPPORTED;
@@ -1157,7 +1163,7 @@ int o1d_pointwise_in(const void *x, const float *w, const float *bias, void *y, 
     const long long blocks = (npix + per_block - 1) / per_block;
     if (blocks > 0x7fffffffLL) return O1D_ERR_UNSUPPORTED;
 #define O1D_PW(T, CIN)                                                                                     \
-    pointwise_in_kernel<T, CIN><<<(unsigned)blocks, kPointwiseThreads, 0, st>>>((const T *)x, w, bias, (T *)y, npix, \
+    pointwise_in_kernel<T, CIN><<<(unsigned)blocks, kPointwiseThreads, 0, st>>>((const T *)x, w, bias, pbf16, (T *)y, npix, \
                                                                                 (int)HW, Cout)
     if (dtype == O1D_F32) {
         switch (Cin) { case 1: O1D_PW(float, 1); break; case 2: O1D_PW(float, 2); break;

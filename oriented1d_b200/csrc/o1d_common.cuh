@@ -75,6 +75,14 @@ __device__ __forceinline__ float ld(const __nv_bfloat16 *p) {
 __device__ __forceinline__ void st(float *p, float v) { *p = v; }
 __device__ __forceinline__ void st(__nv_bfloat16 *p, float v) { *p = __float2bfloat16_rn(v); }
 
+// Element i of a parameter vector stored in fp32, or in bf16 when `bf16` is set.
+__device__ __forceinline__ float ld_param(const void *p, size_t i, int bf16) {
+    return bf16 ? __bfloat162float(static_cast<const __nv_bfloat16 *>(p)[i]) : __ldg(static_cast<const float *>(p) + i);
+}
+__device__ __forceinline__ void st_param(void *p, size_t i, int bf16, float v) {
+    if (bf16) static_cast<__nv_bfloat16 *>(p)[i] = __float2bfloat16_rn(v); else static_cast<float *>(p)[i] = v;
+}
+
 // Index of element (n, c, h, w) in an [N,C,H,W] tensor stored NCHW (LAYOUT 0) or NHWC (1).
 template <int LAYOUT>
 __device__ __forceinline__ int64_t at(int n, int c, int h, int w, int C, int H, int W) {

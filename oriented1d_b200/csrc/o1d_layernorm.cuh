@@ -20,7 +20,7 @@ __device__ __forceinline__ float gelu_erf(float v) { return 0.5f * v * (1.f + er
 // G lanes per row, VPL vectors per lane (row length C <= G * VPL * VE, C % VE == 0)
 template <typename T, int G, int VPL>
 __global__ void __launch_bounds__(kLnThreads)
-layernorm_cl_kernel(const T *__restrict__ x, const float *__restrict__ gamma, const float *__restrict__ beta,
+layernorm_cl_kernel(const T *__restrict__ x, const void *__restrict__ gamma, const void *__restrict__ beta, int pbf16,
                     T *__restrict__ y, int64_t rows, int C, float eps, int gelu) {
     constexpr int VE = GVec<T>::N;
     const int lane_in_group = threadIdx.x % G;
@@ -34,8 +34,8 @@ layernorm_cl_kernel(const T *__restrict__ x, const float *__restrict__ gamma, co
         const int vi = lane_in_group + v * G;
 #pragma unroll
         for (int j = 0; j < VE; j++) {
-            g[v][j] = (vi < nvec) ? __ldg(gamma + vi * VE + j) : 0.f;
-            b[v][j] = (vi < nvec) ? __ldg(beta + vi * VE + j) : 0.f;
+            g[v][j] = (vi < nvec) ? ld_param(gamma, vi * VE + j, pbf16) : 0.f;
+            b[v][j] = (vi < nvec) ? ld_param(beta, vi * VE + j, pbf16) : 0.f;
         }
     }
     const float inv_c = 1.f / (float)C;
@@ -99,8 +99,8 @@ layernorm_cl_kernel(const T *__restrict__ x, const float *__restrict__ gamma, co
 // GELU output and is first multiplied by GELU'(xhat * gamma + beta).
 template <typename T, int G, int VPL, bool GELU>
 __global__ void __launch_bounds__(kLnThreads)
-layernorm_cl_bwd_kernel(const T *__restrict__ x, const T *__restrict__ dy, const float *__restrict__ gamma,
-                        const float *__restrict__ beta, T *__restrict__ dx, float *__restrict__ partial, int64_t rows,
+layernorm_cl_bwd_kernel(const T *__restrict__ x, const T *__restrict__ dy, const void *__restrict__ gamma,
+                        const void *__restrict__ beta, int pbf16, T *__restrict__ dx, float *__restrict__ partial, int64_t rows,
                         int C, float eps) {
     extern __shared__ float ln_red[];                 // [warps][2][C]
     constexpr int VE = GVec<T>::N;
@@ -114,8 +114,8 @@ layernorm_cl_bwd_kernel(const T *__restrict__ x, const T *__restrict__ dy, const
         const int vi = lane_in_group + v * G;
 #pragma unroll
         for (int j = 0; j < VE; j++) {
-            g[v][j] = (vi < nvec) ? __ldg(gamma + vi * VE + j) : 0.f;
-            if (GELU) bt[GELU ? v : 0][j] = (vi < nvec) ? __ldg(beta + vi * VE + j) : 0.f;
+            g[v][j] = (vi < nvec) ? ld_param(gamma, vi * VE + j, pbf16) : 0.f;
+            if (GELU) bt[GELU ? v : 0][j] = (vi < nvec) ? ld_param(beta, vi * VE + j, pbf16) : 0.f;
             sg[v][j] = 0.f; sb[v][j] = 0.f;
         }
     }
@@ -229,8 +229,8 @@ layernorm_cl_bwd_kernel(const T *__restrict__ x, const T *__restrict__ dy, const
 // dgamma[c] = sum over CTAs of partial[cta][0][c], dbeta likewise from partial[cta][1][c].  Block (32, 8):
 // thread (x, y) adds the CTAs congruent to y modulo 8 for one column, the eight sums are then added in
 // order of y: a fixed order, with an eighth of the dependent loads per thread.
-__global__ void layernorm_cl_bwd_final_kernel(const float *__restrict__ partial, float *__restrict__ dgamma,
-                                              float *__restrict__ dbeta, int ctas, int C) {
+__global__ void layernorm_cl_bwd_final_kernel(const float *__restrict__ partial, void *__restrict__ dgamma,
+                                              void *__restrict__ dbeta, int pbf16, int ctas, int C) {
     __shared__ float part[8][33];
     const int e = blockIdx.x * 32 + threadIdx.x;
     float s = 0.f;
@@ -242,7 +242,7 @@ __global__ void layernorm_cl_bwd_final_kernel(const float *__restrict__ partial,
         float t = 0.f;
 #pragma unroll
         for (int y = 0; y < 8; y++) t += part[y][threadIdx.x];
-        if (e < C) dgamma[e] = t; else dbeta[e - C] = t;
+        st_param(e < C ? dgamma : dbeta, e < C ? e : e - C, pbf16, t);
     }
 }
 

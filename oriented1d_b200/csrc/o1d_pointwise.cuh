@@ -19,7 +19,7 @@ constexpr int kPointwisePasses = 8;      // pixels per thread
 // registers while it walks kPointwisePasses pixels.
 template <typename T, int CIN>
 __global__ void __launch_bounds__(kPointwiseThreads)
-pointwise_in_kernel(const T *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
+pointwise_in_kernel(const T *__restrict__ x, const void *__restrict__ w, const void *__restrict__ b, int pbf16,
                     T *__restrict__ y, long long npix, int HW, int Cout) {
     const int groups = Cout / 8;
     const int ppp = kPointwiseThreads / groups;            // pixels per pass of the block
@@ -28,9 +28,9 @@ pointwise_in_kernel(const T *__restrict__ x, const float *__restrict__ w, const 
     float wr[8][CIN], br[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-        br[j] = b ? __ldg(b + g * 8 + j) : 0.f;
+        br[j] = b ? ld_param(b, g * 8 + j, pbf16) : 0.f;
 #pragma unroll
-        for (int c = 0; c < CIN; c++) wr[j][c] = __ldg(w + (g * 8 + j) * CIN + c);
+        for (int c = 0; c < CIN; c++) wr[j][c] = ld_param(w, (g * 8 + j) * CIN + c, pbf16);
     }
     const long long first = (long long)blockIdx.x * ppp * kPointwisePasses + lp;
 #pragma unroll 2
@@ -131,7 +131,7 @@ colsum_partial_kernel(const T *__restrict__ x, float *__restrict__ partial, int6
 }
 
 // out[c] = sum over slices (in a fixed order) of partial[slice][c].  Block (32, 8) as in the LayerNorm backward.
-__global__ void colsum_final_kernel(const float *__restrict__ partial, float *__restrict__ out, int slices, int C) {
+__global__ void colsum_final_kernel(const float *__restrict__ partial, void *__restrict__ out, int pbf16, int slices, int C) {
     __shared__ float part[8][33];
     const int c = blockIdx.x * 32 + threadIdx.x;
     float s = 0.f;
@@ -143,7 +143,7 @@ __global__ void colsum_final_kernel(const float *__restrict__ partial, float *__
         float t = 0.f;
 #pragma unroll
         for (int y = 0; y < 8; y++) t += part[y][threadIdx.x];
-        out[c] = t;
+        st_param(out, c, pbf16, t);
     }
 }
 

@@ -30,6 +30,15 @@ from . import ops
 __all__ = ["DepthwiseOrientedConv1d", "get_dwoconv1d_kernel", "oriented_dwconv1d_get_module_from_params"]
 
 
+def _via_nhwc(x, plan, stride) -> bool:
+    """Does an NCHW tensor go through its NHWC form?  Where that form has a fast path."""
+    if not x.is_cuda or x.dim() != 4:
+        return False
+    N, C, H, W = x.shape
+    return (ops.uses_tiled(plan, N, H, W, stride, True, x.dtype)
+            and not ops.uses_tiled(plan, N, H, W, stride, False, x.dtype))
+
+
 class _DepthwiseOrientedConv1d(torch.autograd.Function):
     """Counterpart of the reference's autograd function (dwoconv1d.py:18-69).
 
@@ -43,11 +52,7 @@ class _DepthwiseOrientedConv1d(torch.autograd.Function):
         x = x.contiguous()
         ctx.set_materialize_grads(False)
         ctx.gelu_input = gelu_input
-        via_nhwc = False
-        if not nhwc and not gelu_input and x.is_cuda and x.dim() == 4:
-            N, C, H, W = x.shape
-            via_nhwc = (ops.uses_tiled(plan, N, H, W, stride, True, x.dtype)
-                        and not ops.uses_tiled(plan, N, H, W, stride, False, x.dtype))
+        via_nhwc = not nhwc and not gelu_input and _via_nhwc(x, plan, stride)
         ctx.plan, ctx.stride, ctx.nhwc, ctx.add_identity = plan, stride, nhwc, add_identity
         ctx.via_nhwc = via_nhwc
         ctx.has_bias = bias is not None
@@ -81,10 +86,10 @@ class _DepthwiseOrientedConv1d(torch.autograd.Function):
                 dx = ops.nhwc_to_nchw(dx)
         need_db = ctx.has_bias and ctx.needs_input_grad[3]
         if ctx.needs_input_grad[1] or need_db:
-            dw, db = ops.wgrad(dy, x, ctx.plan, ctx.stride, nhwc, with_bias=need_db, gelu_input=ctx.gelu_input)
-            dw = dw.to(w.dtype) if ctx.needs_input_grad[1] else None
             # bias shares the weight's dtype in an nn.Conv2d
-            db = db.to(w.dtype) if need_db else None
+            dw, db = ops.wgrad(dy, x, ctx.plan, ctx.stride, nhwc, with_bias=need_db, gelu_input=ctx.gelu_input,
+                               out_dtype=w.dtype)
+            dw = dw if ctx.needs_input_grad[1] else None
         return dx, dw, None, db, None, None, None, None, None
 
 
@@ -173,6 +178,12 @@ class DepthwiseOrientedConv1d(nn.Conv2d):
         gelu = self._gelu_in_kernel(x)
         if self.gelu_input and not gelu:
             x = torch.nn.functional.gelu(x)
+        if not torch.is_grad_enabled():      # inference: the kernel call alone
+            plan, stride = self._get_plan(), self.stride[0]
+            if not self.nhwc and not gelu and _via_nhwc(x, plan, stride):
+                return ops.nhwc_to_nchw(ops.fprop(ops.nchw_to_nhwc(x), self.weight, self.bias, plan, stride, True,
+                                                  self.add_identity))
+            return ops.fprop(x, self.weight, self.bias, plan, stride, self.nhwc, self.add_identity, gelu)
         return _DepthwiseOrientedConv1d.apply(x, self.weight, self.theta, self.bias, self._get_plan(),
                                               self.stride[0], self.nhwc, self.add_identity, gelu)
 

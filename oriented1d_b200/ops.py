@@ -1,7 +1,8 @@
 """torch-facing wrappers of the C ABI: tensors in, tensors out.
 
 torch is used for device memory (its caching allocator owns every buffer) and for the
-current stream; all arithmetic happens in libo1d.so.  There is no CPU path: every
+current stream; all arithmetic happens in libo1d.so, reached through csrc/o1d_torch.cpp (checks,
+allocation, stream and call in native code).  There is no CPU path: every
 function raises on a non-CUDA tensor, as the reference's extension does
 (CHECK_CUDA, models/dwoconv1d/kernels/kernels.cu:11).
 """
@@ -11,29 +12,12 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import lib, check
+from ._lib import ext, lib, check
 
 # kernels launched by one call of each entry point (used by the benchmark's launch count)
 KERNELS_PER_CALL = {"fprop": 1, "dgrad": 1, "wgrad": 2, "transpose": 1}
 
 _DTYPES = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16}
-
-
-def _dtype_code(t: torch.Tensor) -> int:
-    try:
-        return _DTYPES[t.dtype]
-    except KeyError:
-        raise TypeError(f"oriented1d_b200 supports float32 and bfloat16 tensors, got {t.dtype}") from None
-
-
-def _need_cuda(*tensors: torch.Tensor) -> None:
-    for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise RuntimeError("tensor must be a CUDA tensor (oriented1d_b200 has no CPU path)")
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def offsets(theta, K: int):
@@ -60,6 +44,7 @@ class Plan:
         check(lib.o1d_plan_build(th.data_ptr(), self.C, self.K, self.host.data_ptr()), "o1d_plan_build")
         self.num_classes = lib.o1d_plan_num_classes(self.host.data_ptr())
         self._dev: dict[torch.device, torch.Tensor] = {}
+        self._ptrs: dict = {}                # device index -> addresses of the host and the device copy
 
     def on(self, device: torch.device) -> torch.Tensor:
         d = self._dev.get(device)
@@ -68,140 +53,56 @@ class Plan:
             self._dev[device] = d
         return d
 
-
-def _dims(t: torch.Tensor, nhwc: bool):
-    if t.dim() != 4:
-        raise ValueError("expected a 4-D tensor")
-    if nhwc:
-        n, h, w, c = t.shape
-    else:
-        n, c, h, w = t.shape
-    return n, c, h, w
-
-
-def _check_params(plan: Plan, C: int, w=None, bias=None) -> None:
-    """The kernels index w as [C, K] and bias as [C]: a shorter buffer would be read past its end."""
-    if plan.C != C:
-        raise ValueError(f"plan was built for {plan.C} channels, tensor has {C}")
-    if w is not None and w.numel() != C * plan.K:
-        raise ValueError(f"weight has {w.numel()} elements, expected C*K = {C * plan.K}")
-    if bias is not None and bias.numel() != C:
-        raise ValueError(f"bias has {bias.numel()} elements, expected C = {C}")
+    def pointers(self, t: torch.Tensor):
+        """Addresses of the two copies for a call on t's device ((0, 0) when t is not on one: the
+        call then reports what is wrong with its arguments)."""
+        p = self._ptrs.get(t.get_device())
+        if p is None:
+            if not t.is_cuda:
+                return 0, 0
+            p = self._ptrs[t.get_device()] = (self.host.data_ptr(), self.on(t.device).data_ptr())
+        return p
 
 
 def fprop(x, w, bias, plan: Plan, stride: int = 1, nhwc: bool = False, add_identity: bool = False,
           gelu_input: bool = False):
     """y = oriented conv of x.  x: [N,C,H,W] (or [N,H,W,C] if nhwc), contiguous.  gelu_input: x is a
     pre-activation tensor and exact GELU is applied as it is loaded, y = conv(GELU(x))."""
-    N, C, H, W = _dims(x, nhwc)
-    K = plan.K
-    _check_params(plan, C, w, bias)
-    _need_cuda(x, w, bias)
-    x = x.contiguous()
-    w32 = w.detach().reshape(C, K).to(torch.float32).contiguous()
-    b32 = bias.detach().to(torch.float32).contiguous() if bias is not None else None
-    P, Q = -(-H // stride), -(-W // stride)
-    y = torch.empty((N, P, Q, C) if nhwc else (N, C, P, Q), dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
-        check(lib.o1d_fprop(x.data_ptr(), w32.data_ptr(), b32.data_ptr() if b32 is not None else None,
-                            plan.host.data_ptr(), plan.on(x.device).data_ptr(), y.data_ptr(),
-                            N, H, W, C, K, stride, int(nhwc), _dtype_code(x),
-                            int(bool(add_identity)) * _lib.FLAG_IDENTITY + int(bool(gelu_input)) * _lib.FLAG_GELU_INPUT,
-                            _stream()), "o1d_fprop")
-    return y
+    return ext.fprop(x, w, bias, plan.C, plan.K, *plan.pointers(x), stride, bool(nhwc), bool(add_identity), bool(gelu_input))
 
 
 def dgrad(dy, w, plan: Plan, H: int, W: int, stride: int = 1, nhwc: bool = False,
           add_identity: bool = False, pre=None):
     """dx [.., H, W ..] from dy [.., ceil(H/s), ceil(W/s) ..].  pre (shape of dx): the forward pass was
     conv(GELU(pre)); the result is then the gradient with respect to pre (times GELU'(pre))."""
-    N, C, P, Q = _dims(dy, nhwc)
-    if P != -(-H // stride) or Q != -(-W // stride):
-        raise ValueError("dy extents do not match ceil(H/stride) x ceil(W/stride)")
-    K = plan.K
-    _check_params(plan, C, w)
-    _need_cuda(dy, w)
-    dy = dy.contiguous()
-    w32 = w.detach().reshape(C, K).to(torch.float32).contiguous()
-    dx = torch.empty((N, H, W, C) if nhwc else (N, C, H, W), dtype=dy.dtype, device=dy.device)
-    if pre is not None:
-        if tuple(pre.shape) != tuple(dx.shape) or pre.dtype != dy.dtype:
-            raise ValueError("pre must have the shape and dtype of dx")
-        _need_cuda(pre)
-        pre = pre.contiguous()
-    with torch.cuda.device(dy.device):
-        check(lib.o1d_dgrad_act(dy.data_ptr(), w32.data_ptr(), pre.data_ptr() if pre is not None else None,
-                                plan.host.data_ptr(), plan.on(dy.device).data_ptr(), dx.data_ptr(), N, H, W, C, K,
-                                stride, int(nhwc), _dtype_code(dy), int(bool(add_identity)), _stream()),
-              "o1d_dgrad")
-    return dx
+    return ext.dgrad(dy, w, plan.C, plan.K, *plan.pointers(dy), H, W, stride, bool(nhwc), bool(add_identity), pre)
 
 
 def wgrad(dy, x, plan: Plan, stride: int = 1, nhwc: bool = False, with_bias: bool = False,
-          gelu_input: bool = False):
-    """(dw [C,1,1,K] fp32, db [C] fp32 or None).  Deterministic.  gelu_input: x is the pre-activation
+          gelu_input: bool = False, out_dtype: torch.dtype = torch.float32):
+    """(dw [C,1,1,K], db [C] or None) in `out_dtype`.  Deterministic.  gelu_input: x is the pre-activation
     tensor of a forward pass conv(GELU(x))."""
-    if dy.dtype != x.dtype:
-        raise TypeError("dy and x must have the same dtype")
-    N, C, H, W = _dims(x, nhwc)
-    K = plan.K
-    _check_params(plan, C)
-    P, Q = -(-H // stride), -(-W // stride)
-    if tuple(dy.shape) != ((N, P, Q, C) if nhwc else (N, C, P, Q)):
-        raise ValueError(f"dy has shape {tuple(dy.shape)}, expected the output shape of x "
-                         f"({(N, P, Q, C) if nhwc else (N, C, P, Q)})")
-    _need_cuda(dy, x)
-    dy, x = dy.contiguous(), x.contiguous()
-    code = _dtype_code(x)
-    dw = torch.empty((C, 1, 1, K), dtype=torch.float32, device=x.device)
-    db = torch.empty((C,), dtype=torch.float32, device=x.device) if with_bias else None
-    nbytes = lib.o1d_wgrad_workspace_bytes(N, H, W, C, K, stride, int(nhwc), code)
-    ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        check(lib.o1d_wgrad_act(dy.data_ptr(), x.data_ptr(), plan.host.data_ptr(),
-                                plan.on(x.device).data_ptr(), dw.data_ptr(),
-                                db.data_ptr() if db is not None else None, ws.data_ptr(), ws.numel(),
-                                N, H, W, C, K, stride, int(nhwc), code,
-                                _lib.FLAG_GELU_INPUT if gelu_input else 0, _stream()), "o1d_wgrad")
+    bf16 = out_dtype == torch.bfloat16
+    dw, db = ext.wgrad(dy, x, plan.C, plan.K, *plan.pointers(x), stride, bool(nhwc), bool(with_bias), bool(gelu_input), bf16)
+    if not bf16 and out_dtype != torch.float32:
+        dw, db = dw.to(out_dtype), None if db is None else db.to(out_dtype)
     return dw, db
-
-
-def _transpose(t: torch.Tensor, n: int, a: int, b: int, out_shape):
-    _need_cuda(t)
-    t = t.contiguous()
-    out = torch.empty(out_shape, dtype=t.dtype, device=t.device)
-    with torch.cuda.device(t.device):
-        check(lib.o1d_transpose(t.data_ptr(), out.data_ptr(), n, a, b, _dtype_code(t), _stream()),
-              "o1d_transpose")
-    return out
 
 
 def nhwc_to_nchw(x):
     """[N,H,W,C] -> [N,C,H,W], contiguous (reference: kernels.cu:56-61)."""
-    N, H, W, C = x.shape
-    return _transpose(x, N, H * W, C, (N, C, H, W))
+    return ext.transpose(x, False)
 
 
 def nchw_to_nhwc(x):
     """[N,C,H,W] -> [N,H,W,C], contiguous (reference: kernels.cu:63-68)."""
-    N, C, H, W = x.shape
-    return _transpose(x, N, C, H * W, (N, H, W, C))
+    return ext.transpose(x, True)
 
 
 def layer_norm_cl(x, weight, bias, eps: float = 1e-6, gelu: bool = False):
     """LayerNorm over the last (contiguous) axis, optionally fused with exact GELU.  Forward
     only (no autograd): for inference and for callers that handle gradients themselves."""
-    _need_cuda(x, weight, bias)
-    x = x.contiguous()
-    C = x.shape[-1]
-    rows = x.numel() // C
-    y = torch.empty_like(x)
-    g32 = weight.detach().to(torch.float32).contiguous()
-    b32 = bias.detach().to(torch.float32).contiguous()
-    with torch.cuda.device(x.device):
-        check(lib.o1d_layernorm_cl(x.data_ptr(), g32.data_ptr(), b32.data_ptr(), y.data_ptr(), rows, C, float(eps),
-                                   _dtype_code(x), int(gelu), _stream()), "o1d_layernorm_cl")
-    return y
+    return ext.layer_norm_cl(x, weight, bias, float(eps), bool(gelu))
 
 
 def layer_norm_cl_supported(x, gelu: bool = False, backward: bool = False) -> bool:
@@ -218,28 +119,7 @@ def layer_norm_cl_bwd(x, dy, weight, eps: float = 1e-6, bias=None, gelu: bool = 
     """Gradients of layer_norm_cl: dx in x's dtype, dweight and dbias in fp32.  With gelu=True the
     forward call ended in exact GELU and `bias` is needed again.  The statistics are recomputed
     from x; dweight / dbias are summed in a fixed order."""
-    _need_cuda(x, dy, weight)
-    x, dy = x.contiguous(), dy.contiguous()
-    if dy.shape != x.shape or dy.dtype != x.dtype:
-        raise ValueError(f"dy {tuple(dy.shape)} {dy.dtype} does not match x {tuple(x.shape)} {x.dtype}")
-    C = x.shape[-1]
-    if weight.numel() != C:
-        raise ValueError(f"weight has {weight.numel()} elements, expected {C}")
-    rows = x.numel() // C
-    dx = torch.empty_like(x)
-    g32 = weight.detach().to(torch.float32).contiguous()
-    if gelu and (bias is None or bias.numel() != C):
-        raise ValueError("gelu=True needs the forward call's bias")
-    b32 = bias.detach().to(torch.float32).contiguous() if gelu else None
-    dg = torch.empty((C,), dtype=torch.float32, device=x.device)
-    db = torch.empty((C,), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        nbytes = lib.o1d_layernorm_cl_bwd_workspace_bytes(rows, C)
-        ws = torch.empty((max(nbytes, 4),), dtype=torch.uint8, device=x.device)
-        check(lib.o1d_layernorm_cl_bwd(x.data_ptr(), dy.data_ptr(), g32.data_ptr(), b32.data_ptr() if gelu else None,
-                                       dx.data_ptr(), dg.data_ptr(), db.data_ptr(), ws.data_ptr(), nbytes, rows, C,
-                                       float(eps), _dtype_code(x), int(gelu), _stream()), "o1d_layernorm_cl_bwd")
-    return dx, dg, db
+    return ext.layer_norm_cl_bwd(x, dy, weight, float(eps), bias, bool(gelu), False)
 
 
 class LayerNormCL(torch.autograd.Function):
@@ -256,25 +136,14 @@ class LayerNormCL(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, weight, bias = ctx.saved_tensors
-        dx, dg, db = layer_norm_cl_bwd(x, dy, weight, ctx.eps, bias, ctx.gelu)
-        return (dx if ctx.needs_input_grad[0] else None, dg.to(weight.dtype) if ctx.needs_input_grad[1] else None,
-                db.to(bias.dtype) if ctx.needs_input_grad[2] else None, None, None)
+        dx, dg, db = ext.layer_norm_cl_bwd(x, dy, weight, ctx.eps, bias, ctx.gelu, True)
+        return (dx if ctx.needs_input_grad[0] else None, dg if ctx.needs_input_grad[1] else None,
+                db if ctx.needs_input_grad[2] else None, None, None)
 
 
 def colsum(x):
     """Sum over all but the last (contiguous) axis, in fp32 and in a fixed order: [..., C] -> [C]."""
-    _need_cuda(x)
-    x = x.contiguous()
-    C = x.shape[-1]
-    rows = x.numel() // C
-    out = torch.empty((C,), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        code = _dtype_code(x)
-        nbytes = lib.o1d_colsum_workspace_bytes(rows, C, code)
-        ws = torch.empty((max(nbytes, 4),), dtype=torch.uint8, device=x.device)
-        check(lib.o1d_colsum(x.data_ptr(), out.data_ptr(), ws.data_ptr(), nbytes, rows, C, code, _stream()),
-              "o1d_colsum")
-    return out
+    return ext.colsum(x, False)
 
 
 class LinearCL(torch.autograd.Function):
@@ -299,7 +168,9 @@ class LinearCL(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             dw = dy2.t() @ x.reshape(-1, x.shape[-1])
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = colsum(dy2).to(ctx.bias_dtype)
+            bf16 = ctx.bias_dtype == torch.bfloat16
+            db = ext.colsum(dy2, bf16)
+            db = db if bf16 else db.to(ctx.bias_dtype)
         return dx, dw, db
 
 
@@ -316,17 +187,7 @@ def pointwise_in(x, weight, bias):
     """Channels-last ``Linear`` over the few channels of an NCHW image: x [N,Cin,H,W] (Cin <= 4),
     weight [Cout,Cin], bias [Cout] or None -> [N,H,W,Cout] (models/convnext.py:143,170-176 in one
     pass).  Forward only."""
-    _need_cuda(x, weight)
-    x = x.contiguous()
-    N, Cin, H, W = x.shape
-    Cout = weight.shape[0]
-    y = torch.empty((N, H, W, Cout), dtype=x.dtype, device=x.device)
-    w32 = weight.detach().to(torch.float32).contiguous()
-    b32 = None if bias is None else bias.detach().to(torch.float32).contiguous()
-    with torch.cuda.device(x.device):
-        check(lib.o1d_pointwise_in(x.data_ptr(), w32.data_ptr(), 0 if b32 is None else b32.data_ptr(), y.data_ptr(),
-                                   N, Cin, H * W, Cout, _dtype_code(x), _stream()), "o1d_pointwise_in")
-    return y
+    return ext.pointwise_in(x, weight, bias)
 
 
 def uses_tiled(plan: Plan, N: int, H: int, W: int, stride: int, nhwc: bool, dtype: torch.dtype) -> bool:
