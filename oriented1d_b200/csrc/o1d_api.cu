@@ -247,7 +247,7 @@ int try_direct(const void *x, const float *w, const float *bias, const PlanHeade
 }
 
 // Forward / stride-1 input gradient of 7x7 maps with one channel plane per thread.
-int try_small7(const void *x, const float *w, const float *bias, const PlanHeader &ph, const void *plan_dev, void *y,
+int try_small7(const void *x, const void *w, const void *bias, int pbf16, const PlanHeader &ph, const void *plan_dev, void *y,
                int N, int H, int W, int C, int K, int stride, int layout, int dtype, int add_identity, int flip,
                cudaStream_t st, const DeviceInfo &d) {
     if (g_force_generic) return kNotTiled;
@@ -260,16 +260,16 @@ int try_small7(const void *x, const float *w, const float *bias, const PlanHeade
     cfg.p.flip = flip;
     cfg.p.add_identity = add_identity;
     PlanView pv = plan_view(plan_dev, ph);
-    const cudaError_t e = dtype == O1D_F32 ? launch_small7<float>(cfg, map, w, bias, pv.chan, y, st)
-                                           : launch_small7<__nv_bfloat16>(cfg, map, w, bias, pv.chan, y, st);
+    const cudaError_t e = dtype == O1D_F32 ? launch_small7<float>(cfg, map, w, bias, pbf16, pv.chan, y, st)
+                                           : launch_small7<__nv_bfloat16>(cfg, map, w, bias, pbf16, pv.chan, y, st);
     if (e != cudaSuccess) return cuda_fail(e, "7x7 plane kernel launch");
     g_last_route = O1D_ROUTE_PLANE7;
     return O1D_OK;
 }
 
 // Weight gradient of 7x7 maps with one channel plane per thread.
-int try_small7_wgrad(const void *dy, const void *x, const PlanHeader &ph, const void *plan_dev, float *dw, float *db,
-                     void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K, int stride,
+int try_small7_wgrad(const void *dy, const void *x, const PlanHeader &ph, const void *plan_dev, void *dw, void *db,
+                     int pbf16, void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K, int stride,
                      int layout, int dtype, cudaStream_t st, const DeviceInfo &d) {
     if (g_force_generic) return kNotTiled;
     const int esize = dtype == O1D_F32 ? 4 : 2;
@@ -286,7 +286,7 @@ int try_small7_wgrad(const void *dy, const void *x, const PlanHeader &ph, const 
                                            : launch_small7_wgrad<__nv_bfloat16>(cfg, mx, mdy, pv.chan, partial, st);
     if (e != cudaSuccess) return cuda_fail(e, "7x7 plane wgrad launch");
     const int tot = C * (K + 1);
-    small7_wgrad_final_kernel<<<ceil_div(tot, 128), 128, 0, st>>>(partial, dw, db, C, K, cfg.p.CCs, cfg.p.nchunks,
+    small7_wgrad_final_kernel<<<ceil_div(tot, 128), 128, 0, st>>>(partial, dw, db, pbf16, C, K, cfg.p.CCs, cfg.p.nchunks,
                                                                   cfg.p.tiles_n);
     O1D_CUDA(cudaGetLastError());
     g_last_route = O1D_ROUTE_PLANE7;
@@ -422,6 +422,10 @@ int route_forward(const void *x, const float *w, const float *bias, int wbf16, c
                      st, d);
         if (rc != kNotTiled) return rc;
     }
+    if (g_prefer == 0) {       // 7x7 maps on canonical lines: a channel plane per thread
+        rc = try_small7(x, w, bias, wbf16, ph, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip, st, d);
+        if (rc != kNotTiled) return rc;
+    }
     if (wbf16) return O1D_ERR_UNSUPPORTED;       // the other families read fp32 parameters
     if (g_prefer == 0 || g_prefer == 5) {   // items computed in place in their NHWC layout
         rc = try_walk(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip,
@@ -431,10 +435,6 @@ int route_forward(const void *x, const float *w, const float *bias, int wbf16, c
     if (g_prefer == 0 || g_prefer == 4) {   // stage maps with whole lines per thread
         rc = try_wline(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity,
                        flip, st, d, /*need_two_ctas=*/g_prefer == 0);
-        if (rc != kNotTiled) return rc;
-    }
-    if (g_prefer == 0) {       // 7x7 maps on canonical lines: a channel plane per thread
-        rc = try_small7(x, w, bias, ph, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip, st, d);
         if (rc != kNotTiled) return rc;
     }
     // Layers whose chunks are all of one line kind (the models' block-wise angle assignment) can
@@ -839,15 +839,15 @@ int wgrad_dispatch(const void *dy, const void *x, const PlanHeader &ph, const vo
                            layout, dtype, st, d);
         if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
     }
+    if (g_prefer == 0 && !act) {       // 7x7 maps on canonical lines: a channel plane per thread
+        rc = try_small7_wgrad(dy, x, ph, plan_dev, dw, db, out_bf16, workspace, workspace_bytes, N, H, W, C, K, stride, layout,
+                              dtype, st, d);
+        if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
+    }
     if (out_bf16) return O1D_ERR_UNSUPPORTED;                 // the other families write fp32 gradients
     if (act) {                 // x is GELU(pre), applied on load: tiled kernels, else general
         rc = try_tiled_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, workspace, workspace_bytes, N, H, W, C, K, stride,
                              layout, dtype, act, st, d, nullptr);
-        if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
-    } else
-    if (g_prefer == 0) {       // 7x7 maps on canonical lines: a channel plane per thread
-        rc = try_small7_wgrad(dy, x, ph, plan_dev, dw, db, workspace, workspace_bytes, N, H, W, C, K, stride, layout,
-                              dtype, st, d);
         if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
     }
     const bool small_map = (dtype == O1D_F32) ? (H * W <= 32 * 32) : (H * W <= 10 * 10);

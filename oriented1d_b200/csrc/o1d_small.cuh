@@ -68,8 +68,8 @@ __device__ __forceinline__ void small_plane(const float (&x)[kSmallPix], const f
 
 template <typename T>
 __global__ void __launch_bounds__(512, 1)
-small7_fprop_kernel(const __grid_constant__ CUtensorMap tmap, const float *__restrict__ wgt,
-                    const float *__restrict__ bias, const int8_t *__restrict__ chan, T *__restrict__ y,
+small7_fprop_kernel(const __grid_constant__ CUtensorMap tmap, const void *__restrict__ wgt,
+                    const void *__restrict__ bias, int pbf16, const int8_t *__restrict__ chan, T *__restrict__ y,
                     const SmallParams p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float *planes = reinterpret_cast<float *>(smem_raw + p.off_planes_bytes);
@@ -122,12 +122,12 @@ small7_fprop_kernel(const __grid_constant__ CUtensorMap tmap, const float *__res
             const int kk = k - kHalf + p.K / 2;
             if (k < kMaxTaps && kk >= 0 && kk < p.K) {
                 const int src = p.flip ? p.K - 1 - kk : kk;
-                v = __ldg(wgt + (size_t)(c0 + i) * p.K + src);
+                v = ld_param(wgt, (size_t)(c0 + i) * p.K + src, pbf16);
                 if (p.add_identity && src == p.K / 2) v += 1.f;
             }
             s_w[e] = v;
         }
-        const float bv = bias ? __ldg(bias + c0 + ch) : 0.f;
+        const float bv = bias ? ld_param(bias, c0 + ch, pbf16) : 0.f;
         const int line = chan[c0 + ch];                    // canonical line of this warp's channel
         if (!failed && !mbar_wait(&full[b], (it / p.nbuf) & 1)) failed = true;
         // ---- tile [image][pixel][channel] -> planes [channel][image][pixel] ----------------
@@ -285,8 +285,8 @@ small7_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
 }
 
 // dw[c][kk] = sum over the tiles of c's chunk, in tile order, of the partial of canonical tap kk - K/2 + 15.
-__global__ void small7_wgrad_final_kernel(const float *__restrict__ partial, float *__restrict__ dw,
-                                          float *__restrict__ db, int C, int K, int CCs, int nchunks, int tiles_n) {
+__global__ void small7_wgrad_final_kernel(const float *__restrict__ partial, void *__restrict__ dw,
+                                          void *__restrict__ db, int pbf16, int C, int K, int CCs, int nchunks, int tiles_n) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= C * (K + 1)) return;
     const int c = idx / (K + 1), kk = idx % (K + 1);
@@ -295,7 +295,7 @@ __global__ void small7_wgrad_final_kernel(const float *__restrict__ partial, flo
     const int slot = kk == K ? 31 : kk - K / 2 + kHalf;
     float sum = 0.f;
     for (int t = 0; t < tiles_n; t++) sum += partial[((size_t)(t * nchunks + chunk) * CCs + cl) * 32 + slot];
-    if (kk == K) db[c] = sum; else dw[(size_t)c * K + kk] = sum;
+    st_param(kk == K ? db : dw, kk == K ? (size_t)c : (size_t)c * K + kk, pbf16, sum);
 }
 
 // ---- host side -------------------------------------------------------------------------
@@ -335,12 +335,12 @@ inline int make_small7_tensor_map(CUtensorMap *map, const void *base, int N, int
 }
 
 template <typename T>
-cudaError_t launch_small7(const SmallConfig &cfg, const CUtensorMap &map, const float *w, const float *bias,
+cudaError_t launch_small7(const SmallConfig &cfg, const CUtensorMap &map, const void *w, const void *bias, int pbf16,
                           const int8_t *chan, void *y, cudaStream_t st) {
     auto kern = small7_fprop_kernel<T>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg.smem_bytes);
     if (e != cudaSuccess) return e;
-    kern<<<cfg.grid, cfg.threads, cfg.smem_bytes, st>>>(map, w, bias, chan, (T *)y, cfg.p);
+    kern<<<cfg.grid, cfg.threads, cfg.smem_bytes, st>>>(map, w, bias, pbf16, chan, (T *)y, cfg.p);
     return cudaGetLastError();
 }
 

@@ -56,7 +56,6 @@ struct Params {
 };
 // f(flag) with the parameters as stored, and again with fp32 ones where the library declines those.
 template <class F> void call(Params &p, const char *what, F &&f) {
-    py::gil_scoped_release gil;
     int rc = f(p.flag());
     if (rc == O1D_ERR_UNSUPPORTED && p.bf16) {
         p.widen();
@@ -155,20 +154,17 @@ std::tuple<Tensor, OptTensor> wgrad(const Tensor &dy_, const Tensor &x_, int64_t
                              with_bias ? (float *)db.data_ptr() : nullptr, ws.data_ptr(), bytes, (int)d.n, (int)d.h, (int)d.w, (int)d.c,
                              (int)K, (int)stride, nhwc, code, (gelu ? O1D_FLAG_GELU_INPUT : 0) | flag, st);
     };
-    {
-        py::gil_scoped_release gil;
-        int rc = run(bf16 ? O1D_FLAG_PARAMS_BF16 : 0);
-        if (rc == O1D_ERR_UNSUPPORTED && bf16) {         // kernels that write fp32 gradients only
-            dw = at::empty({d.c, 1, 1, K}, x.options().dtype(at::kFloat));
-            if (with_bias) db = at::empty({d.c}, x.options().dtype(at::kFloat));
-            rc = run(0);
-            if (rc == O1D_OK) {
-                dw = dw.to(at::kBFloat16);
-                if (with_bias) db = db.to(at::kBFloat16);
-            }
+    int rc = run(bf16 ? O1D_FLAG_PARAMS_BF16 : 0);
+    if (rc == O1D_ERR_UNSUPPORTED && bf16) {             // kernels that write fp32 gradients only
+        dw = at::empty({d.c, 1, 1, K}, x.options().dtype(at::kFloat));
+        if (with_bias) db = at::empty({d.c}, x.options().dtype(at::kFloat));
+        rc = run(0);
+        if (rc == O1D_OK) {
+            dw = dw.to(at::kBFloat16);
+            if (with_bias) db = db.to(at::kBFloat16);
         }
-        check(rc, "o1d_wgrad");
     }
+    check(rc, "o1d_wgrad");
     return {dw, with_bias ? OptTensor(db) : std::nullopt};
 }
 
@@ -180,7 +176,6 @@ Tensor transpose(const Tensor &t_, bool to_nhwc) {
     const int code = dtype_code(t);
     const int64_t n = t.size(0), hw = to_nhwc ? t.size(2) * t.size(3) : t.size(1) * t.size(2), c = to_nhwc ? t.size(1) : t.size(3);
     Tensor out = to_nhwc ? at::empty({n, t.size(2), t.size(3), c}, t.options()) : at::empty({n, c, t.size(1), t.size(2)}, t.options());
-    py::gil_scoped_release gil;
     check(o1d_transpose(ptr(t), out.data_ptr(), (int)n, (int)(to_nhwc ? c : hw), (int)(to_nhwc ? hw : c), code, stream()), "o1d_transpose");
     return out;
 }
@@ -224,7 +219,6 @@ std::tuple<Tensor, Tensor, Tensor> layer_norm_cl_bwd(const Tensor &x_, const Ten
     Tensor dg = at::empty({C}, opts), db = at::empty({C}, opts);
     const size_t bytes = o1d_layernorm_cl_bwd_workspace_bytes(rows, (int)C);
     Tensor ws = at::empty({(int64_t)std::max<size_t>(bytes, 4)}, x.options().dtype(at::kByte));
-    py::gil_scoped_release gil;
     check(o1d_layernorm_cl_bwd(ptr(x), ptr(dy), (const float *)ptr(p.w), (const float *)ptr(p.b), dx.data_ptr(), (float *)dg.data_ptr(),
                                (float *)db.data_ptr(), ws.data_ptr(), bytes, rows, (int)C, (float)eps, code,
                                (gelu ? 1 : 0) | (out_bf16 ? O1D_FLAG_PARAMS_BF16 : 0), stream()),
@@ -242,7 +236,6 @@ Tensor colsum(const Tensor &x_, bool bf16) {
     Tensor out = at::empty({C}, x.options().dtype(bf16 ? at::kBFloat16 : at::kFloat));
     const size_t bytes = o1d_colsum_workspace_bytes(rows, (int)C, code);
     Tensor ws = at::empty({(int64_t)std::max<size_t>(bytes, 4)}, x.options().dtype(at::kByte));
-    py::gil_scoped_release gil;
     check(o1d_colsum(ptr(x), (float *)out.data_ptr(), ws.data_ptr(), bytes, rows, (int)C, code | (bf16 ? O1D_FLAG_PARAMS_BF16 : 0), stream()),
           "o1d_colsum");
     return out;
@@ -263,16 +256,113 @@ Tensor pointwise_in(const Tensor &x_, const Tensor &w, const OptTensor &bias) {
     return y;
 }
 
+// The operator's autograd node (reference: models/dwoconv1d/dwoconv1d.py:18-69), free of Python on the
+// backward thread.  An NCHW tensor whose NHWC form has a fast path (`via`) is converted on the way in and
+// out, and its NHWC form is what backward keeps.
+struct ConvFn : torch::autograd::Function<ConvFn> {
+    static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x_, const Tensor &w, const Tensor &theta,
+                          const OptTensor &bias, const Tensor &host, const Tensor &dev, int64_t plan_c, int64_t K, int64_t stride, bool nhwc,
+                          bool via, bool identity, bool gelu) {
+        (void)theta;
+        const Tensor x = via ? transpose(x_, true) : x_.contiguous();
+        ctx->set_materialize_grads(false);
+        ctx->save_for_backward({x, w});
+        ctx->saved_data["host"] = host;
+        ctx->saved_data["dev"] = dev;
+        ctx->saved_data["p"] = std::vector<int64_t>{plan_c, K, stride, nhwc, via, identity, gelu, bias.has_value()};
+        const Tensor y = fprop(x, w, bias, plan_c, K, (int64_t)host.const_data_ptr(), (int64_t)dev.const_data_ptr(), stride, nhwc || via,
+                               identity, gelu);
+        return via ? transpose(y, false) : y;
+    }
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
+        torch::autograd::variable_list out(13);
+        Tensor dy = grads[0];
+        if (!dy.defined()) return out;
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &x = saved[0], &w = saved[1];
+        const auto p = ctx->saved_data["p"].toIntVector();
+        const int64_t plan_c = p[0], K = p[1], stride = p[2], host = (int64_t)ctx->saved_data["host"].toTensor().const_data_ptr(),
+                      dev = (int64_t)ctx->saved_data["dev"].toTensor().const_data_ptr();
+        const bool nhwc = p[3] || p[4], via = p[4], identity = p[5], gelu = p[6], has_bias = p[7];
+        if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
+        dy = via ? transpose(dy, true) : dy.contiguous();
+        if (ctx->needs_input_grad(0)) {
+            out[0] = dgrad(dy, w, plan_c, K, host, dev, x.size(nhwc ? 1 : 2), x.size(nhwc ? 2 : 3), stride, nhwc, identity,
+                           gelu ? OptTensor(x) : std::nullopt);
+            if (via) out[0] = transpose(out[0], false);
+        }
+        const bool need_w = ctx->needs_input_grad(1), need_b = has_bias && ctx->needs_input_grad(3);
+        if (need_w || need_b) {
+            auto [dw, db] = wgrad(dy, x, plan_c, K, host, dev, stride, nhwc, need_b, gelu, is_bf16(w));
+            const auto dt = w.scalar_type();             // the bias shares the weight's dtype
+            if (need_w) out[1] = dw.scalar_type() == dt ? dw : dw.to(dt);
+            if (need_b) out[3] = db->scalar_type() == dt ? *db : db->to(dt);
+        }
+        return out;
+    }
+};
+
+// Channels-last LayerNorm (and GELU) with this library's kernels on both passes.
+struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
+    static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x_, const Tensor &g, const Tensor &b, double eps, bool gelu) {
+        const Tensor x = x_.contiguous();
+        ctx->save_for_backward({x, g, b});
+        ctx->saved_data["eps"] = eps;
+        ctx->saved_data["gelu"] = gelu;
+        return layer_norm_cl(x, g, b, eps, gelu);
+    }
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        auto [dx, dg, db] = layer_norm_cl_bwd(saved[0], grads[0], saved[1], ctx->saved_data["eps"].toDouble(), saved[2],
+                                              ctx->saved_data["gelu"].toBool(), true);
+        return {ctx->needs_input_grad(0) ? dx : Tensor(), ctx->needs_input_grad(1) ? dg : Tensor(), ctx->needs_input_grad(2) ? db : Tensor(),
+                Tensor(), Tensor()};
+    }
+};
+Tensor layer_norm_train(const Tensor &x, const Tensor &g, const Tensor &b, double eps, bool gelu) { return LayerNormFn::apply(x, g, b, eps, gelu); }
+
+// Linear on channels-last activations whose bias gradient is this library's column sum; the two matrix
+// products stay with the GEMM library.
+struct LinearFn : torch::autograd::Function<LinearFn> {
+    static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x, const Tensor &w, const Tensor &b) {
+        ctx->save_for_backward({x, w});
+        ctx->saved_data["bias"] = (int64_t)b.scalar_type();
+        return at::linear(x, w, b);
+    }
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &x = saved[0], &w = saved[1], dy = grads[0].reshape({-1, grads[0].size(-1)});
+        torch::autograd::variable_list out(3);
+        if (ctx->needs_input_grad(0)) out[0] = dy.matmul(w).reshape(x.sizes());
+        if (ctx->needs_input_grad(1)) out[1] = dy.t().matmul(x.reshape({-1, x.size(-1)}));
+        if (ctx->needs_input_grad(2)) {
+            const auto dt = (at::ScalarType)ctx->saved_data["bias"].toInt();
+            out[2] = colsum(dy, dt == at::kBFloat16);
+            if (out[2].scalar_type() != dt) out[2] = out[2].to(dt);
+        }
+        return out;
+    }
+};
+Tensor linear_train(const Tensor &x, const Tensor &w, const Tensor &b) { return LinearFn::apply(x, w, b); }
+
+Tensor conv(const Tensor &x, const Tensor &w, const Tensor &theta, const OptTensor &bias, const Tensor &host, const Tensor &dev,
+            int64_t plan_c, int64_t K, int64_t stride, bool nhwc, bool via, bool identity, bool gelu) {
+    return ConvFn::apply(x, w, theta, bias, host, dev, plan_c, K, stride, nhwc, via, identity, gelu);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_o1d_torch, m) {
     m.def("set_check", [](py::object f) { g_check = new py::object(std::move(f)); });
-    m.def("fprop", &fprop);
-    m.def("dgrad", &dgrad);
-    m.def("wgrad", &wgrad);
-    m.def("transpose", &transpose);
-    m.def("layer_norm_cl", &layer_norm_cl);
-    m.def("layer_norm_cl_bwd", &layer_norm_cl_bwd);
-    m.def("colsum", &colsum);
-    m.def("pointwise_in", &pointwise_in);
+    m.def("fprop", &fprop, py::call_guard<py::gil_scoped_release>());
+    m.def("dgrad", &dgrad, py::call_guard<py::gil_scoped_release>());
+    m.def("wgrad", &wgrad, py::call_guard<py::gil_scoped_release>());
+    m.def("conv", &conv, py::call_guard<py::gil_scoped_release>());
+    m.def("layer_norm_train", &layer_norm_train, py::call_guard<py::gil_scoped_release>());
+    m.def("linear_train", &linear_train, py::call_guard<py::gil_scoped_release>());
+    m.def("transpose", &transpose, py::call_guard<py::gil_scoped_release>());
+    m.def("layer_norm_cl", &layer_norm_cl, py::call_guard<py::gil_scoped_release>());
+    m.def("layer_norm_cl_bwd", &layer_norm_cl_bwd, py::call_guard<py::gil_scoped_release>());
+    m.def("colsum", &colsum, py::call_guard<py::gil_scoped_release>());
+    m.def("pointwise_in", &pointwise_in, py::call_guard<py::gil_scoped_release>());
 }

@@ -30,6 +30,9 @@ from . import ops
 __all__ = ["DepthwiseOrientedConv1d", "get_dwoconv1d_kernel", "oriented_dwconv1d_get_module_from_params"]
 
 
+_native_dgrad, _native_wgrad = ops.dgrad, ops.wgrad
+
+
 def _via_nhwc(x, plan, stride) -> bool:
     """Does an NCHW tensor go through its NHWC form?  Where that form has a fast path."""
     if not x.is_cuda or x.dim() != 4:
@@ -184,8 +187,15 @@ class DepthwiseOrientedConv1d(nn.Conv2d):
                 return ops.nhwc_to_nchw(ops.fprop(ops.nchw_to_nhwc(x), self.weight, self.bias, plan, stride, True,
                                                   self.add_identity))
             return ops.fprop(x, self.weight, self.bias, plan, stride, self.nhwc, self.add_identity, gelu)
-        return _DepthwiseOrientedConv1d.apply(x, self.weight, self.theta, self.bias, self._get_plan(),
-                                              self.stride[0], self.nhwc, self.add_identity, gelu)
+        plan, stride = self._get_plan(), self.stride[0]
+        if ops.dgrad is _native_dgrad and ops.wgrad is _native_wgrad and x.is_cuda:
+            # the same node in native code: Python on the backward thread costs 60 us a call
+            via = not self.nhwc and not gelu and _via_nhwc(x, plan, stride)
+            return ops.ext.conv(x, self.weight, self.theta, self.bias, plan.host, plan.on(x.device), plan.C, plan.K, stride,
+                                self.nhwc, via, self.add_identity, gelu)
+        # gradients replaced by a caller (tracing, tests): the node that calls them by name
+        return _DepthwiseOrientedConv1d.apply(x, self.weight, self.theta, self.bias, plan, stride, self.nhwc,
+                                              self.add_identity, gelu)
 
     def forward_safe(self, x):
         """Any H x W; output extents ceil(H/stride) x ceil(W/stride) (dwoconv1d.py:154-187)."""

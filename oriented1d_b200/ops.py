@@ -122,23 +122,13 @@ def layer_norm_cl_bwd(x, dy, weight, eps: float = 1e-6, bias=None, gelu: bool = 
     return ext.layer_norm_cl_bwd(x, dy, weight, float(eps), bias, bool(gelu), False)
 
 
-class LayerNormCL(torch.autograd.Function):
+class LayerNormCL:
     """Channels-last LayerNorm with this library's kernels on both passes (F.layer_norm and its
-    autograd backward in the reference, models/convnext.py:28-56)."""
+    autograd backward in the reference, models/convnext.py:28-56).  The node lives in native code."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, eps, gelu=False):
-        x = x.contiguous()
-        ctx.save_for_backward(x, weight, bias)
-        ctx.eps, ctx.gelu = eps, bool(gelu)
-        return layer_norm_cl(x, weight, bias, eps, gelu)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, weight, bias = ctx.saved_tensors
-        dx, dg, db = ext.layer_norm_cl_bwd(x, dy, weight, ctx.eps, bias, ctx.gelu, True)
-        return (dx if ctx.needs_input_grad[0] else None, dg if ctx.needs_input_grad[1] else None,
-                db if ctx.needs_input_grad[2] else None, None, None)
+    def apply(x, weight, bias, eps, gelu=False):
+        return ext.layer_norm_train(x, weight, bias, float(eps), bool(gelu))
 
 
 def colsum(x):
@@ -146,32 +136,14 @@ def colsum(x):
     return ext.colsum(x, False)
 
 
-class LinearCL(torch.autograd.Function):
+class LinearCL:
     """F.linear on channels-last activations whose bias gradient is this library's column sum
     (autograd's own is a generic reduction that runs at a fifth of the memory rate on these
     shapes); the two matrix products stay with the GEMM library, as in nn.Linear."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias):
-        ctx.save_for_backward(x, weight)
-        ctx.has_bias = bias is not None
-        ctx.bias_dtype = bias.dtype if bias is not None else None
-        return torch.nn.functional.linear(x, weight, bias)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, weight = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1])
-        dx = dw = db = None
-        if ctx.needs_input_grad[0]:
-            dx = (dy2 @ weight).reshape(x.shape)
-        if ctx.needs_input_grad[1]:
-            dw = dy2.t() @ x.reshape(-1, x.shape[-1])
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            bf16 = ctx.bias_dtype == torch.bfloat16
-            db = ext.colsum(dy2, bf16)
-            db = db if bf16 else db.to(ctx.bias_dtype)
-        return dx, dw, db
+    def apply(x, weight, bias):
+        return torch.nn.functional.linear(x, weight) if bias is None else ext.linear_train(x, weight, bias)
 
 
 def linear_cl(module, x):
