@@ -215,6 +215,17 @@ int try_tiled(const void *x, const float *w, const float *bias, const PlanHeader
     return O1D_OK;
 }
 
+// Tiled kernels with a segment for less than this share of their threads give way to the direct ones.
+constexpr double kWeakTiled = 0.7;
+
+// Do the direct kernels come before the tiled ones?  Measured, they only win while several images share a
+// tile (7x7: 34 vs 37 us fp32, 39 vs 41 bf16; 14x14: 68 vs 63 fp32, 95 vs 63 bf16).
+bool direct_first(const PlanHeader &ph, const void *plan_host, int N, int H, int W, int C, int K, int stride, int layout, int esize,
+                  const DeviceInfo &d, DirectLaunchSet *ls) {
+    return direct_plan_launches(ph, plan_host, N, H, W, C, K, stride, layout, esize, d.smem_optin, d.sms, DIRECT_FPROP, ls) &&
+           ls->whole_image && ls->cfg[0].p.NI >= 2;
+}
+
 // Forward / stride-1 input gradient through the direct kernels; kNotTiled when they do not apply.
 int try_direct(const void *x, const float *w, const float *bias, const PlanHeader &ph, const void *plan_host,
                const void *plan_dev, void *y, int N, int H, int W, int C, int K, int stride, int layout, int dtype,
@@ -222,12 +233,10 @@ int try_direct(const void *x, const float *w, const float *bias, const PlanHeade
     if (g_force_generic) return kNotTiled;
     const int esize = dtype == O1D_F32 ? 4 : 2;
     DirectLaunchSet ls;
-    if (!direct_plan_launches(ph, plan_host, N, H, W, C, K, stride, layout, esize, d.smem_optin, d.sms, DIRECT_FPROP, &ls))
+    if (whole_image_only ? !direct_first(ph, plan_host, N, H, W, C, K, stride, layout, esize, d, &ls)
+                         : !direct_plan_launches(ph, plan_host, N, H, W, C, K, stride, layout, esize, d.smem_optin, d.sms,
+                                                 DIRECT_FPROP, &ls))
         return kNotTiled;
-    if (whole_image_only && !ls.whole_image) return kNotTiled;
-    // measured against the tiled kernels the direct ones only win while several images share a
-    // tile (7x7: 34 vs 37 us fp32, 39 vs 41 bf16; 14x14: 68 vs 63 fp32, 95 vs 63 bf16)
-    if (whole_image_only && ls.cfg[0].p.NI < 2) return kNotTiled;
     if (((uintptr_t)y & 3) != 0) return kNotTiled;
     for (int i = 0; i < ls.n; i++) {
         ls.cfg[i].p.flip = flip;
@@ -332,16 +341,28 @@ int try_seg(const void *x, const void *w, const void *bias, int wbf16, const Pla
     if (g_force_generic || !ph.all_canon || ph.chan_off == 0 || stride != 1 || layout != O1D_NHWC) return kNotTiled;
     const int esize = dtype == O1D_F32 ? 4 : 2;
     const int8_t *chan_host = reinterpret_cast<const int8_t *>(static_cast<const char *>(plan_host) + ph.chan_off);
-    const SegConfig *cfg = nullptr;
+    SegConfig *cfg = nullptr;
     if (!seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, false, &cfg)) return kNotTiled;
     if (((uintptr_t)y & 15) != 0) return kNotTiled;
+    // bf16 results have the bits of the family that the shape would otherwise take; fp32 ones the fastest order
+    int order = SEG_ANY;
+    if (esize == 2) {
+        if (cfg->order == SEG_UNSET) {
+            TiledConfig t;
+            DirectLaunchSet ls;
+            const bool tiled = tiled_configure(ph, plan_host, N, H, W, C, K, stride, layout, esize, d.smem_optin, d.sms, OP_FPROP, &t) &&
+                               t.util >= kWeakTiled;
+            cfg->order = tiled && !direct_first(ph, plan_host, N, H, W, C, K, stride, layout, esize, d, &ls) ? SEG_TILED : SEG_ASCENDING;
+        }
+        order = cfg->order;
+    }
     SegMaps maps;
     int rc = seg_maps(*cfg, x, true, &maps, "segment fprop");
     if (rc) return rc;
     int *flag = nullptr;
     if ((rc = device_flag_ptr(&flag))) return rc;
     PlanView pv = plan_view(plan_dev, ph);
-    const cudaError_t e = seg_launch_conv(*cfg, maps, w, bias, wbf16, pv.chan, y, flip, add_identity, flag, st);
+    const cudaError_t e = seg_launch_conv(*cfg, maps, w, bias, wbf16, pv.chan, y, flip, add_identity, order, flag, st);
     if (e != cudaSuccess) return cuda_fail(e, "segment fprop launch");
     g_last_route = O1D_ROUTE_DIRECT;
     return O1D_OK;
@@ -445,7 +466,7 @@ int route_forward(const void *x, const float *w, const float *bias, int wbf16, c
         TiledConfig t;
         if (tiled_configure(ph, plan_host, N, H, W, C, K, stride, layout, dtype == O1D_F32 ? 4 : 2, d.smem_optin, d.sms,
                             OP_FPROP, &t))
-            weak_tiled = t.util < 0.7;
+            weak_tiled = t.util < kWeakTiled;
     }
     if (g_prefer != 2) {
         rc = try_direct(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity,
@@ -557,7 +578,7 @@ int try_seg_wgrad(const void *dy, const void *x, const PlanHeader &ph, const voi
     if (g_force_generic || !ph.all_canon || ph.chan_off == 0 || stride != 1 || layout != O1D_NHWC) return kNotTiled;
     const int esize = dtype == O1D_F32 ? 4 : 2;
     const int8_t *chan_host = reinterpret_cast<const int8_t *>(static_cast<const char *>(plan_host) + ph.chan_off);
-    const SegConfig *cfg = nullptr;
+    SegConfig *cfg = nullptr;
     if (!seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, true, &cfg)) return kNotTiled;
     if (((uintptr_t)dy & 15) != 0 || ((uintptr_t)workspace & 15) != 0) return kNotTiled;
     if (workspace_bytes < seg_wgrad_bytes(*cfg)) return O1D_ERR_WORKSPACE;
@@ -856,7 +877,7 @@ int wgrad_dispatch(const void *dy, const void *x, const PlanHeader &ph, const vo
         TiledConfig t;
         if (tiled_configure(ph, plan_host, N, H, W, C, K, stride, layout, dtype == O1D_F32 ? 4 : 2, d.smem_optin, d.sms,
                             OP_WGRAD, &t))
-            weak_tiled = t.util < 0.7;
+            weak_tiled = t.util < kWeakTiled;
     }
     const bool direct_first = !act && (g_prefer == 3 || (g_prefer == 0 && (small_map || weak_tiled)));
     if (direct_first) {

@@ -212,7 +212,7 @@ constexpr size_t kKept = 64;
 }  // namespace
 
 bool seg_configure(const int8_t *chan, int N, int H, int W, int C, int K, int esize, int smem_optin, int sms, bool wgrad,
-                   const SegConfig **cfg) {
+                   SegConfig **cfg) {
     thread_local std::vector<std::unique_ptr<Entry>> kept;
     thread_local size_t oldest = 0;
     for (const auto &e : kept)
@@ -244,26 +244,28 @@ struct Args {
     SegParams p;
     cudaStream_t st;
 };
-template <typename T, int R, int LT, bool WG> cudaError_t launch(const SegConfig &cfg, const Args &a) {
-    auto kern = seg::seg_kernel<T, R, LT, WG>;
+template <typename T, int R, int LT, bool WG, bool MERGED> cudaError_t launch(const SegConfig &cfg, const Args &a) {
+    auto kern = seg::seg_kernel<T, R, LT, WG, MERGED>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg.smem_bytes);
     if (e != cudaSuccess) return e;
     kern<<<cfg.grid, seg::kThreads, cfg.smem_bytes, a.st>>>(*a.maps, *a.dy_maps, a.w, a.bias, a.wbf16, a.chan, (T *)a.y, a.partial,
                                                             a.err_flag, a.p);
     return cudaGetLastError();
 }
-template <typename T, bool WG> cudaError_t launch_any(const SegConfig &cfg, const Args &a) {
-    if (cfg.short_reach) return cfg.line_block == 28 ? launch<T, 7, 28, WG>(cfg, a) : launch<T, 7, 14, WG>(cfg, a);
-    return cfg.line_block == 28 ? launch<T, 15, 28, WG>(cfg, a) : launch<T, 15, 14, WG>(cfg, a);
+template <typename T, bool WG, bool MERGED> cudaError_t launch_any(const SegConfig &cfg, const Args &a) {
+    if (cfg.short_reach) return cfg.line_block == 28 ? launch<T, 7, 28, WG, MERGED>(cfg, a) : launch<T, 7, 14, WG, MERGED>(cfg, a);
+    return cfg.line_block == 28 ? launch<T, 15, 28, WG, MERGED>(cfg, a) : launch<T, 15, 14, WG, MERGED>(cfg, a);
 }
 }  // namespace
 
 cudaError_t seg_launch_conv(const SegConfig &cfg, const SegMaps &maps, const void *w, const void *bias, int wbf16,
-                            const int8_t *chan, void *y, int flip, int identity, int *err_flag, cudaStream_t st) {
+                            const int8_t *chan, void *y, int flip, int identity, int order, int *err_flag, cudaStream_t st) {
     Args a{&maps, &maps, w, bias, wbf16, chan, y, nullptr, err_flag, cfg.p, st};
     a.p.flip = flip;
     a.p.identity = identity;
-    return cfg.esize == 4 ? launch_any<float, false>(cfg, a) : launch_any<__nv_bfloat16, false>(cfg, a);
+    a.p.tiled_order = order == SEG_TILED;
+    if (cfg.esize == 4) return launch_any<float, false, true>(cfg, a);
+    return order == SEG_ASCENDING ? launch_any<__nv_bfloat16, false, false>(cfg, a) : launch_any<__nv_bfloat16, false, true>(cfg, a);
 }
 
 size_t seg_wgrad_bytes(const SegConfig &cfg) {
@@ -274,7 +276,7 @@ size_t seg_wgrad_bytes(const SegConfig &cfg) {
 cudaError_t seg_launch_wgrad(const SegConfig &cfg, const SegMaps &maps, const SegMaps &dy_maps, const int8_t *chan, const void *dy,
                              void *dw, void *db, int out_bf16, float *partial, int *err_flag, cudaStream_t st) {
     Args a{&maps, &dy_maps, nullptr, nullptr, 0, chan, const_cast<void *>(dy), partial, err_flag, cfg.p, st};
-    const cudaError_t e = cfg.esize == 4 ? launch_any<float, true>(cfg, a) : launch_any<__nv_bfloat16, true>(cfg, a);
+    const cudaError_t e = cfg.esize == 4 ? launch_any<float, true, true>(cfg, a) : launch_any<__nv_bfloat16, true, true>(cfg, a);
     if (e != cudaSuccess) return e;
     seg::seg_wgrad_final_kernel<<<dim3(ceil_div(cfg.p.C, cfg.p.CC), ceil_div(cfg.p.CC * 32, 256)), 256, 0, st>>>(partial, chan, dw, db, out_bf16, cfg.grid, cfg.p);
     return cudaGetLastError();

@@ -130,39 +130,68 @@ template <> struct Pair<__nv_bfloat16> {
     }
 };
 
-// Frame of canonical line o: positions run along image columns (H), rows (V) or both (diagonals, from
-// row to row); stored tap t of the base line has weight t, or 30 - t when rev is set, and line offset
-// sgn * dh (o1d_lines.cuh).
+// Order of a sum: taps ascending, one FMA each on top of the bias, as in the general and the direct kernels,
+// so that a layer's result has the same bits whichever family computes it (a bf16 network amplifies
+// differences of the last bit to the size of its gradients' noise).  The tiled kernels add taps that fall on
+// one pixel first, and walk canonical lines 3 and 4 from the last tap to the first: p.tiled_order does the same
+// for shapes whose other family they are.
+//
+// Frame of canonical line o: positions run along image columns (H), rows (V) or both (diagonals, from row to
+// row), in the direction in which the taps ascend: base tap m of the line is met m-th.  Lines whose tap k
+// ascends against the image axis are walked backwards (`mirrored`), and the base line's taps are
+// point-symmetric, so all lines of a kind run the same code; sgn: direction of a slanted line's steps across.
 enum : int { FR_H = 0, FR_V = 1, FR_D = 2 };
 __host__ __device__ constexpr int frame_of(int o) { return (o == 0 || o == 1 || o == 7) ? FR_H : (o == 2 || o == 6) ? FR_D : FR_V; }
 __host__ __device__ constexpr int kind_of(int o) { return (o == 0 || o == 4) ? KIND_AXIS : (o == 2 || o == 6) ? KIND_DIAG : KIND_SLANT; }
-__host__ __device__ constexpr int sgn_of(int o) { return (o == 5 || o == 7) ? -1 : 1; }
-__host__ __device__ constexpr int rev_of(int o) { return (o == 0 || o == 1) ? 0 : 1; }
+__host__ __device__ constexpr bool backwards(int o, bool tiled) { return tiled && (o == 3 || o == 4); }   // m = 30 - k
+__host__ __device__ constexpr bool mirrored(int o, bool tiled) { return o > 1 && !backwards(o, tiled); }
+__host__ __device__ constexpr int sgn_of(int o, bool tiled) { return ((o == 5 || o == 7) != mirrored(o, tiled)) ? -1 : 1; }
 constexpr bool frames_consistent() {
     for (int o = 0; o < 8; o++)
-        for (int t = 0; t < kMaxTaps; t++) {
-            const int k = rev_of(o) ? kMaxTaps - 1 - t : t;
-            const int dh = kCanonDh[o][k], dw = kCanonDw[o][k], b = kind_of(o), fr = frame_of(o);
-            const int pos = fr == FR_H ? dw : dh;
-            const int line = fr == FR_H ? dh : fr == FR_V ? dw : o == 2 ? dw + dh : dw - dh;
-            if (pos != kCanonDw[b][t]) return false;
-            if (line != (b == KIND_SLANT ? sgn_of(o) * kCanonDh[1][t] : 0)) return false;
-        }
+        for (int m = 0; m < kMaxTaps; m++)
+            for (int tiled = 0; tiled < 2; tiled++) {
+                const int k = backwards(o, tiled) ? kMaxTaps - 1 - m : m, b = kind_of(o), fr = frame_of(o);
+                const int dir = mirrored(o, tiled) ? -1 : 1;
+                const int dh = kCanonDh[o][k], dw = kCanonDw[o][k];
+                const int pos = fr == FR_H ? dw : dh;
+                const int line = fr == FR_H ? dh : fr == FR_V ? dw : o == 2 ? dw + dh : dw - dh;
+                if (dir * pos != kCanonDw[b][m]) return false;
+                if (line != (b == KIND_SLANT ? sgn_of(o, tiled) * kCanonDh[1][m] : 0)) return false;
+            }
     return true;
 }
 static_assert(frames_consistent(), "every canonical line must be a line (or a staircase of lines) of its frame");
 
-// Tap number of a slanted line at (line offset, position offset); the three centre taps share 15.
-constexpr int slant_tap(int dr, int dp, int half) {
+// Taps of a block's input, a run of n stored taps.  MERGED: taps that fall on one pixel are stored as one.
+struct Taps { int first, n; };
+constexpr Taps slant_taps(int dr, int dp, int half, bool merged) {
+    Taps f{0, 0};
     for (int t = kHalf - half; t <= kHalf + half; t++)
-        if (kCanonDh[1][t] == dr && kCanonDw[1][t] == dp) return (t == 14 || t == 16) ? 15 : t;
-    return -1;
+        if (kCanonDh[1][t] == dr && kCanonDw[1][t] == dp) {
+            if (f.n == 0) f.first = t;
+            f.n++;
+        }
+    if (merged && f.n == 3) f = {kHalf, 1};                     // the three centre taps share 15
+    return f;
+}
+// j: position offset; merged diagonals are stored by position
+template <int KIND, bool MERGED> constexpr Taps line_taps(int j, int half) {
+    Taps f{kHalf + j, j >= -half && j <= half ? 1 : 0};
+    if (KIND == KIND_DIAG && !MERGED) {
+        f.n = 0;
+        for (int t = kHalf - half; t <= kHalf + half; t++)
+            if (kCanonDw[2][t] == j) {
+                if (f.n == 0) f.first = t;
+                f.n++;
+            }
+    }
+    return f;
 }
 // Does input (rho, pi) reach any output of a slanted block?
 constexpr bool slant_used(int rho, int pi, int half) {
     for (int r = 0; r < kSR; r++)
         for (int t = 0; t < kST; t++)
-            if (slant_tap(rho - r, pi - t, half) >= 0) return true;
+            if (slant_taps(rho - r, pi - t, half, true).n) return true;
     return false;
 }
 constexpr int slant_first(int rho, int half) {
@@ -177,79 +206,85 @@ constexpr int slant_last(int rho, int half) {
 // ---- bodies ----------------------------------------------------------------------------------------
 // O: the block's outputs (or, for the weight gradient, the values of dy there); Wt: the weights (or the
 // accumulators of their gradient), by stored tap.  Addresses are byte offsets in shared memory, of the
-// lane's channel pair.  Inputs are visited outwards from the block's first position, so that one add-and-clamp
-// per input keeps the address inside the line.
-template <bool WG> __device__ __forceinline__ void use(f32x2 &o, f32x2 &w, f32x2 x) {
-    if (WG) fma2(w, o, x); else fma2(o, w, x);
+// lane's channel pair.  Inputs are visited in ascending position, one compare and one predicated add each: the
+// address stays where it is while the position is before `first` or past `last`.
+template <bool WG, int M, int NM> __device__ __forceinline__ void use(f32x2 &o, f32x2 (&w)[kMaxTaps], f32x2 x) {
+    static_for<M, M + NM>([&](auto m_) {
+        constexpr int m = decltype(m_)::value;
+        if (WG) fma2(w[m], o, x); else fma2(o, w[m], x);
+    });
+}
+// From position I to I + 1.
+template <int I> __device__ __forceinline__ void step_from(int &a, int step, int first) {
+    asm("{.reg .pred p;\n setp.le.s32 p, %2, %3;\n @p add.s32 %0, %0, %1;}" : "+r"(a) : "r"(step), "r"(first), "n"(I));
+}
+template <int I> __device__ __forceinline__ void step_to(int &a, int step, int last) {
+    asm("{.reg .pred p;\n setp.gt.s32 p, %2, %3;\n @p add.s32 %0, %0, %1;}" : "+r"(a) : "r"(step), "r"(last), "n"(I));
+}
+template <int I> __device__ __forceinline__ void step_between(int &a, int step, int first, int last) {
+    asm("{.reg .pred p;\n setp.le.s32 p, %2, %4;\n setp.gt.and.s32 p, %3, %4, p;\n @p add.s32 %0, %0, %1;}"
+        : "+r"(a) : "r"(step), "r"(first), "r"(last), "n"(I));
 }
 
-// Line: a = address of the block's first position, step between positions, lo / hi = addresses the line is
-// clamped to.  OUTSIDE: the first position itself may lie before lo (diagonals).  left / right: run the
-// inputs before / behind the block.
-template <typename T, int R, int NO, bool OUTSIDE, bool WG>
-__device__ __forceinline__ void line_body(int a, int step, int lo, int hi, bool left, bool right, f32x2 (&O)[NO],
+// Line (KIND_AXIS, KIND_DIAG): a = address of the block's first position, step between positions.  A diagonal's
+// first position may itself lie before `first` (never past `last`).  left / right: run the inputs before /
+// behind the block.
+template <typename T, int KIND, int R, int NO, bool WG, bool MERGED>
+__device__ __forceinline__ void line_body(int a, int step, int first, int last, bool left, bool right, f32x2 (&O)[NO],
                                           f32x2 (&Wt)[kMaxTaps]) {
+    constexpr int RP = KIND == KIND_DIAG ? kCanonDh[2][kHalf - R] : R;       // reach in positions
     auto input = [&](auto i_, f32x2 x) {            // position i relative to the first output
         constexpr int i = decltype(i_)::value;
         static_for<0, NO>([&](auto o_) {
-            constexpr int o = decltype(o_)::value, j = i - o;
-            if constexpr (j >= -R && j <= R) use<WG>(O[o], Wt[kHalf + j], x);
+            constexpr int o = decltype(o_)::value;
+            constexpr Taps f = line_taps<KIND, MERGED>(i - o, KIND == KIND_DIAG && MERGED ? RP : R);
+            if constexpr (f.n > 0) use<WG, f.first, f.n>(O[o], Wt, x);
         });
     };
     if (left) {
-        int b = OUTSIDE ? max(a, lo) : a;
-        static_for<0, R>([&](auto i_) {
-            b = max(b - step, lo);
-            input(std::integral_constant<int, -1 - decltype(i_)::value>{}, Pair<T>::lds(b));
+        int b = a + max(-RP, first) * step;
+        static_for<-RP, 0>([&](auto i_) {
+            input(i_, Pair<T>::lds(b));
+            step_from<decltype(i_)::value>(b, step, first);
         });
     }
+    if constexpr (KIND == KIND_DIAG) a += max(0, first) * step;
     static_for<0, NO>([&](auto i_) {
-        input(i_, Pair<T>::lds(OUTSIDE ? max(a, lo) : a));
-        a = min(a + step, hi);
+        input(i_, Pair<T>::lds(a));
+        if constexpr (KIND == KIND_DIAG) step_between<decltype(i_)::value>(a, step, first, last);
+        else step_to<decltype(i_)::value>(a, step, last);
     });
     if (right)
-        static_for<NO, NO + R>([&](auto i_) {
-            input(i_, Pair<T>::lds(OUTSIDE ? max(a, lo) : a));
-            a = min(a + step, hi);
+        static_for<NO, NO + RP>([&](auto i_) {
+            input(i_, Pair<T>::lds(a));
+            step_to<decltype(i_)::value>(a, step, last);
         });
 }
 
 // Slanted line: 3 lines (l0.., in direction sgn) x 8 positions.  base = address of line 0, first position of
-// the block; lines outside [llo, lhi] read line lzero.  lo, hi: the clamps relative to the first position.
-template <typename T, int HALF, bool WG>
-__device__ __forceinline__ void slant_body(int base, int lstep, int pstep, int l0, int sgn, int llo, int lhi, int lzero, int lo,
-                                           int hi, f32x2 (&O)[kSR * kST], f32x2 (&Wt)[kMaxTaps]) {
+// the block; lines outside [llo, lhi] read line lzero.  Taps ascend from the line furthest ahead to the last.
+template <typename T, int HALF, bool WG, bool MERGED>
+__device__ __forceinline__ void slant_body(int base, int lstep, int pstep, int l0, int sgn, int llo, int lhi, int lzero, int first,
+                                           int last, f32x2 (&O)[kSR * kST], f32x2 (&Wt)[kMaxTaps]) {
     constexpr int D = kCanonDh[1][kHalf - HALF];     // reach in lines
     static_for<0, kSR + 2 * D>([&](auto r_) {
-        constexpr int rho = decltype(r_)::value - D, first = slant_first(rho, HALF), last = slant_last(rho, HALF);
+        constexpr int rho = kSR - 1 + D - decltype(r_)::value, p0 = slant_first(rho, HALF), p1 = slant_last(rho, HALF);
         int l = sgn > 0 ? l0 + rho : l0 + kSR - 1 - rho;
         l = l < llo || l > lhi ? lzero : l;
-        const int la = base + l * lstep, alo = la + lo, ahi = la + hi;
-        auto input = [&](auto pi_, f32x2 x) {
+        int a = base + l * lstep + (p0 < 0 ? max(p0, first) : min(p0, last)) * pstep;
+        static_for<p0, p1 + 1>([&](auto pi_) {
             constexpr int pi = decltype(pi_)::value;
-            static_for<0, kSR * kST>([&](auto o_) {
-                constexpr int o = decltype(o_)::value, t = slant_tap(rho - o / kST, pi - o % kST, HALF);
-                if constexpr (t >= 0) use<WG>(O[o], Wt[t], x);
-            });
-        };
-        if constexpr (first < 0) {
-            constexpr int s = last < 0 ? last : -1;
-            int b = max(la + s * pstep, alo);
-            static_for<0, s - first + 1>([&](auto i_) {
-                constexpr int pi = s - decltype(i_)::value;
-                if constexpr (slant_used(rho, pi, HALF)) input(std::integral_constant<int, pi>{}, Pair<T>::lds(b));
-                b = max(b - pstep, alo);
-            });
-        }
-        if constexpr (last >= 0) {
-            constexpr int s = first < 0 ? 0 : first;
-            int b = min(la + s * pstep, ahi);
-            static_for<0, last + 1 - s>([&](auto i_) {
-                constexpr int pi = decltype(i_)::value + s;
-                if constexpr (slant_used(rho, pi, HALF)) input(std::integral_constant<int, pi>{}, Pair<T>::lds(b));
-                b = min(b + pstep, ahi);
-            });
-        }
+            if constexpr (slant_used(rho, pi, HALF)) {
+                const f32x2 x = Pair<T>::lds(a);
+                static_for<0, kSR * kST>([&](auto o_) {
+                    constexpr int o = decltype(o_)::value;
+                    constexpr Taps f = slant_taps(rho - o / kST, pi - o % kST, HALF, MERGED);
+                    if constexpr (f.n > 0) use<WG, f.first, f.n>(O[o], Wt, x);
+                });
+            }
+            if constexpr (pi < 0) step_from<pi>(a, pstep, first);
+            else step_to<pi>(a, pstep, last);
+        });
     });
 }
 
@@ -263,12 +298,12 @@ struct Class {
     int entry[kMaxPairs];
 };        // entry: pair | channels of it (1 low, 2 high) << 4; full: all are 3
 struct Tables {
-    f32x2 w[32][kMaxPairs];                  // by stored tap (colliding taps summed) and pair
+    f32x2 w[32][kMaxPairs];                  // by stored tap and pair
     f32x2 bias[kMaxPairs];
     int ncls, ids[kMaxCC];
     Class cls[12];
 };
-// Taps summed into stored tap i of a line kind (three 5-bit numbers, 31 = none).
+// MERGED: taps summed into stored tap i of a line kind (three 5-bit numbers, 31 = none).
 struct MergeTable { uint16_t src[3][32]; };
 constexpr MergeTable make_merge() {
     MergeTable m{};
@@ -284,7 +319,7 @@ constexpr MergeTable make_merge() {
     return m;
 }
 static __device__ const MergeTable g_merge = make_merge();
-// Stored tap of each tap of a diagonal.
+// MERGED: stored tap of each tap of a diagonal.
 struct DiagTable { int8_t at[kMaxTaps]; __device__ int operator[](int t) const { return at[t]; } };
 constexpr DiagTable make_diag() {
     DiagTable d{};
@@ -293,15 +328,18 @@ constexpr DiagTable make_diag() {
 }
 static __device__ const DiagTable g_diag_at = make_diag();
 
-// Weight of base tap t of channel c on canonical line id (0 when the kernel is shorter than the line).
-__device__ __forceinline__ float base_weight(const void *w, int wbf16, int c, int id, int t, const SegParams &p) {
-    if (t >= kMaxTaps) return 0.f;
-    const int k = ((rev_of(id) ^ p.flip) ? kMaxTaps - 1 - t : t) - kHalf + p.K / 2;
+// Weight of tap m (in the order of the sum) of channel c on canonical line id, the identity added to the
+// centre tap (0 when the kernel is shorter than the line).
+__device__ __forceinline__ float base_weight(const void *w, int wbf16, int c, int id, int m, const SegParams &p) {
+    if (m >= kMaxTaps) return 0.f;
+    const int k = (backwards(id, p.tiled_order) != (p.flip != 0) ? kMaxTaps - 1 - m : m) - kHalf + p.K / 2;
     if (k < 0 || k >= p.K) return 0.f;
     const size_t at = (size_t)c * p.K + k;
-    return wbf16 ? __bfloat162float(((const __nv_bfloat16 *)w)[at]) : __ldg((const float *)w + at);
+    const float v = wbf16 ? __bfloat162float(((const __nv_bfloat16 *)w)[at]) : __ldg((const float *)w + at);
+    return m == kHalf && p.identity ? v + 1.f : v;
 }
 // Tables of the chunk that starts at channel c0; ends in a barrier.
+template <bool MERGED>
 __device__ __noinline__ void build_tables(Tables *tab, const SegParams &p, const void *w, const void *bias, int wbf16,
                                           const int8_t *chan, int c0) {
     const int tid = threadIdx.x;
@@ -317,10 +355,10 @@ __device__ __noinline__ void build_tables(Tables *tab, const SegParams &p, const
             const int c = i >> 5, t = i & 31, id = tab->ids[c];
             float v = 0.f;
             if (id >= 0) {
-                const uint32_t src = g_merge.src[kind_of(id)][t];
-                v = base_weight(w, wbf16, c0 + c, id, src & 31, p) + base_weight(w, wbf16, c0 + c, id, src >> 5 & 31, p) +
-                    base_weight(w, wbf16, c0 + c, id, src >> 10 & 31, p);
-                if (t == kHalf && p.identity) v += 1.f;
+                const uint32_t src = MERGED ? g_merge.src[kind_of(id)][t] : t;
+                v = base_weight(w, wbf16, c0 + c, id, src & 31, p);
+                if (MERGED)
+                    v = v + base_weight(w, wbf16, c0 + c, id, src >> 5 & 31, p) + base_weight(w, wbf16, c0 + c, id, src >> 10 & 31, p);
             }
             reinterpret_cast<float *>(&tab->w[t][c >> 1])[c & 1] = v;
         }
@@ -491,15 +529,16 @@ __device__ __forceinline__ bool first_segment(const SegParams &p, Segment &g, Sp
 }
 
 // R: reach of the taps (15, or 7 for kernels of up to 15 taps); LT: outputs of a thread along a line.
+// MERGED: taps of a line that fall on one pixel are added before the products (see the order of a sum above).
 // WG = false: y = conv(x) + bias.  WG = true: y is dy, and each CTA leaves its share of the weight and bias
 // gradients of its chunks in `partial` ([slot][channel of the chunk][32], by stored tap, the bias last).
-template <typename T, int R, int LT, bool WG>
+template <typename T, int R, int LT, bool WG, bool MERGED>
 __global__ void __launch_bounds__(kThreads, 1)
 seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps dy_maps, const void *__restrict__ wv,
            const void *__restrict__ biasv, int wbf16, const int8_t *__restrict__ chan, T *__restrict__ y,
            float *__restrict__ partial, int *__restrict__ err_flag, const __grid_constant__ SegParams p) {
     char *sm = g_smem;
-    constexpr int PB = Pair<T>::kBytes, RD = kCanonDh[2][kHalf - R];
+    constexpr int PB = Pair<T>::kBytes;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     Tables *tab = reinterpret_cast<Tables *>(sm + p.off_tab);
     uint64_t *full = reinterpret_cast<uint64_t *>(sm + p.off_bar);
@@ -553,7 +592,7 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
         for (int i = tid; i < ge.nbuf * 16; i += kThreads)
             if ((i & 15) * 4 < px)
                 *reinterpret_cast<float *>(sm + p.off_tile + ((i >> 4) + 1) * ge.buf_bytes - px + (i & 15) * 4) = 0.f;
-        build_tables(tab, p, wv, biasv, wbf16, chan, c0);
+        build_tables<MERGED>(tab, p, wv, biasv, wbf16, chan, c0);
         int buf = 0, my_class = 0, stride = kWarps;
         f32x2 Wg[kMaxTaps], dbias = 0;           // weight gradient: the warp's accumulators
         if constexpr (WG) {
@@ -602,11 +641,14 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                     const bool act = ln < lpg && gi < imgs;
                     const int gt = tbuf + pair * PB + (act ? gi : 0) * ge.img_bytes;         // first output of the image
                     T *yi = y + ((size_t)(n0 + gi) * p.H + h0) * p.W * p.C + (size_t)w0 * p.C + c0 + 2 * pair;
-                    const int p0 = pb * bl;
+                    // the block's first position in the direction of the walk, and in the image
+                    const int q0 = pb * bl;
+                    const bool mir = mirrored(id, p.tiled_order);
+                    const int p0 = mir ? plen - 1 - q0 : q0;
                     auto task = [&](f32x2 (&Wt)[kMaxTaps], f32x2 bias) {
                     if (kind == KIND_SLANT) {
                         f32x2 O[kSR * kST];
-                        const int l0 = line * kSR;
+                        const int l0 = line * kSR, sgn = sgn_of(id, p.tiled_order);
                         const bool hf = fr == FR_H;
                         const int lstep = hf ? row_bytes : px, pstep = hf ? px : row_bytes;
                         const int plo = hf ? ge.plo_w : ge.plo_h, phi = hf ? ge.phi_w : ge.phi_h;
@@ -619,8 +661,8 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                             const ptrdiff_t ls = hf ? (ptrdiff_t)p.W * p.C : p.C, ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
 #pragma unroll
                             for (int r = 0; r < kSR; r++) {
-                                const int l = sgn_of(id) > 0 ? l0 + r : l0 + kSR - 1 - r;
-                                f(r, yi + l * ls + p0 * ps, ps, act && l < llen ? plen - p0 : 0);
+                                const int l = sgn > 0 ? l0 + r : l0 + kSR - 1 - r;
+                                f(r, yi + l * ls + p0 * ps, mir ? -ps : ps, act && l < llen ? plen - q0 : 0);
                             }
                         };
                         if constexpr (WG) each_line([&](int r, T *q, ptrdiff_t ps, int left) { load_line<T, kST>(q, ps, &O[r * kST], left); });
@@ -628,8 +670,8 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
 #pragma unroll
                             for (int o = 0; o < kSR * kST; o++) O[o] = bias;
                         }
-                        slant_body<T, R, WG>(gt + p0 * pstep, lstep, pstep, l0, sgn_of(id), llo, lhi, lzero, (plo - p0) * pstep,
-                                             (phi - p0) * pstep, O, Wt);
+                        slant_body<T, R, WG, MERGED>(gt + p0 * pstep, lstep, mir ? -pstep : pstep, l0, sgn, llo, lhi, lzero,
+                                                     mir ? p0 - phi : plo - p0, mir ? p0 - plo : phi - p0, O, Wt);
                         if constexpr (WG) {
 #pragma unroll
                             for (int o = 0; o < kSR * kST; o++) add2(dbias, O[o]);
@@ -639,30 +681,32 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                         f32x2 O[LT];
                         const bool hf = fr == FR_H;
                         const int step = hf ? px : row_bytes, base = gt + line * (hf ? row_bytes : px);
+                        const int plo = hf ? ge.plo_w : ge.plo_h, phi = hf ? ge.phi_w : ge.phi_h;
                         const bool cut = hf ? ge.halo_w : ge.halo_h;
                         auto place = [&](auto &&f) {
                             const ptrdiff_t ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
-                            f(yi + line * (hf ? (ptrdiff_t)p.W * p.C : p.C) + p0 * ps, ps);
+                            f(yi + line * (hf ? (ptrdiff_t)p.W * p.C : p.C) + p0 * ps, mir ? -ps : ps);
                         };
-                        if constexpr (WG) place([&](T *q, ptrdiff_t ps) { load_line<T, LT>(q, ps, O, act ? plen - p0 : 0); });
+                        if constexpr (WG) place([&](T *q, ptrdiff_t ps) { load_line<T, LT>(q, ps, O, act ? plen - q0 : 0); });
                         else {
 #pragma unroll
                             for (int o = 0; o < LT; o++) O[o] = bias;
                         }
-                        line_body<T, R, LT, false, WG>(base + p0 * step, step, base + (hf ? ge.plo_w : ge.plo_h) * step,
-                                                       base + (hf ? ge.phi_w : ge.phi_h) * step, p0 > 0 || cut, p0 + LT < plen || cut, O, Wt);
+                        line_body<T, KIND_AXIS, R, LT, WG, MERGED>(base + p0 * step, mir ? -step : step, mir ? p0 - phi : plo - p0,
+                                                                   mir ? p0 - plo : phi - p0, q0 > 0 || cut, q0 + LT < plen || cut, O, Wt);
                         if constexpr (WG) {
 #pragma unroll
                             for (int o = 0; o < LT; o++) add2(dbias, O[o]);
                         } else
-                            place([&](T *q, ptrdiff_t ps) { store_line<T, LT>(q, ps, O, act ? plen - p0 : 0, all, mask); });
+                            place([&](T *q, ptrdiff_t ps) { store_line<T, LT>(q, ps, O, act ? plen - q0 : 0, all, mask); });
                     } else {
                         f32x2 O[kTD];
-                        const int dw = id == 2 ? -1 : 1, w = dw > 0 ? line - (kTD - 1) : line;
-                        auto in = [&](int o) { return act && p0 + o < plen && (unsigned)(w + o * dw) < (unsigned)lenw; };
+                        // per position: dh rows down, dw pixels to the right
+                        const int dh = mir ? -1 : 1, dw = (id == 2) == mir ? 1 : -1, w = dw > 0 ? line - (kTD - 1) : line;
+                        auto in = [&](int o) { return act && q0 + o < plen && (unsigned)(w + o * dw) < (unsigned)lenw; };
                         if constexpr (WG) {
                             const T *q = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
-                            const ptrdiff_t ps = ((ptrdiff_t)p.W + dw) * p.C;
+                            const ptrdiff_t ps = ((ptrdiff_t)dh * p.W + dw) * p.C;
 #pragma unroll
                             for (int o = 0; o < kTD; o++) { O[o] = Pair<T>::ldg_if(in(o), q); q += ps; }
                         } else {
@@ -670,19 +714,19 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                             for (int o = 0; o < kTD; o++) O[o] = bias;
                         }
                         // where the diagonal enters and leaves the tile (at the zeros around a whole map), from the block's first position
-                        const int f = max(dw > 0 ? ge.plo_w - w : w - ge.phi_w, ge.plo_h - p0);
-                        const int l = min(dw > 0 ? ge.phi_w - w : w - ge.plo_w, ge.phi_h - p0);
+                        const int f = max(dw > 0 ? ge.plo_w - w : w - ge.phi_w, dh > 0 ? ge.plo_h - p0 : p0 - ge.phi_h);
+                        const int l = min(dw > 0 ? ge.phi_w - w : w - ge.plo_w, dh > 0 ? ge.phi_h - p0 : p0 - ge.plo_h);
                         // (a diagonal that misses the tile reads its first row, zeros around a whole map)
                         const bool miss = f > l;
-                        const int step = row_bytes + dw * px, a0 = miss ? gt + ge.plo_h * row_bytes : gt + p0 * row_bytes + w * px;
-                        line_body<T, RD, kTD, true, WG>(a0, step, miss ? a0 : a0 + f * step, miss ? a0 : a0 + l * step, p0 > 0 || ge.halo_h,
-                                                        p0 + kTD < plen || ge.halo_h, O, Wt);
+                        line_body<T, KIND_DIAG, R, kTD, WG, MERGED>(miss ? gt + ge.plo_h * row_bytes : gt + p0 * row_bytes + w * px,
+                                                                    dh * row_bytes + dw * px, miss ? 0 : f, miss ? 0 : l,
+                                                                    q0 > 0 || ge.halo_h, q0 + kTD < plen || ge.halo_h, O, Wt);
                         if constexpr (WG) {
 #pragma unroll
                             for (int o = 0; o < kTD; o++) add2(dbias, O[o]);
                         } else {
                             T *yl = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
-                            const ptrdiff_t ps = ((ptrdiff_t)p.W + dw) * p.C;
+                            const ptrdiff_t ps = ((ptrdiff_t)dh * p.W + dw) * p.C;
 #pragma unroll
                             for (int o = 0; o < kTD; o++) {
                                 if (in(o)) {
@@ -793,7 +837,7 @@ seg_wgrad_final_kernel(const float *__restrict__ partial, const int8_t *__restri
         if (c >= p.C || (k < 31 ? k >= p.K : db == nullptr)) continue;
         int at = 31;
         if (k < 31) {
-            const int id = chan[c], j = k - p.K / 2 + kHalf, t = rev_of(id) ? kMaxTaps - 1 - j : j, kind = kind_of(id);
+            const int kind = kind_of(chan[c]), t = k - p.K / 2 + kHalf;
             at = kind == KIND_SLANT ? (t == 14 || t == 16 ? 15 : t) : kind == KIND_DIAG ? g_diag_at[t] : t;
         }
         float sum = 0.f;

@@ -8,6 +8,8 @@
 namespace o1d {
 
 constexpr int kSegGeos = 6, kSegRuns = 20;
+// Order of the sums (o1d_seg.cuh): any; taps ascending; as the tiled kernels.
+enum : int { SEG_UNSET = 0, SEG_ANY, SEG_ASCENDING, SEG_TILED };
 
 // How the maps of a run of chunks are cut into items: G whole images, or one tile of an image.
 struct SegGeo {
@@ -33,6 +35,7 @@ struct SegParams {
     int nruns, per_chunk;
     int off_tile, off_tab, off_bar;
     int flip, identity;
+    int tiled_order;                     // order of the sums, see o1d_seg.cuh
     long long total_cost;
     SegGeo geo[kSegGeos];
     SegRun run[kSegRuns];
@@ -42,16 +45,18 @@ struct SegMaps { CUtensorMap m[kSegGeos]; };
 struct SegConfig {
     SegParams p;
     int esize, short_reach, line_block, smem_bytes, grid, ngeos;
+    int order;                           // order of the sums, for the caller to keep here: SEG_UNSET at first
 };
 
 // Do the segment kernels take this request (NHWC, stride 1, canonical lines)?  `chan`: canonical line of
 // every channel (host copy of the plan's table).  The answer for a shape is kept per thread.
 bool seg_configure(const int8_t *chan, int N, int H, int W, int C, int K, int esize, int smem_optin, int sms, bool wgrad,
-                   const SegConfig **cfg);
+                   SegConfig **cfg);
 
 // y = conv(x) + bias (flip = 1: input gradient).  w, bias fp32, or bf16 when wbf16 is set.
+// order: SEG_ANY is the fastest.
 cudaError_t seg_launch_conv(const SegConfig &cfg, const SegMaps &maps, const void *w, const void *bias, int wbf16,
-                            const int8_t *chan, void *y, int flip, int identity, int *err_flag, cudaStream_t st);
+                            const int8_t *chan, void *y, int flip, int identity, int order, int *err_flag, cudaStream_t st);
 
 // Weight gradient (and bias gradient when db is not null): dw, db fp32, or bf16 when out_bf16 is set.
 // `partial`: seg_wgrad_bytes() of scratch.
