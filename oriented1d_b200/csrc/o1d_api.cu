@@ -345,7 +345,7 @@ int try_seg(const void *x, const void *w, const void *bias, int wbf16, const Pla
     if (!seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, false, &cfg)) return kNotTiled;
     if (((uintptr_t)y & 15) != 0) return kNotTiled;
     // bf16 results have the bits of the family that the shape would otherwise take; fp32 ones the fastest order
-    int order = SEG_ANY;
+    int order = SEG_TILED;
     if (esize == 2) {
         if (cfg->order == SEG_UNSET) {
             TiledConfig t;

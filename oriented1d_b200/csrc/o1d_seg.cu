@@ -263,7 +263,6 @@ cudaError_t seg_launch_conv(const SegConfig &cfg, const SegMaps &maps, const voi
     Args a{&maps, &maps, w, bias, wbf16, chan, y, nullptr, err_flag, cfg.p, st};
     a.p.flip = flip;
     a.p.identity = identity;
-    a.p.tiled_order = order == SEG_TILED;
     if (cfg.esize == 4) return launch_any<float, false, true>(cfg, a);
     return order == SEG_ASCENDING ? launch_any<__nv_bfloat16, false, false>(cfg, a) : launch_any<__nv_bfloat16, false, true>(cfg, a);
 }

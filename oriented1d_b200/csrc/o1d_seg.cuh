@@ -133,8 +133,8 @@ template <> struct Pair<__nv_bfloat16> {
 // Order of a sum: taps ascending, one FMA each on top of the bias, as in the general and the direct kernels,
 // so that a layer's result has the same bits whichever family computes it (a bf16 network amplifies
 // differences of the last bit to the size of its gradients' noise).  The tiled kernels add taps that fall on
-// one pixel first, and walk canonical lines 3 and 4 from the last tap to the first: p.tiled_order does the same
-// for shapes whose other family they are.
+// one pixel first, and walk canonical lines 3 and 4 from the last tap to the first: MERGED does the same, for
+// shapes whose other family they are and wherever the order is free (21 FMAs instead of 31 on a diagonal).
 //
 // Frame of canonical line o: positions run along image columns (H), rows (V) or both (diagonals, from row to
 // row), in the direction in which the taps ascend: base tap m of the line is met m-th.  Lines whose tap k
@@ -224,6 +224,12 @@ template <int I> __device__ __forceinline__ void step_to(int &a, int step, int l
 template <int I> __device__ __forceinline__ void step_between(int &a, int step, int first, int last) {
     asm("{.reg .pred p;\n setp.le.s32 p, %2, %4;\n setp.gt.and.s32 p, %3, %4, p;\n @p add.s32 %0, %0, %1;}"
         : "+r"(a) : "r"(step), "r"(first), "r"(last), "n"(I));
+}
+
+// The same number, but not known to be: what is derived from it is derived anew.
+__device__ __forceinline__ int anew(int v) {
+    asm volatile("" : "+r"(v));
+    return v;
 }
 
 // Line (KIND_AXIS, KIND_DIAG): a = address of the block's first position, step between positions.  A diagonal's
@@ -330,9 +336,10 @@ static __device__ const DiagTable g_diag_at = make_diag();
 
 // Weight of tap m (in the order of the sum) of channel c on canonical line id, the identity added to the
 // centre tap (0 when the kernel is shorter than the line).
+template <bool MERGED>
 __device__ __forceinline__ float base_weight(const void *w, int wbf16, int c, int id, int m, const SegParams &p) {
     if (m >= kMaxTaps) return 0.f;
-    const int k = (backwards(id, p.tiled_order) != (p.flip != 0) ? kMaxTaps - 1 - m : m) - kHalf + p.K / 2;
+    const int k = (backwards(id, MERGED) != (p.flip != 0) ? kMaxTaps - 1 - m : m) - kHalf + p.K / 2;
     if (k < 0 || k >= p.K) return 0.f;
     const size_t at = (size_t)c * p.K + k;
     const float v = wbf16 ? __bfloat162float(((const __nv_bfloat16 *)w)[at]) : __ldg((const float *)w + at);
@@ -356,9 +363,9 @@ __device__ __noinline__ void build_tables(Tables *tab, const SegParams &p, const
             float v = 0.f;
             if (id >= 0) {
                 const uint32_t src = MERGED ? g_merge.src[kind_of(id)][t] : t;
-                v = base_weight(w, wbf16, c0 + c, id, src & 31, p);
+                v = base_weight<MERGED>(w, wbf16, c0 + c, id, src & 31, p);
                 if (MERGED)
-                    v = v + base_weight(w, wbf16, c0 + c, id, src >> 5 & 31, p) + base_weight(w, wbf16, c0 + c, id, src >> 10 & 31, p);
+                    v = v + base_weight<MERGED>(w, wbf16, c0 + c, id, src >> 5 & 31, p) + base_weight<MERGED>(w, wbf16, c0 + c, id, src >> 10 & 31, p);
             }
             reinterpret_cast<float *>(&tab->w[t][c >> 1])[c & 1] = v;
         }
@@ -529,7 +536,7 @@ __device__ __forceinline__ bool first_segment(const SegParams &p, Segment &g, Sp
 }
 
 // R: reach of the taps (15, or 7 for kernels of up to 15 taps); LT: outputs of a thread along a line.
-// MERGED: taps of a line that fall on one pixel are added before the products (see the order of a sum above).
+// MERGED: the tiled kernels' order of a sum (see above).
 // WG = false: y = conv(x) + bias.  WG = true: y is dy, and each CTA leaves its share of the weight and bias
 // gradients of its chunks in `partial` ([slot][channel of the chunk][32], by stored tap, the bias last).
 template <typename T, int R, int LT, bool WG, bool MERGED>
@@ -640,32 +647,37 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                     const int li = ug * lpg + ln, gi = ge.G == 1 ? (li >= nlines) : li / nlines, line = li - gi * nlines;
                     const bool act = ln < lpg && gi < imgs;
                     const int gt = tbuf + pair * PB + (act ? gi : 0) * ge.img_bytes;         // first output of the image
-                    T *yi = y + ((size_t)(n0 + gi) * p.H + h0) * p.W * p.C + (size_t)w0 * p.C + c0 + 2 * pair;
                     // the block's first position in the direction of the walk, and in the image
                     const int q0 = pb * bl;
-                    const bool mir = mirrored(id, p.tiled_order);
+                    const bool mir = mirrored(id, MERGED);
                     const int p0 = mir ? plen - 1 - q0 : q0;
+                    // Output pixel.  Where a block's outputs lie is worked out from a few numbers, anew behind the body:
+                    // kept over it the addresses and strides cost registers (56x56x96 bf16, batch 128: 194 us, now 169).
+                    auto out = [&](int gi, int h, int w) {
+                        return y + (((size_t)(n0 + gi) * p.H + h0 + h) * p.W + w0 + w) * p.C + c0 + 2 * pair;
+                    };
                     auto task = [&](f32x2 (&Wt)[kMaxTaps], f32x2 bias) {
                     if (kind == KIND_SLANT) {
                         f32x2 O[kSR * kST];
-                        const int l0 = line * kSR, sgn = sgn_of(id, p.tiled_order);
+                        const int l0 = line * kSR, sgn = sgn_of(id, MERGED);
                         const bool hf = fr == FR_H;
                         const int lstep = hf ? row_bytes : px, pstep = hf ? px : row_bytes;
                         const int plo = hf ? ge.plo_w : ge.plo_h, phi = hf ? ge.phi_w : ge.phi_h;
                         const int cut = hf ? ge.halo_h : ge.halo_w;
                         const int llo = (hf ? ge.plo_h : ge.plo_w) + 1 - cut, lhi = (hf ? ge.phi_h : ge.phi_w) - 1 + cut;
                         const int lzero = cut ? 0 : hf ? ge.plo_h : ge.phi_w;
-                        // line r of the block, `left` positions of it (addresses are formed where they are used: kept
-                        // over the body they cost registers, 10 % of the time)
-                        auto each_line = [&](auto &&f) {
-                            const ptrdiff_t ls = hf ? (ptrdiff_t)p.W * p.C : p.C, ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
+                        // line r of the block, `left` positions of it
+                        auto each_line = [&](int id, int l0, int gi, int q0, auto &&f) {
+                            const bool hf = frame_of(id) == FR_H, mir = mirrored(id, MERGED);
+                            const int plen = hf ? lenw : lenh, llen = hf ? lenh : lenw, p0 = mir ? plen - 1 - q0 : q0, sgn = sgn_of(id, MERGED);
+                            const ptrdiff_t ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
 #pragma unroll
                             for (int r = 0; r < kSR; r++) {
                                 const int l = sgn > 0 ? l0 + r : l0 + kSR - 1 - r;
-                                f(r, yi + l * ls + p0 * ps, mir ? -ps : ps, act && l < llen ? plen - q0 : 0);
+                                f(r, out(gi, hf ? l : p0, hf ? p0 : l), mir ? -ps : ps, act && l < llen ? plen - q0 : 0);
                             }
                         };
-                        if constexpr (WG) each_line([&](int r, T *q, ptrdiff_t ps, int left) { load_line<T, kST>(q, ps, &O[r * kST], left); });
+                        if constexpr (WG) each_line(id, l0, gi, q0, [&](int r, T *q, ptrdiff_t ps, int left) { load_line<T, kST>(q, ps, &O[r * kST], left); });
                         else {
 #pragma unroll
                             for (int o = 0; o < kSR * kST; o++) O[o] = bias;
@@ -676,18 +688,20 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
 #pragma unroll
                             for (int o = 0; o < kSR * kST; o++) add2(dbias, O[o]);
                         } else
-                            each_line([&](int r, T *q, ptrdiff_t ps, int left) { store_line<T, kST>(q, ps, &O[r * kST], left, all, mask); });
+                            each_line(anew(id), anew(l0), anew(gi), anew(q0), [&](int r, T *q, ptrdiff_t ps, int left) { store_line<T, kST>(q, ps, &O[r * kST], left, all, mask); });
                     } else if (kind == KIND_AXIS) {
                         f32x2 O[LT];
                         const bool hf = fr == FR_H;
                         const int step = hf ? px : row_bytes, base = gt + line * (hf ? row_bytes : px);
                         const int plo = hf ? ge.plo_w : ge.plo_h, phi = hf ? ge.phi_w : ge.phi_h;
                         const bool cut = hf ? ge.halo_w : ge.halo_h;
-                        auto place = [&](auto &&f) {
+                        auto place = [&](int id, int line, int gi, int q0, auto &&f) {
+                            const bool hf = frame_of(id) == FR_H, mir = mirrored(id, MERGED);
+                            const int plen = hf ? lenw : lenh, p0 = mir ? plen - 1 - q0 : q0;
                             const ptrdiff_t ps = hf ? p.C : (ptrdiff_t)p.W * p.C;
-                            f(yi + line * (hf ? (ptrdiff_t)p.W * p.C : p.C) + p0 * ps, mir ? -ps : ps);
+                            f(out(gi, hf ? line : p0, hf ? p0 : line), mir ? -ps : ps, act ? plen - q0 : 0);
                         };
-                        if constexpr (WG) place([&](T *q, ptrdiff_t ps) { load_line<T, LT>(q, ps, O, act ? plen - q0 : 0); });
+                        if constexpr (WG) place(id, line, gi, q0, [&](T *q, ptrdiff_t ps, int left) { load_line<T, LT>(q, ps, O, left); });
                         else {
 #pragma unroll
                             for (int o = 0; o < LT; o++) O[o] = bias;
@@ -698,42 +712,44 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
 #pragma unroll
                             for (int o = 0; o < LT; o++) add2(dbias, O[o]);
                         } else
-                            place([&](T *q, ptrdiff_t ps) { store_line<T, LT>(q, ps, O, act ? plen - q0 : 0, all, mask); });
+                            place(anew(id), anew(line), anew(gi), anew(q0), [&](T *q, ptrdiff_t ps, int left) { store_line<T, LT>(q, ps, O, left, all, mask); });
                     } else {
                         f32x2 O[kTD];
-                        // per position: dh rows down, dw pixels to the right
-                        const int dh = mir ? -1 : 1, dw = (id == 2) == mir ? 1 : -1, w = dw > 0 ? line - (kTD - 1) : line;
-                        auto in = [&](int o) { return act && q0 + o < plen && (unsigned)(w + o * dw) < (unsigned)lenw; };
-                        if constexpr (WG) {
-                            const T *q = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
-                            const ptrdiff_t ps = ((ptrdiff_t)dh * p.W + dw) * p.C;
+                        // per position: a row up, dw pixels to the right
+                        const int dw = id == 2 ? 1 : -1, w = dw > 0 ? line - (kTD - 1) : line;
+                        auto outputs = [&](int id, int line, int gi, int q0, auto &&f) {
+                            const int dw = id == 2 ? 1 : -1, w = dw > 0 ? line - (kTD - 1) : line;
+                            T *q = out(gi, lenh - 1 - q0, w);
+                            const ptrdiff_t ps = ((ptrdiff_t)dw - p.W) * p.C;
 #pragma unroll
-                            for (int o = 0; o < kTD; o++) { O[o] = Pair<T>::ldg_if(in(o), q); q += ps; }
+                            for (int o = 0; o < kTD; o++) {
+                                f(o, q, act && q0 + o < lenh && (unsigned)(w + o * dw) < (unsigned)lenw);
+                                q += ps;
+                            }
+                        };
+                        if constexpr (WG) {
+                            outputs(id, line, gi, q0, [&](int o, const T *q, bool in) { O[o] = Pair<T>::ldg_if(in, q); });
                         } else {
 #pragma unroll
                             for (int o = 0; o < kTD; o++) O[o] = bias;
                         }
                         // where the diagonal enters and leaves the tile (at the zeros around a whole map), from the block's first position
-                        const int f = max(dw > 0 ? ge.plo_w - w : w - ge.phi_w, dh > 0 ? ge.plo_h - p0 : p0 - ge.phi_h);
-                        const int l = min(dw > 0 ? ge.phi_w - w : w - ge.plo_w, dh > 0 ? ge.phi_h - p0 : p0 - ge.plo_h);
+                        const int f = max(dw > 0 ? ge.plo_w - w : w - ge.phi_w, p0 - ge.phi_h);
+                        const int l = min(dw > 0 ? ge.phi_w - w : w - ge.plo_w, p0 - ge.plo_h);
                         // (a diagonal that misses the tile reads its first row, zeros around a whole map)
                         const bool miss = f > l;
                         line_body<T, KIND_DIAG, R, kTD, WG, MERGED>(miss ? gt + ge.plo_h * row_bytes : gt + p0 * row_bytes + w * px,
-                                                                    dh * row_bytes + dw * px, miss ? 0 : f, miss ? 0 : l,
+                                                                    dw * px - row_bytes, miss ? 0 : f, miss ? 0 : l,
                                                                     q0 > 0 || ge.halo_h, q0 + kTD < plen || ge.halo_h, O, Wt);
                         if constexpr (WG) {
 #pragma unroll
                             for (int o = 0; o < kTD; o++) add2(dbias, O[o]);
                         } else {
-                            T *yl = yi + ((ptrdiff_t)p0 * p.W + w) * p.C;
-                            const ptrdiff_t ps = ((ptrdiff_t)dh * p.W + dw) * p.C;
-#pragma unroll
-                            for (int o = 0; o < kTD; o++) {
-                                if (in(o)) {
-                                    if (all) Pair<T>::st(yl, O[o]); else store_pair(yl, O[o], mask);
+                            outputs(anew(id), anew(line), anew(gi), anew(q0), [&](int o, T *q, bool in) {
+                                if (in) {
+                                    if (all) Pair<T>::st(q, O[o]); else store_pair(q, O[o], mask);
                                 }
-                                yl += ps;
-                            }
+                            });
                         }
                     }
                     };
@@ -837,7 +853,7 @@ seg_wgrad_final_kernel(const float *__restrict__ partial, const int8_t *__restri
         if (c >= p.C || (k < 31 ? k >= p.K : db == nullptr)) continue;
         int at = 31;
         if (k < 31) {
-            const int kind = kind_of(chan[c]), t = k - p.K / 2 + kHalf;
+            const int id = chan[c], kind = kind_of(id), j = k - p.K / 2 + kHalf, t = backwards(id, true) ? kMaxTaps - 1 - j : j;
             at = kind == KIND_SLANT ? (t == 14 || t == 16 ? 15 : t) : kind == KIND_DIAG ? g_diag_at[t] : t;
         }
         float sum = 0.f;

@@ -8,8 +8,8 @@
 namespace o1d {
 
 constexpr int kSegGeos = 6, kSegRuns = 20;
-// Order of the sums (o1d_seg.cuh): any; taps ascending; as the tiled kernels.
-enum : int { SEG_UNSET = 0, SEG_ANY, SEG_ASCENDING, SEG_TILED };
+// Order of the sums (o1d_seg.cuh): taps ascending, or as in the tiled kernels (the faster one).
+enum : int { SEG_UNSET = 0, SEG_ASCENDING, SEG_TILED };
 
 // How the maps of a run of chunks are cut into items: G whole images, or one tile of an image.
 struct SegGeo {
@@ -35,7 +35,6 @@ struct SegParams {
     int nruns, per_chunk;
     int off_tile, off_tab, off_bar;
     int flip, identity;
-    int tiled_order;                     // order of the sums, see o1d_seg.cuh
     long long total_cost;
     SegGeo geo[kSegGeos];
     SegRun run[kSegRuns];
@@ -54,7 +53,7 @@ bool seg_configure(const int8_t *chan, int N, int H, int W, int C, int K, int es
                    SegConfig **cfg);
 
 // y = conv(x) + bias (flip = 1: input gradient).  w, bias fp32, or bf16 when wbf16 is set.
-// order: SEG_ANY is the fastest.
+// order: SEG_ASCENDING (bf16 only) or SEG_TILED.
 cudaError_t seg_launch_conv(const SegConfig &cfg, const SegMaps &maps, const void *w, const void *bias, int wbf16,
                             const int8_t *chan, void *y, int flip, int identity, int order, int *err_flag, cudaStream_t st);
 

@@ -58,3 +58,23 @@ def test_segments_equal_general(shape, dtype):
         assert float((a - b).abs().max()) <= 1e-4 * float(b.abs().max())
     again = run(0)[0]
     assert all(torch.equal(a, b) for a, b in zip(got, again))        # same bits again
+
+
+# bf16 sums have the bits of a family that the shape would otherwise take (2: tiled, 3: direct)
+@pytest.mark.parametrize("shape", [(2, 56, 56, 96, 31), (8, 28, 28, 96, 31), (3, 28, 28, 192, 31), (33, 14, 14, 384, 31), (1, 13, 29, 32, 15)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_bits_of_the_family_replaced(shape):
+    N, H, W, C, K = shape
+    x = torch.randn((N, H, W, C), device=DEV).to(torch.bfloat16)
+    w, bias = 0.1 * torch.randn((C, 1, 1, K), device=DEV), torch.randn((C,), device=DEV)
+    plan = _plan("model", C, K)
+
+    def run(route):
+        try:
+            o1d.ops.set_route(route)
+            return o1d.fprop(x, w, bias, plan, 1, True, True), o1d.dgrad(x, w, plan, H, W, 1, True)
+        finally:
+            o1d.ops.set_route(0)
+
+    got = run(0)
+    assert any(all(torch.equal(a, b) for a, b in zip(got, run(route))) for route in (2, 3))
