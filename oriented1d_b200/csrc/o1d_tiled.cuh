@@ -480,7 +480,9 @@ tiled_nhwc_kernel(const __grid_constant__ CUtensorMap tmap, const float *__restr
                 }
             }
         }
-        if (p.rezero) {
+        // A chunk of other lines may lay its planes out with the other pitch: the zeros around the lines are
+        // then where the previous chunk had pixels.
+        if (p.rezero || (new_chunk && it > 0 && p.pitch_n != p.pitch_t)) {
             for (int i = tid; i < p.off_zero - 32; i += nt) sm[p.off_planar + 32 + i] = 0.f;
         }
         if (new_chunk || p.rezero) __syncthreads();

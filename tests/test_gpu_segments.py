@@ -61,7 +61,7 @@ def test_segments_equal_general(shape, dtype):
 
 
 # bf16 sums have the bits of a family that the shape would otherwise take (2: tiled, 3: direct)
-@pytest.mark.parametrize("shape", [(2, 56, 56, 96, 31), (8, 28, 28, 96, 31), (3, 28, 28, 192, 31), (33, 14, 14, 384, 31), (1, 13, 29, 32, 15)],
+@pytest.mark.parametrize("shape", [(2, 56, 56, 96, 31), (8, 28, 28, 96, 31), (64, 28, 28, 96, 31), (3, 28, 28, 192, 31), (33, 14, 14, 384, 31), (1, 13, 29, 32, 15)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_bits_of_the_family_replaced(shape):
     N, H, W, C, K = shape
