@@ -58,10 +58,12 @@ bool choose_geo(const Chunk &k, const SegParams &p, int room, int LT, SegGeo *ou
     double best = 0;
     for (int nth = 1; nth <= 64; nth++) {
         const int TH = ceil_div(p.H, nth);
-        if (nth > 1 && (TH < 6 || ceil_div(p.H, TH) != nth)) continue;
+        if (nth > 1 && TH < 6) break;
+        if (ceil_div(p.H, TH) != nth) continue;
         for (int ntw = 1; ntw <= 64; ntw++) {
             const int TW = ceil_div(p.W, ntw);
-            if (ntw > 1 && (TW < 6 || ceil_div(p.W, TW) != ntw)) continue;
+            if (ntw > 1 && TW < 6) break;
+            if (ceil_div(p.W, TW) != ntw) continue;
             SegGeo g{};
             g.nth = nth; g.ntw = ntw; g.TH = TH; g.TW = TW;
             g.halo_h = nth > 1; g.halo_w = ntw > 1;
