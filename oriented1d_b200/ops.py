@@ -44,7 +44,6 @@ class Plan:
         check(lib.o1d_plan_build(th.data_ptr(), self.C, self.K, self.host.data_ptr()), "o1d_plan_build")
         self.num_classes = lib.o1d_plan_num_classes(self.host.data_ptr())
         self._dev: dict[torch.device, torch.Tensor] = {}
-        self._ptrs: dict = {}                # device index -> addresses of the host and the device copy
 
     def on(self, device: torch.device) -> torch.Tensor:
         d = self._dev.get(device)
@@ -55,13 +54,12 @@ class Plan:
 
     def pointers(self, t: torch.Tensor):
         """Addresses of the two copies for a call on t's device ((0, 0) when t is not on one: the
-        call then reports what is wrong with its arguments)."""
-        p = self._ptrs.get(t.get_device())
-        if p is None:
-            if not t.is_cuda:
-                return 0, 0
-            p = self._ptrs[t.get_device()] = (self.host.data_ptr(), self.on(t.device).data_ptr())
-        return p
+        call then reports what is wrong with its arguments).  Taken from the tensors at each call:
+        a copy of a plan has tensors of its own, and an address kept beside them would still name
+        the original's."""
+        if not t.is_cuda:
+            return 0, 0
+        return self.host.data_ptr(), self.on(t.device).data_ptr()
 
 
 def fprop(x, w, bias, plan: Plan, stride: int = 1, nhwc: bool = False, add_identity: bool = False,

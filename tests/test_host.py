@@ -195,6 +195,23 @@ def test_plan_cache_does_not_outlive_its_angles():
     assert b is not a and b.host[:64].view(torch.int32).tolist()[4] == 15
 
 
+@pytest.mark.parametrize("how", ["deepcopy", "copy", "pickle"])
+def test_a_copied_plan_has_addresses_of_its_own(how):
+    """A copy outlives its original: a call with it must get the addresses of the copy's tensors."""
+    import copy
+    import pickle
+    import types
+    here = types.SimpleNamespace(is_cuda=True, device=torch.device("cpu"), get_device=lambda: 0)   # a tensor "on a device"
+    plan = o1d.Plan(angle_list("model", 64), 31)
+    assert plan.pointers(here) == (plan.host.data_ptr(), plan.on(here.device).data_ptr())
+    other = {"deepcopy": copy.deepcopy, "copy": copy.copy, "pickle": lambda p: pickle.loads(pickle.dumps(p))}[how](plan)
+    assert other.pointers(here) == (other.host.data_ptr(), other.on(here.device).data_ptr())
+    assert torch.equal(other.host, plan.host)
+    # tensors that move under a plan (shared memory for another process) are followed too
+    plan.host = plan.host.clone()
+    assert plan.pointers(here)[0] == plan.host.data_ptr()
+
+
 def test_last_route_starts_unset():
     import threading
     out = []
