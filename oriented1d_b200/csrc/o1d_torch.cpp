@@ -180,7 +180,20 @@ Tensor transpose(const Tensor &t_, bool to_nhwc) {
     return out;
 }
 
+// The kernels read `expected` elements of a parameter: a shorter buffer would be read past its end.
+void need_numel(const Tensor &t, int64_t expected, const char *what) {
+    if (t.numel() != expected)
+        throw py::value_error(std::string(what) + " has " + std::to_string(t.numel()) + " elements, expected " + std::to_string(expected));
+}
+// Length of the last axis of a tensor that is normalised or summed by rows.
+int64_t row_length(const Tensor &x) {
+    if (x.dim() == 0 || x.numel() == 0) throw py::value_error("expected a tensor with at least one row");
+    return x.size(-1);
+}
+
 Tensor layer_norm_cl(const Tensor &x_, const Tensor &g, const Tensor &b, double eps, bool gelu) {
+    need_numel(g, row_length(x_), "weight");
+    need_numel(b, row_length(x_), "bias");
     need_cuda(x_); need_cuda(g); need_cuda(b);
     const c10::cuda::CUDAGuard guard(x_.device());
     const Tensor x = x_.contiguous();
@@ -199,16 +212,17 @@ Tensor layer_norm_cl(const Tensor &x_, const Tensor &g, const Tensor &b, double 
 // dx, dweight, dbias; the last two in fp32, or in the parameters' dtype when `as_params` is set.
 std::tuple<Tensor, Tensor, Tensor> layer_norm_cl_bwd(const Tensor &x_, const Tensor &dy_, const Tensor &g, double eps, const OptTensor &b,
                                                      bool gelu, bool as_params) {
-    need_cuda(x_); need_cuda(dy_); need_cuda(g);
-    const Tensor x = x_.contiguous(), dy = dy_.contiguous();
-    if (dy.sizes() != x.sizes() || dy.scalar_type() != x.scalar_type()) {
+    if (dy_.sizes() != x_.sizes() || dy_.scalar_type() != x_.scalar_type()) {
         std::ostringstream s;
-        s << "dy " << dy.sizes() << " " << dy.scalar_type() << " does not match x " << x.sizes() << " " << x.scalar_type();
+        s << "dy " << dy_.sizes() << " " << dy_.scalar_type() << " does not match x " << x_.sizes() << " " << x_.scalar_type();
         throw py::value_error(s.str());
     }
-    const int64_t C = x.size(-1), rows = x.numel() / C;
-    if (g.numel() != C) throw py::value_error("weight has " + std::to_string(g.numel()) + " elements, expected " + std::to_string(C));
+    const int64_t C = row_length(x_), rows = x_.numel() / C;
+    need_numel(g, C, "weight");
     if (gelu && (!b || b->numel() != C)) throw py::value_error("gelu=True needs the forward call's bias");
+    need_cuda(x_); need_cuda(dy_); need_cuda(g);
+    if (gelu) need_cuda(b);
+    const Tensor x = x_.contiguous(), dy = dy_.contiguous();
     const c10::cuda::CUDAGuard guard(x.device());
     const int code = dtype_code(x);
     Params p(g, gelu ? b : OptTensor());
@@ -228,10 +242,10 @@ std::tuple<Tensor, Tensor, Tensor> layer_norm_cl_bwd(const Tensor &x_, const Ten
 }
 
 Tensor colsum(const Tensor &x_, bool bf16) {
+    const int64_t C = row_length(x_), rows = x_.numel() / C;
     need_cuda(x_);
     const c10::cuda::CUDAGuard guard(x_.device());
     const Tensor x = x_.contiguous();
-    const int64_t C = x.size(-1), rows = x.numel() / C;
     const int code = dtype_code(x);
     Tensor out = at::empty({C}, x.options().dtype(bf16 ? at::kBFloat16 : at::kFloat));
     const size_t bytes = o1d_colsum_workspace_bytes(rows, (int)C, code);

@@ -164,6 +164,28 @@ def test_shape_mismatches_raise_before_any_launch():
         m.wgrad(torch.zeros(2, 8, 6, 5), x, torch.zeros(8))
 
 
+def test_layer_norm_parameters_of_the_wrong_length_raise():
+    """Every channel's weight and bias are read: shorter ones would be read past their end."""
+    x, ok = torch.zeros(4, 16), torch.ones(16)
+    for short in (torch.ones(15), torch.ones(8), torch.ones(0)):
+        for call in (o1d.ops.layer_norm_cl, lambda *a: o1d.ops.LayerNormCL.apply(*a, 1e-6)):
+            with pytest.raises(ValueError, match="weight has"):
+                call(x, short, ok)
+            with pytest.raises(ValueError, match="bias has"):
+                call(x, ok, short)
+        with pytest.raises(ValueError, match="weight has"):
+            o1d.ops.layer_norm_cl_bwd(x, x, short)
+        with pytest.raises(ValueError, match="bias"):
+            o1d.ops.layer_norm_cl_bwd(x, x, ok, 1e-6, short, True)
+    for none in (torch.zeros(4, 0), torch.zeros(0, 16), torch.zeros(())):
+        with pytest.raises(ValueError, match="at least one row"):
+            o1d.ops.layer_norm_cl(none, ok, ok)
+        with pytest.raises(ValueError, match="at least one row"):
+            o1d.ops.colsum(none)
+    with pytest.raises(RuntimeError, match="CUDA"):          # lengths are right: the device is what is left to refuse
+        o1d.ops.layer_norm_cl(x, ok, ok)
+
+
 def test_plan_cache_does_not_outlive_its_angles():
     """The 5-callable module caches plans per theta tensor.  A second tensor with other angles
     must get its own plan even if the allocator reuses the first one's address."""
