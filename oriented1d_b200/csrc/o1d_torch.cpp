@@ -256,7 +256,11 @@ Tensor colsum(const Tensor &x_, bool bf16) {
 }
 
 Tensor pointwise_in(const Tensor &x_, const Tensor &w, const OptTensor &bias) {
-    need_cuda(x_); need_cuda(w);
+    if (x_.dim() != 4) throw py::value_error("expected a 4-D tensor");
+    if (w.dim() == 0) throw py::value_error("weight must be [Cout, Cin]");
+    need_numel(w, w.size(0) * x_.size(1), "weight");
+    if (bias) need_numel(*bias, w.size(0), "bias");
+    need_cuda(x_); need_cuda(w); need_cuda(bias);
     const c10::cuda::CUDAGuard guard(x_.device());
     const Tensor x = x_.contiguous();
     const int code = dtype_code(x);

@@ -186,6 +186,21 @@ def test_layer_norm_parameters_of_the_wrong_length_raise():
         o1d.ops.layer_norm_cl(x, ok, ok)
 
 
+def test_pointwise_parameters_of_the_wrong_length_raise():
+    """The stem projection reads Cout x Cin weights and Cout biases."""
+    x, w, b = torch.zeros(2, 3, 8, 8), torch.zeros(64, 3), torch.zeros(64)
+    with pytest.raises(ValueError, match="weight has"):
+        o1d.ops.pointwise_in(x, torch.zeros(64, 2), b)
+    with pytest.raises(ValueError, match="bias has"):
+        o1d.ops.pointwise_in(x, w, torch.zeros(63))
+    with pytest.raises(ValueError, match="4-D"):
+        o1d.ops.pointwise_in(x[0], w, b)
+    with pytest.raises(ValueError, match="Cout"):
+        o1d.ops.pointwise_in(x, torch.zeros(()), b)
+    with pytest.raises(RuntimeError, match="CUDA"):
+        o1d.ops.pointwise_in(x, w, b)
+
+
 def test_plan_cache_does_not_outlive_its_angles():
     """The 5-callable module caches plans per theta tensor.  A second tensor with other angles
     must get its own plan even if the allocator reuses the first one's address."""
