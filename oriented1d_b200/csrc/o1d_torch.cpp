@@ -78,6 +78,10 @@ void check_params(int64_t plan_c, int64_t K, int64_t C, const Tensor *w, const O
     if (bias && *bias && (*bias)->numel() != C)
         throw py::value_error("bias has " + std::to_string((*bias)->numel()) + " elements, expected C = " + std::to_string(C));
 }
+// Extents of an output are divided by the stride before the library sees it.
+void need_stride(int64_t stride) {
+    if (stride <= 0) throw py::value_error("stride must be positive, got " + std::to_string(stride));
+}
 std::vector<int64_t> shape(int64_t n, int64_t h, int64_t w, int64_t c, bool nhwc) {
     return nhwc ? std::vector<int64_t>{n, h, w, c} : std::vector<int64_t>{n, c, h, w};
 }
@@ -85,6 +89,7 @@ std::vector<int64_t> shape(int64_t n, int64_t h, int64_t w, int64_t c, bool nhwc
 Tensor fprop(const Tensor &x_, const Tensor &w, const OptTensor &bias, int64_t plan_c, int64_t K, int64_t host, int64_t dev,
              int64_t stride, bool nhwc, bool identity, bool gelu) {
     const Dims d = dims(x_, nhwc);
+    need_stride(stride);
     check_params(plan_c, K, d.c, &w, &bias);
     need_cuda(x_); need_cuda(w); need_cuda(bias);
     const c10::cuda::CUDAGuard guard(x_.device());
@@ -104,6 +109,7 @@ Tensor fprop(const Tensor &x_, const Tensor &w, const OptTensor &bias, int64_t p
 Tensor dgrad(const Tensor &dy_, const Tensor &w, int64_t plan_c, int64_t K, int64_t host, int64_t dev, int64_t H, int64_t W,
              int64_t stride, bool nhwc, bool identity, const OptTensor &pre_) {
     const Dims d = dims(dy_, nhwc);
+    need_stride(stride);
     if (d.h != (H + stride - 1) / stride || d.w != (W + stride - 1) / stride)
         throw py::value_error("dy extents do not match ceil(H/stride) x ceil(W/stride)");
     check_params(plan_c, K, d.c, &w, nullptr);
@@ -132,6 +138,7 @@ std::tuple<Tensor, OptTensor> wgrad(const Tensor &dy_, const Tensor &x_, int64_t
                                     int64_t stride, bool nhwc, bool with_bias, bool gelu, bool bf16) {
     if (dy_.scalar_type() != x_.scalar_type()) throw py::type_error("dy and x must have the same dtype");
     const Dims d = dims(x_, nhwc);
+    need_stride(stride);
     check_params(plan_c, K, d.c, nullptr, nullptr);
     const auto want = shape(d.n, (d.h + stride - 1) / stride, (d.w + stride - 1) / stride, d.c, nhwc);
     if (dy_.sizes() != at::IntArrayRef(want)) {

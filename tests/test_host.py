@@ -159,6 +159,13 @@ def test_shape_mismatches_raise_before_any_launch():
         o1d.fprop(torch.zeros(2, 4, 6, 6), w, None, plan)
     with pytest.raises(ValueError, match="dy extents"):
         o1d.dgrad(torch.zeros(2, 8, 3, 3), w, plan, 6, 6, 1)
+    for stride in (0, -1):                                  # extents are divided by it
+        with pytest.raises(ValueError, match="stride"):
+            o1d.fprop(x, w, None, plan, stride)
+        with pytest.raises(ValueError, match="stride"):
+            o1d.dgrad(x, w, plan, 6, 6, stride)
+        with pytest.raises(ValueError, match="stride"):
+            o1d.wgrad(x, x, plan, stride)
     m = o1d.get_dwoconv1d_kernel("float", 7, 1, 3)
     with pytest.raises(ValueError, match="dy has shape"):
         m.wgrad(torch.zeros(2, 8, 6, 5), x, torch.zeros(8))
