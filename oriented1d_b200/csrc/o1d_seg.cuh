@@ -82,6 +82,13 @@ __device__ __noinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err_
     *err_flag = 1;
     return false;
 }
+// One more warp is through with a buffer; true for the last of the kWarps, and the count starts over.  Acquire
+// and release: every warp's reads of the buffer come before the refill that the last one issues.
+__device__ __forceinline__ bool last_warp(int *count) {
+    uint32_t before;
+    asm volatile("atom.acq_rel.cta.shared::cta.inc.u32 %0, [%1], %2;" : "=r"(before) : "r"(smem_u32(count)), "n"(kWarps - 1) : "memory");
+    return before == kWarps - 1;
+}
 __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0, int c1, int c2, int c3) {
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
@@ -766,10 +773,7 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
                 }
             }
             __syncwarp();
-            if (lane == 0 && atomicAdd(&cnt[buf], 1) == kWarps - 1) {       // last warp through: refill
-                cnt[buf] = 0;
-                if (s + ge.nbuf < nitems) issue(g, s + ge.nbuf, buf);
-            }
+            if (lane == 0 && last_warp(&cnt[buf]) && s + ge.nbuf < nitems) issue(g, s + ge.nbuf, buf);
             if (++buf == ge.nbuf) buf = 0;
         }
         if constexpr (WG) {

@@ -25,6 +25,11 @@ SHAPES = [(1, 1, 1, 16, 31, "one2"), (3, 1, 29, 16, 31, "one1"), (2, 30, 1, 8, 1
           (1, 99, 301, 16, 31, "one6"), (1, 300, 301, 8, 31, "one4")]
 
 
+# buffers refilled many times while the warps are at different items: lines of unequal cost in one chunk, two
+# buffers and four, whole images and cut ones
+SHAPES += [(2500, 28, 14, 32, 31, "model+"), (900, 32, 33, 16, 31, "model"), (24, 150, 150, 48, 31, "model+")]
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
 def test_segments_equal_general(shape, dtype):
