@@ -596,8 +596,10 @@ seg_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ SegMaps
         const SegGeo &ge = p.geo[p.run[g.run].geo];
         const int c0 = (p.run[g.run].chunk0 + g.chunk) * p.CC, tiles = ge.nth * ge.ntw, row_bytes = ge.P * p.px, px = p.px;
         const int nitems = g.count();
-        if (WG) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();                         // the previous segment is done with tables and buffers
+        // The previous segment is done with tables and buffers.  What it stored there itself (pixels of zeros, where
+        // its buffers ended; sums over the warps) comes before the copies issued below.
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
         if (tid == 0) {
 #pragma unroll 1
             for (int b = 0; b < ge.nbuf && b < nitems; b++) issue(g, b, b);

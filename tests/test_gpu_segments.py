@@ -28,6 +28,8 @@ SHAPES = [(1, 1, 1, 16, 31, "one2"), (3, 1, 29, 16, 31, "one1"), (2, 30, 1, 8, 1
 # buffers refilled many times while the warps are at different items: lines of unequal cost in one chunk, two
 # buffers and four, whole images and cut ones
 SHAPES += [(2500, 28, 14, 32, 31, "model+"), (900, 32, 33, 16, 31, "model"), (24, 150, 150, 48, 31, "model+")]
+# more chunks than a third of the CTAs: a CTA goes from one cut of the map, and size of the buffers, to another
+SHAPES += [(2, 30, 61, 2048, 31, "model"), (3, 28, 100, 1536, 31, "model")]
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
