@@ -1030,9 +1030,9 @@ def main():
     ap.add_argument("--batch", type=int, default=64, help="batch for --case")
     ap.add_argument("--reps", type=int, default=3, help="launches for --case")
     ap.add_argument("--angles", default="rr", choices=["rr", "block", "zero"], help="channel->orientation map for --case")
-    ap.add_argument("--route", type=int, default=0, choices=[0, 1, 2, 3, 4, 5],
+    ap.add_argument("--route", type=int, default=0, choices=[0, 1, 2, 3, 4, 5, 6],
                     help="kernel family: 0 automatic (default), 1 general only, 2 prefer tiled, 3 prefer direct, "
-                         "4 prefer whole-line")
+                         "4 prefer whole-line, 5 prefer walker, 6 prefer segments")
     ap.add_argument("--fuse-gelu", action="store_true",
                     help="train workload: apply each block's GELU inside its second oriented conv's kernels")
     ap.add_argument("--graph-collective", action="store_true",

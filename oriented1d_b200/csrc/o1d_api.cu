@@ -27,7 +27,7 @@ namespace {
 thread_local char g_err[256] = "";
 thread_local int g_last_route = O1D_ROUTE_NONE;   // kernel family of this thread's last operator call
 int g_force_generic = 0;   // o1d_set_route(): 1 = general kernels only (testing aid)
-int g_prefer = 0;          // o1d_set_route(): 2 = prefer the tiled kernels, 3 = direct, 4 = whole-line, 5 = walker
+int g_prefer = 0;          // o1d_set_route(): 2 = prefer the tiled kernels, 3 = direct, 4 = whole-line, 5 = walker, 6 = segments
 
 int cuda_fail(cudaError_t e, const char *what) {
     snprintf(g_err, sizeof(g_err), "%s: %s", what, cudaGetErrorString(e));
@@ -364,7 +364,7 @@ int try_seg(const void *x, const void *w, const void *bias, int wbf16, const Pla
     PlanView pv = plan_view(plan_dev, ph);
     const cudaError_t e = seg_launch_conv(*cfg, maps, w, bias, wbf16, pv.chan, y, flip, add_identity, order, flag, st);
     if (e != cudaSuccess) return cuda_fail(e, "segment fprop launch");
-    g_last_route = O1D_ROUTE_DIRECT;
+    g_last_route = O1D_ROUTE_SEGMENTS;
     return O1D_OK;
 }
 
@@ -423,10 +423,13 @@ int try_walk(const void *x, const float *w, const float *bias, const PlanHeader 
 }
 
 // Route of a forward-type call (flip = 1: stride-1 input gradient):
-//   1. direct kernels when one tile holds a whole image (small maps),
-//   2. tiled kernels (canonical lines, stride 1, sizes in multiples of 7/8),
-//   3. direct kernels with row/column tiles (stems, large maps, arbitrary angles),
-//   4. general kernels (the caller falls through on kNotTiled).
+//   1. segment kernels (NHWC, stride 1, neighbouring channels mostly on one canonical line; not 7x7),
+//   2. plane kernels (7x7, canonical lines),
+//   3. walker and whole-line kernels, for the fp32 stage maps where they are the faster ones,
+//   4. direct kernels when one tile holds several whole images, or where the tiled ones would idle,
+//   5. tiled kernels (canonical lines, stride 1, sizes in multiples of 7/8),
+//   6. direct kernels with row/column tiles (stems, large maps, arbitrary angles),
+//   7. general kernels (the caller falls through on kNotTiled).
 int route_forward(const void *x, const float *w, const float *bias, int wbf16, const PlanHeader &ph, const void *plan_host,
                   const void *plan_dev, void *y, int N, int H, int W, int C, int K, int stride, int layout,
                   int dtype, int add_identity, int flip, int act, const void *pre, cudaStream_t st,
@@ -438,7 +441,7 @@ int route_forward(const void *x, const float *w, const float *bias, int wbf16, c
                          flip, act, pre, st, d);
     // Neighbouring channels on one canonical line: packed-FMA segments, everywhere but on 7x7 maps, which fill
     // half of a segment (7x7x4096, batch 64: 92 us against 35 us for the plane kernels).
-    if (g_prefer == 0 && !(H == 7 && W == 7)) {
+    if (g_prefer == 6 || (g_prefer == 0 && !(H == 7 && W == 7))) {
         rc = try_seg(x, w, bias, wbf16, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip,
                      st, d);
         if (rc != kNotTiled) return rc;
@@ -591,7 +594,7 @@ int try_seg_wgrad(const void *dy, const void *x, const PlanHeader &ph, const voi
     PlanView pv = plan_view(plan_dev, ph);
     const cudaError_t e = seg_launch_wgrad(*cfg, maps, dy_maps, pv.chan, dy, dw, db, out_bf16, (float *)workspace, flag, st);
     if (e != cudaSuccess) return cuda_fail(e, "segment wgrad launch");
-    g_last_route = O1D_ROUTE_DIRECT;
+    g_last_route = O1D_ROUTE_SEGMENTS;
     return O1D_OK;
 }
 
@@ -624,7 +627,7 @@ const char *o1d_last_error(void) { return g_err; }
 int o1d_last_route(void) { return g_last_route; }
 
 int o1d_set_route(int route) {
-    if (route < 0 || route > 5) return O1D_ERR_INVALID;
+    if (route < 0 || route > 6) return O1D_ERR_INVALID;
     g_force_generic = (route == 1);
     g_prefer = (route >= 2) ? route : 0;
     return O1D_OK;
@@ -855,7 +858,7 @@ int wgrad_dispatch(const void *dy, const void *x, const PlanHeader &ph, const vo
                    float *dw, float *db, void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K,
                    int stride, int layout, int dtype, int act, int out_bf16, cudaStream_t st, const DeviceInfo &d) {
     int rc;
-    if (g_prefer == 0 && !act && !(H == 7 && W == 7)) {       // see route_forward
+    if (!act && (g_prefer == 6 || (g_prefer == 0 && !(H == 7 && W == 7)))) {       // see route_forward
         rc = try_seg_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, out_bf16, workspace, workspace_bytes, N, H, W, C, K, stride,
                            layout, dtype, st, d);
         if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;

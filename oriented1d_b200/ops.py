@@ -171,11 +171,12 @@ def uses_tiled(plan: Plan, N: int, H: int, W: int, stride: int, nhwc: bool, dtyp
 def set_route(route) -> None:
     """Testing aid.  False/0: automatic choice; True/1: general kernels only; 2: prefer the
     tiled kernels; 3: prefer the direct kernels; 4: the whole-line kernels; 5: the walker kernels
-    (the last two serve square fp32 NHWC stage maps only and fall through elsewhere)."""
+    (these two serve square fp32 NHWC stage maps only and fall through elsewhere); 6: the segment
+    kernels, on 7x7 maps too."""
     check(lib.o1d_set_route(int(route)), "o1d_set_route")
 
 
-ROUTE_NAMES = {-1: "none", 0: "general", 1: "tiled", 2: "direct", 3: "plane7", 4: "lines", 5: "walk"}
+ROUTE_NAMES = {-1: "none", 0: "general", 1: "tiled", 2: "direct", 3: "plane7", 4: "lines", 5: "walk", 6: "segments"}
 
 
 def last_route() -> str:

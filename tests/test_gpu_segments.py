@@ -54,7 +54,7 @@ def test_segments_equal_general(shape, dtype):
 
     ref, _ = run(1)
     got, name = run(0)
-    assert name == "direct" and o1d.ops.device_status() == 0
+    assert name == "segments" and o1d.ops.device_status() == 0
     for a, b in zip(got[:2], ref[:2]):
         a, b = a.float(), b.float()
         if dtype == torch.float32:

@@ -263,6 +263,12 @@ def test_last_route_starts_unset():
     t.start(); t.join()
     assert out == [-1]                                    # per thread, no call made yet
     assert o1d.ops.ROUTE_NAMES[-1] == "none"
+    # every family that the header names has a name here, and the routes a caller may ask for are 0 .. 6
+    header = open(os.path.join(ROOT, "include", "o1d.h")).read()
+    ids = {int(v) for v in re.findall(r"O1D_ROUTE_[A-Z0-9]+ = (-?\d+)", header)}
+    assert ids == set(o1d.ops.ROUTE_NAMES) and len(set(o1d.ops.ROUTE_NAMES.values())) == len(ids)
+    with pytest.raises(ValueError):
+        o1d.ops.set_route(7)
 
 
 def test_cpu_tensors_are_refused():
