@@ -109,6 +109,11 @@ int o1d_selftest_wait_timeout(int *scratch_dev, void *stream);
 int o1d_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int stride,
                    int layout, int dtype);
 
+/* 1 if requests with O1D_FLAG_GELU_INPUT (forward and both gradients; NHWC, stride 1) would run on the
+ * tiled kernels, 0 if on the general ones.  Lets a host choose between activation on load and a
+ * pass of its own.  Host-only; no counterpart in the reference. */
+int o1d_gelu_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int dtype);
+
 /* Rasterised tap offsets of C channels, computed on the host exactly as the reference's
  * CPU loops do (kernels.cpp:37,43-44).  theta_host: C floats (radians, fp32);
  * dh, dw: C*K int8 each.  Requires K odd, K <= 255. */

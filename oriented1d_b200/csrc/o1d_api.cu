@@ -670,6 +670,19 @@ int o1d_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int
     return direct_configure(ph, plan_host, all, N, H, W, C, K, stride, layout, esize, 232448, 148, false, false, &dcfg) ? 1 : 0;
 }
 
+int o1d_gelu_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int dtype) {
+    if (bad_common(N, H, W, C, K, 1, O1D_NHWC, dtype) || g_force_generic) return 0;
+    PlanHeader ph;
+    if (check_plan(plan_host, C, K, &ph)) return 0;
+    for (int op : {OP_FPROP, OP_WGRAD}) {          // the input gradient is a forward call
+        TiledConfig cfg;
+        if (!tiled_configure(ph, plan_host, N, H, W, C, K, 1, O1D_NHWC, dtype == O1D_F32 ? 4 : 2, 232448, 148, op, &cfg) ||
+            !tiled_supports_act(cfg))
+            return 0;
+    }
+    return 1;
+}
+
 int o1d_offsets(const float *theta_host, int C, int K, int8_t *dh, int8_t *dw) {
     if (!theta_host || !dh || !dw || C <= 0 || K <= 0 || (K & 1) == 0 || K > 255) return O1D_ERR_INVALID;
     for (int c = 0; c < C; c++) raster(theta_host[c], K, dh + (size_t)c * K, dw + (size_t)c * K);

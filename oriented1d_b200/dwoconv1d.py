@@ -165,7 +165,7 @@ class DepthwiseOrientedConv1d(nn.Conv2d):
 
     def _gelu_in_kernel(self, x) -> bool:
         """The "auto" rule: activation on load only on maps of 28x28 and larger that the tiled
-        kernels serve anyway.  What it buys is memory (the GELU output is never stored, one 4*dim
+        kernels, the only fast ones with an activation, can serve.  What it buys is memory (the GELU output is never stored, one 4*dim
         activation less per block kept for backward), not time: the tiled kernels are bound by
         instruction issue, so the erf costs more there than the memory pass it removes (B200,
         ConvNeXt-B-1D++ training step, batch 64: 60.3 ms unfused, 63.5 ms with this rule, 74.1 ms
@@ -175,7 +175,7 @@ class DepthwiseOrientedConv1d(nn.Conv2d):
         if not (x.is_cuda and x.dim() == 4 and self.nhwc and self.stride[0] == 1):
             return False
         N, H, W, _ = x.shape
-        return H * W >= 28 * 28 and ops.uses_tiled(self._get_plan(), N, H, W, 1, True, x.dtype)
+        return H * W >= 28 * 28 and ops.gelu_uses_tiled(self._get_plan(), N, H, W, x.dtype)
 
     def _apply_op(self, x):
         gelu = self._gelu_in_kernel(x)

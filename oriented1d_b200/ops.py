@@ -168,6 +168,15 @@ def uses_tiled(plan: Plan, N: int, H: int, W: int, stride: int, nhwc: bool, dtyp
     return bool(lib.o1d_uses_tiled(plan.host.data_ptr(), N, H, W, plan.C, plan.K, stride, int(nhwc), code))
 
 
+def gelu_uses_tiled(plan: Plan, N: int, H: int, W: int, dtype: torch.dtype) -> bool:
+    """Would conv(GELU(x)) with the GELU applied on load (NHWC, stride 1) run on the tiled kernels (True)
+    or the general ones (False)?  No other family applies an activation."""
+    code = _DTYPES.get(dtype)
+    if code is None:
+        return False
+    return bool(lib.o1d_gelu_uses_tiled(plan.host.data_ptr(), N, H, W, plan.C, plan.K, code))
+
+
 def set_route(route) -> None:
     """Testing aid.  False/0: automatic choice; True/1: general kernels only; 2: prefer the
     tiled kernels; 3: prefer the direct kernels; 4: the whole-line kernels; 5: the walker kernels

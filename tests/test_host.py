@@ -256,6 +256,22 @@ def test_a_copied_plan_has_addresses_of_its_own(how):
     assert plan.pointers(here)[0] == plan.host.data_ptr()
 
 
+@pytest.mark.parametrize("shape,dtype,inside", [
+    ((2, 56, 56, 96), torch.bfloat16, True), ((2, 28, 28, 64), torch.float32, True),
+    ((2, 14, 14, 96), torch.bfloat16, False),                # small map: a pass of its own
+    ((2, 200, 333, 96), torch.bfloat16, False),              # a size that the tiled kernels refuse
+    ((2, 57, 56, 96), torch.float32, False),
+])
+def test_gelu_auto_stays_off_where_only_general_kernels_have_it(shape, dtype, inside):
+    import types
+    N, H, W, C = shape
+    m = o1d.DepthwiseOrientedConv1d(C, C, 31, groups=C, padding=15, nhwc=True, angle=[float(a) for a in angle_list("model", C)])
+    m.gelu_input = "auto"
+    x = types.SimpleNamespace(is_cuda=True, dim=lambda: 4, shape=shape, dtype=dtype)
+    assert m._gelu_in_kernel(x) is inside
+    assert o1d.ops.gelu_uses_tiled(o1d.Plan(angle_list("random", 96), 31), 2, 56, 56, dtype) is False
+
+
 def test_last_route_starts_unset():
     import threading
     out = []
