@@ -102,9 +102,9 @@ int o1d_device_status_clear(int *flag_out);
  * reads 1 until o1d_device_status_clear() is called.  (No counterpart in the reference.) */
 int o1d_selftest_wait_timeout(int *scratch_dev, void *stream);
 
-/* 1 if o1d_fprop would take one of the TMA-staged kernel families (tiled or direct) for this
- * request, 0 if the general kernels.  Lets a host decide whether converting an NCHW tensor
- * to NHWC first pays off (the tiled kernels are NHWC only).  Host-only; no counterpart in
+/* 1 if o1d_fprop would take one of the TMA-staged kernel families (tiled, direct or segments) for
+ * this request, 0 if the general kernels.  Lets a host decide whether converting an NCHW tensor
+ * to NHWC first pays off (those families are NHWC only).  Host-only; no counterpart in
  * the reference. */
 int o1d_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int stride,
                    int layout, int dtype);

@@ -319,6 +319,19 @@ int device_flag_ptr(int **out) {
     return O1D_OK;
 }
 
+// Configuration of the segment kernels for this request, null where they decline it; kept by the thread until
+// requests of other shapes displace it.
+SegConfig *seg_config(const PlanHeader &ph, const void *plan_host, int N, int H, int W, int C, int K, int stride, int layout, int esize,
+                      const DeviceInfo &d, bool wgrad) {
+    if (g_force_generic || !ph.all_canon || ph.chan_off == 0 || stride != 1 || layout != O1D_NHWC) return nullptr;
+    const int8_t *chan_host = reinterpret_cast<const int8_t *>(static_cast<const char *>(plan_host) + ph.chan_off);
+    SegConfig *cfg = nullptr;
+    return seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, wgrad, &cfg) ? cfg : nullptr;
+}
+// Maps that the automatic route leaves to other families: 7x7 fills half of a segment (7x7x4096, batch 64: 92 us
+// against 35 us for the plane kernels).
+bool seg_route(int H, int W) { return g_prefer == 6 || (g_prefer == 0 && !(H == 7 && W == 7)); }
+
 // Tensor maps of `t` for every way the configuration cuts it: the tiles with their halo, or the outputs alone.
 int seg_maps(const SegConfig &cfg, const void *t, bool with_halo, SegMaps *maps, const char *what) {
     const SegParams &p = cfg.p;
@@ -338,11 +351,9 @@ int seg_maps(const SegConfig &cfg, const void *t, bool with_halo, SegMaps *maps,
 int try_seg(const void *x, const void *w, const void *bias, int wbf16, const PlanHeader &ph, const void *plan_host,
             const void *plan_dev, void *y, int N, int H, int W, int C, int K, int stride, int layout, int dtype,
             int add_identity, int flip, cudaStream_t st, const DeviceInfo &d) {
-    if (g_force_generic || !ph.all_canon || ph.chan_off == 0 || stride != 1 || layout != O1D_NHWC) return kNotTiled;
     const int esize = dtype == O1D_F32 ? 4 : 2;
-    const int8_t *chan_host = reinterpret_cast<const int8_t *>(static_cast<const char *>(plan_host) + ph.chan_off);
-    SegConfig *cfg = nullptr;
-    if (!seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, false, &cfg)) return kNotTiled;
+    SegConfig *cfg = seg_config(ph, plan_host, N, H, W, C, K, stride, layout, esize, d, false);
+    if (!cfg) return kNotTiled;
     if (((uintptr_t)y & 15) != 0) return kNotTiled;
     // bf16 results have the bits of the family that the shape would otherwise take; fp32 ones the fastest order
     int order = SEG_TILED;
@@ -439,9 +450,7 @@ int route_forward(const void *x, const float *w, const float *bias, int wbf16, c
     if (act || pre)       // activation on load / its derivative on store: tiled kernels, else general
         return try_tiled(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity,
                          flip, act, pre, st, d);
-    // Neighbouring channels on one canonical line: packed-FMA segments, everywhere but on 7x7 maps, which fill
-    // half of a segment (7x7x4096, batch 64: 92 us against 35 us for the plane kernels).
-    if (g_prefer == 6 || (g_prefer == 0 && !(H == 7 && W == 7))) {
+    if (seg_route(H, W)) {     // neighbouring channels on one canonical line: packed-FMA segments
         rc = try_seg(x, w, bias, wbf16, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip,
                      st, d);
         if (rc != kNotTiled) return rc;
@@ -578,11 +587,8 @@ int try_direct_wgrad(const void *dy, const void *x, const PlanHeader &ph, const 
 int try_seg_wgrad(const void *dy, const void *x, const PlanHeader &ph, const void *plan_host, const void *plan_dev, void *dw,
                   void *db, int out_bf16, void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K,
                   int stride, int layout, int dtype, cudaStream_t st, const DeviceInfo &d) {
-    if (g_force_generic || !ph.all_canon || ph.chan_off == 0 || stride != 1 || layout != O1D_NHWC) return kNotTiled;
-    const int esize = dtype == O1D_F32 ? 4 : 2;
-    const int8_t *chan_host = reinterpret_cast<const int8_t *>(static_cast<const char *>(plan_host) + ph.chan_off);
-    SegConfig *cfg = nullptr;
-    if (!seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, true, &cfg)) return kNotTiled;
+    SegConfig *cfg = seg_config(ph, plan_host, N, H, W, C, K, stride, layout, dtype == O1D_F32 ? 4 : 2, d, true);
+    if (!cfg) return kNotTiled;
     if (((uintptr_t)dy & 15) != 0 || ((uintptr_t)workspace & 15) != 0) return kNotTiled;
     if (workspace_bytes < seg_wgrad_bytes(*cfg)) return O1D_ERR_WORKSPACE;
     SegMaps maps, dy_maps;
@@ -667,7 +673,9 @@ int o1d_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int
     if (tiled_configure(ph, plan_host, N, H, W, C, K, stride, layout, esize, 232448, 148, OP_FPROP, &cfg)) return 1;
     DirectConfig dcfg;
     const ChunkRange all{0, C / (32 / esize), ph.max_dh, ph.max_dw};
-    return direct_configure(ph, plan_host, all, N, H, W, C, K, stride, layout, esize, 232448, 148, false, false, &dcfg) ? 1 : 0;
+    if (direct_configure(ph, plan_host, all, N, H, W, C, K, stride, layout, esize, 232448, 148, false, false, &dcfg)) return 1;
+    // what those two refuse the segment kernels may take: channels that do not fill groups of 32 bytes
+    return seg_route(H, W) && seg_config(ph, plan_host, N, H, W, C, K, stride, layout, esize, {148, 232448}, false) != nullptr;
 }
 
 int o1d_gelu_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int dtype) {
@@ -871,7 +879,7 @@ int wgrad_dispatch(const void *dy, const void *x, const PlanHeader &ph, const vo
                    float *dw, float *db, void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K,
                    int stride, int layout, int dtype, int act, int out_bf16, cudaStream_t st, const DeviceInfo &d) {
     int rc;
-    if (!act && (g_prefer == 6 || (g_prefer == 0 && !(H == 7 && W == 7)))) {       // see route_forward
+    if (!act && seg_route(H, W)) {
         rc = try_seg_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, out_bf16, workspace, workspace_bytes, N, H, W, C, K, stride,
                            layout, dtype, st, d);
         if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;

@@ -161,7 +161,8 @@ def pointwise_in(x, weight, bias):
 
 
 def uses_tiled(plan: Plan, N: int, H: int, W: int, stride: int, nhwc: bool, dtype: torch.dtype) -> bool:
-    """Would this request run on the tiled kernels (True) or the general ones (False)?"""
+    """Would this request run on one of the TMA-staged families (tiled, direct, segments; True) or on the
+    general kernels (False)?"""
     code = _DTYPES.get(dtype)
     if code is None:
         return False

@@ -67,6 +67,33 @@ def test_segments_equal_general(shape, dtype):
     assert all(torch.equal(a, b) for a, b in zip(got, again))        # same bits again
 
 
+def test_nchw_module_of_odd_channel_groups():
+    """An NCHW bf16 layer whose channels do not fill groups of 32 bytes: the segment kernels behind two
+    layout steps, with the results of the general NCHW kernels."""
+    N, C, H, W, K = 3, 40, 20, 30, 31
+    m = o1d.DepthwiseOrientedConv1d(C, C, K, groups=C, padding=K // 2, angle=[float(a) for a in angle_list("model", C)]).to(DEV, torch.bfloat16)
+    with torch.no_grad():
+        m.weight.mul_(0.3)
+    x, dy = (torch.randn((N, C, H, W), device=DEV).to(torch.bfloat16) for _ in range(2))
+
+    def run(conv):
+        y = conv(x)
+        return (y, o1d.ops.last_route()) + torch.autograd.grad(y, (xr, m.weight, m.bias), dy)
+
+    xr = x.requires_grad_(True)
+    y, name, dx, dw, db = run(m)
+    assert name == "segments" and o1d.ops.device_status() == 0
+    try:
+        o1d.ops.set_route(1)
+        ry, rname, rdx, rdw, rdb = run(m)
+    finally:
+        o1d.ops.set_route(0)
+    assert rname == "general"
+    for a, b in ((y, ry), (dx, rdx), (dw, rdw), (db, rdb)):      # each rounds an fp32 sum: at most one bf16 ulp apart
+        a, b = a.detach().float(), b.detach().float()
+        assert float(((a - b).abs() / b.abs().clamp_min(1e-2 * float(b.abs().max()))).max()) <= 2 ** -7
+
+
 # bf16 sums have the bits of a family that the shape would otherwise take (2: tiled, 3: direct)
 @pytest.mark.parametrize("shape", [(2, 56, 56, 96, 31), (8, 28, 28, 96, 31), (64, 28, 28, 96, 31), (3, 28, 28, 192, 31), (33, 14, 14, 384, 31), (1, 13, 29, 32, 15)],
                          ids=lambda s: "x".join(map(str, s)))

@@ -272,6 +272,21 @@ def test_gelu_auto_stays_off_where_only_general_kernels_have_it(shape, dtype, in
     assert o1d.ops.gelu_uses_tiled(o1d.Plan(angle_list("random", 96), 31), 2, 56, 56, dtype) is False
 
 
+@pytest.mark.parametrize("H,W,C,mode,dtype,fast", [
+    (20, 30, 40, "model", torch.bfloat16, True),             # channels = 8 mod 16, a map the tiled kernels refuse: segments
+    (20, 30, 40, "random", torch.bfloat16, False),
+    (20, 30, 40, "rr", torch.bfloat16, False),               # pairs on two lines: general kernels
+    (20, 30, 48, "rr", torch.bfloat16, True),                # direct kernels
+    (28, 28, 96, "model", torch.bfloat16, True),
+    (20, 30, 44, "model", torch.float32, False),             # channels of the segment kernels come in eights
+])
+def test_nchw_layers_know_every_fast_family(H, W, C, mode, dtype, fast):
+    """The NCHW module converts the layout where NHWC has a fast path, whichever family that is."""
+    plan = o1d.Plan(angle_list(mode, C), 31)
+    assert o1d.ops.uses_tiled(plan, 4, H, W, 1, True, dtype) is fast
+    assert not o1d.ops.uses_tiled(plan, 4, H, W, 1, False, dtype)
+
+
 def test_last_route_starts_unset():
     import threading
     out = []
