@@ -30,70 +30,16 @@ from . import ops
 __all__ = ["DepthwiseOrientedConv1d", "get_dwoconv1d_kernel", "oriented_dwconv1d_get_module_from_params"]
 
 
-_native_dgrad, _native_wgrad = ops.dgrad, ops.wgrad
-
-
 def _via_nhwc(x, plan, stride) -> bool:
-    """Does an NCHW tensor go through its NHWC form?  Where that form has a fast path."""
+    """Does an NCHW tensor go through its NHWC form?  Where that form has a fast path: converting it on
+    the way in and out (two 128-bit transposes) costs far less than the general NCHW kernels, and the
+    NHWC copy is what is kept for backward.  The reference does the opposite: it converts NHWC inputs
+    to NCHW around NCHW-only kernels (dwoconv1d.py:25-26,36-37)."""
     if not x.is_cuda or x.dim() != 4:
         return False
     N, C, H, W = x.shape
     return (ops.uses_tiled(plan, N, H, W, stride, True, x.dtype)
             and not ops.uses_tiled(plan, N, H, W, stride, False, x.dtype))
-
-
-class _DepthwiseOrientedConv1d(torch.autograd.Function):
-    """Counterpart of the reference's autograd function (dwoconv1d.py:18-69).
-
-    NCHW inputs whose NHWC form qualifies for the tiled kernels are converted once on the
-    way in and out (two 128-bit transposes cost far less than the general NCHW kernels); the
-    NHWC copy of x is what is saved for backward.  The reference does the opposite: it
-    converts NHWC inputs to NCHW around NCHW-only kernels (dwoconv1d.py:25-26,36-37)."""
-
-    @staticmethod
-    def forward(ctx, x, w, theta, bias, plan, stride, nhwc=False, add_identity=False, gelu_input=False):
-        x = x.contiguous()
-        ctx.set_materialize_grads(False)
-        ctx.gelu_input = gelu_input
-        via_nhwc = not nhwc and not gelu_input and _via_nhwc(x, plan, stride)
-        ctx.plan, ctx.stride, ctx.nhwc, ctx.add_identity = plan, stride, nhwc, add_identity
-        ctx.via_nhwc = via_nhwc
-        ctx.has_bias = bias is not None
-        if via_nhwc:
-            xh = ops.nchw_to_nhwc(x)
-            ctx.save_for_backward(xh, w)
-            return ops.nhwc_to_nchw(ops.fprop(xh, w, bias, plan, stride, True, add_identity))
-        ctx.save_for_backward(x, w)
-        return ops.fprop(x, w, bias, plan, stride, nhwc, add_identity, gelu_input)
-
-    @staticmethod
-    def backward(ctx, dy):
-        if dy is None:
-            return None, None, None, None, None, None, None, None, None
-        x, w = ctx.saved_tensors
-        dy = dy.contiguous()
-        if dy.dtype != x.dtype:
-            dy = dy.to(x.dtype)
-        nhwc = ctx.nhwc or ctx.via_nhwc           # layout of the saved x and of the kernels
-        if ctx.via_nhwc:
-            dy = ops.nchw_to_nhwc(dy)
-        dx = dw = db = None
-        if nhwc:
-            H, W = x.shape[1], x.shape[2]
-        else:
-            H, W = x.shape[2], x.shape[3]
-        if ctx.needs_input_grad[0]:
-            dx = ops.dgrad(dy, w, ctx.plan, H, W, ctx.stride, nhwc, ctx.add_identity,
-                           pre=x if ctx.gelu_input else None)
-            if ctx.via_nhwc:
-                dx = ops.nhwc_to_nchw(dx)
-        need_db = ctx.has_bias and ctx.needs_input_grad[3]
-        if ctx.needs_input_grad[1] or need_db:
-            # bias shares the weight's dtype in an nn.Conv2d
-            dw, db = ops.wgrad(dy, x, ctx.plan, ctx.stride, nhwc, with_bias=need_db, gelu_input=ctx.gelu_input,
-                               out_dtype=w.dtype)
-            dw = dw if ctx.needs_input_grad[1] else None
-        return dx, dw, None, db, None, None, None, None, None
 
 
 class DepthwiseOrientedConv1d(nn.Conv2d):
@@ -181,21 +127,15 @@ class DepthwiseOrientedConv1d(nn.Conv2d):
         gelu = self._gelu_in_kernel(x)
         if self.gelu_input and not gelu:
             x = torch.nn.functional.gelu(x)
-        if not torch.is_grad_enabled():      # inference: the kernel call alone
-            plan, stride = self._get_plan(), self.stride[0]
-            if not self.nhwc and not gelu and _via_nhwc(x, plan, stride):
-                return ops.nhwc_to_nchw(ops.fprop(ops.nchw_to_nhwc(x), self.weight, self.bias, plan, stride, True,
-                                                  self.add_identity))
-            return ops.fprop(x, self.weight, self.bias, plan, stride, self.nhwc, self.add_identity, gelu)
         plan, stride = self._get_plan(), self.stride[0]
-        if ops.dgrad is _native_dgrad and ops.wgrad is _native_wgrad and x.is_cuda:
-            # the same node in native code: Python on the backward thread costs 60 us a call
-            via = not self.nhwc and not gelu and _via_nhwc(x, plan, stride)
+        via = not self.nhwc and not gelu and _via_nhwc(x, plan, stride)
+        if torch.is_grad_enabled():          # the autograd node (reference: dwoconv1d.py:18-69) lives in native code
             return ops.ext.conv(x, self.weight, self.theta, self.bias, plan.host, plan.on(x.device), plan.C, plan.K, stride,
                                 self.nhwc, via, self.add_identity, gelu)
-        # gradients replaced by a caller (tracing, tests): the node that calls them by name
-        return _DepthwiseOrientedConv1d.apply(x, self.weight, self.theta, self.bias, plan, stride, self.nhwc,
-                                              self.add_identity, gelu)
+        if via:
+            return ops.nhwc_to_nchw(ops.fprop(ops.nchw_to_nhwc(x), self.weight, self.bias, plan, stride, True,
+                                              self.add_identity))
+        return ops.fprop(x, self.weight, self.bias, plan, stride, self.nhwc, self.add_identity, gelu)
 
     def forward_safe(self, x):
         """Any H x W; output extents ceil(H/stride) x ceil(W/stride) (dwoconv1d.py:154-187)."""

@@ -519,37 +519,39 @@ def test_nchw_module_takes_the_tiled_route(oracle):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
-def test_module_forward_and_backward_stay_on_fast_kernels(dtype):
+@pytest.mark.parametrize("mode,families", [("rr", ("tiled", "lines")), ("model", ("segments",))], ids=["rr", "model"])
+def test_module_forward_and_backward_stay_on_fast_kernels(mode, families, dtype):
     """Forward and backward of the nn.Module at a stage shape: every one of the three kernels
     must come from a fast family.  Backward runs on autograd's own worker thread, so the route
-    is recorded from inside a tensor hook on that thread."""
+    is read in a tensor hook on that thread, behind one gradient at a time; a pass through the
+    general kernels before each leaves no fast route there from an earlier call."""
+    import threading
     N, C, hw, K = 2, 96, 56, 31
     m = o1d.DepthwiseOrientedConv1d(C, C, K, groups=C, padding=K // 2, nhwc=True,
-                                    angle=[float(a) for a in angle_list("rr", C)]).to(DEV)
+                                    angle=[float(a) for a in angle_list(mode, C)]).to(DEV)
     x = torch.randn((N, hw, hw, C), device=DEV).to(dtype).requires_grad_(True)
-    seen = {}
-    orig_dgrad, orig_wgrad = o1d.ops.dgrad, o1d.ops.wgrad
+    dy = torch.randn_like(x)
+    seen, threads = [], set()
 
-    def dgrad(*a, **k):
-        out = orig_dgrad(*a, **k)
-        seen["dgrad"] = o1d.ops.last_route()
-        return out
+    def note(grad):
+        seen.append(o1d.ops.last_route())
+        threads.add(threading.get_ident())
 
-    def wgrad(*a, **k):
-        out = orig_wgrad(*a, **k)
-        seen["wgrad"] = o1d.ops.last_route()
-        return out
-
-    o1d.ops.dgrad, o1d.ops.wgrad = dgrad, wgrad
-    try:
-        y = m(x)
-        seen["fprop"] = o1d.ops.last_route()
-        y.backward(torch.randn_like(y))
-        torch.cuda.synchronize()
-    finally:
-        o1d.ops.dgrad, o1d.ops.wgrad = orig_dgrad, orig_wgrad
-    assert set(seen) == {"fprop", "dgrad", "wgrad"}
-    assert all(v in ("tiled", "lines") for v in seen.values()), seen
+    x.register_hook(note)
+    m.weight.register_hook(note)
+    for wanted in (x, m.weight):                  # the input gradient, then the weight gradient
+        for route in (1, 0):
+            try:
+                o1d.ops.set_route(route)
+                y = m(x)
+                seen.append(o1d.ops.last_route())
+                torch.autograd.grad(y, (wanted,), dy)
+            finally:
+                o1d.ops.set_route(0)
+    torch.cuda.synchronize()
+    assert len(seen) == 8 and threading.get_ident() not in threads, seen
+    assert all(seen[i] == "general" for i in (0, 1, 4, 5)), seen
+    assert all(seen[i] in families for i in (2, 3, 6, 7)), seen
     assert o1d.ops.device_status() == 0
 
 
