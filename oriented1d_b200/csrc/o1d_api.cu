@@ -346,6 +346,21 @@ int seg_maps(const SegConfig &cfg, const void *t, bool with_halo, SegMaps *maps,
     return O1D_OK;
 }
 
+// Order of a bf16 sum: that of the family (tiled or direct) which the layer would otherwise take.  Both orders
+// are as far from the 64-bit sums, and neither is the faster one throughout (forward, block angles, ascending
+// against tiled: 14x14x2048 batch 64 97 / 104 us, 40x40x256 batch 32 51 / 54, 28x28x1024 batch 64 148 / 140,
+// 56x56x96 batch 128 192 / 175).  What decides is that a trained bf16 network should not change with the kernel:
+// one order for all of them moves single elements of a ConvNeXt-1D++ gradient by up to twice the gradient's root
+// mean square (0.3 % in the 2-norm).  The family is asked for at a full batch, whatever the call's: an image's
+// result does not depend on the images beside it.
+int seg_order_bf16(const PlanHeader &ph, const void *plan_host, int H, int W, int C, int K, const DeviceInfo &d) {
+    const int N = 16;                            // the direct kernels' tiles hold at most 16 images
+    TiledConfig t;
+    DirectLaunchSet ls;
+    const bool tiled = tiled_configure(ph, plan_host, N, H, W, C, K, 1, O1D_NHWC, 2, d.smem_optin, d.sms, OP_FPROP, &t) && t.util >= kWeakTiled;
+    return tiled && !direct_first(ph, plan_host, N, H, W, C, K, 1, O1D_NHWC, 2, d, &ls) ? SEG_TILED : SEG_ASCENDING;
+}
+
 // Forward / stride-1 input gradient through the segment kernels (canonical lines shared by neighbouring
 // channels).  w and bias are bf16 when `wbf16` is set, fp32 otherwise.
 int try_seg(const void *x, const void *w, const void *bias, int wbf16, const PlanHeader &ph, const void *plan_host,
@@ -355,16 +370,9 @@ int try_seg(const void *x, const void *w, const void *bias, int wbf16, const Pla
     SegConfig *cfg = seg_config(ph, plan_host, N, H, W, C, K, stride, layout, esize, d, false);
     if (!cfg) return kNotTiled;
     if (((uintptr_t)y & 15) != 0) return kNotTiled;
-    // bf16 results have the bits of the family that the shape would otherwise take; fp32 ones the fastest order
-    int order = SEG_TILED;
+    int order = SEG_TILED;                       // fp32: the same order everywhere
     if (esize == 2) {
-        if (cfg->order == SEG_UNSET) {
-            TiledConfig t;
-            DirectLaunchSet ls;
-            const bool tiled = tiled_configure(ph, plan_host, N, H, W, C, K, stride, layout, esize, d.smem_optin, d.sms, OP_FPROP, &t) &&
-                               t.util >= kWeakTiled;
-            cfg->order = tiled && !direct_first(ph, plan_host, N, H, W, C, K, stride, layout, esize, d, &ls) ? SEG_TILED : SEG_ASCENDING;
-        }
+        if (cfg->order == SEG_UNSET) cfg->order = seg_order_bf16(ph, plan_host, H, W, C, K, d);
         order = cfg->order;
     }
     SegMaps maps;

@@ -94,11 +94,13 @@ def test_nchw_module_of_odd_channel_groups():
         assert float(((a - b).abs() / b.abs().clamp_min(1e-2 * float(b.abs().max()))).max()) <= 2 ** -7
 
 
-# bf16 sums have the bits of a family that the shape would otherwise take (2: tiled, 3: direct)
-@pytest.mark.parametrize("shape", [(2, 56, 56, 96, 31), (8, 28, 28, 96, 31), (64, 28, 28, 96, 31), (3, 28, 28, 192, 31), (33, 14, 14, 384, 31), (1, 13, 29, 32, 15)],
-                         ids=lambda s: "x".join(map(str, s)))
-def test_bits_of_the_family_replaced(shape):
+# bf16 sums have the bits of the family that the shape would otherwise take (2: tiled, 3: direct)
+@pytest.mark.parametrize("shape,family", [((2, 56, 56, 96, 31), 2), ((8, 28, 28, 96, 31), 2), ((64, 28, 28, 96, 31), 2), ((3, 28, 28, 192, 31), 3),
+                                          ((33, 14, 14, 384, 31), 3), ((5, 24, 24, 192, 31), 2), ((1, 13, 29, 32, 15), 3)],
+                         ids=lambda s: "x".join(map(str, s)) if isinstance(s, tuple) else str(s))
+def test_bits_of_the_family_replaced(shape, family):
     N, H, W, C, K = shape
+    torch.manual_seed(H * C)
     x = torch.randn((N, H, W, C), device=DEV).to(torch.bfloat16)
     w, bias = 0.1 * torch.randn((C, 1, 1, K), device=DEV), torch.randn((C,), device=DEV)
     plan = _plan("model", C, K)
@@ -110,5 +112,25 @@ def test_bits_of_the_family_replaced(shape):
         finally:
             o1d.ops.set_route(0)
 
-    got = run(0)
-    assert any(all(torch.equal(a, b) for a, b in zip(got, run(route))) for route in (2, 3))
+    got, other = run(0), run(5 - family)
+    assert all(torch.equal(a, b) for a, b in zip(got, run(family)))
+    # the other order shows: a few sums in a hundred thousand round to the other side
+    assert H * W < 400 or not all(torch.equal(a, b) for a, b in zip(got, other))
+
+
+# maps of which the direct kernels' tile holds two images, but not of a batch of one
+@pytest.mark.parametrize("H,W,C,K,mode", [(8, 8, 1536, 31, "one1"), (14, 14, 1536, 15, "one1"), (16, 16, 768, 15, "one2"), (14, 14, 64, 7, "model")])
+def test_an_image_does_not_depend_on_its_batch(H, W, C, K, mode):
+    torch.manual_seed(H * C)
+    x = torch.randn((33, H, W, C), device=DEV).to(torch.bfloat16)
+    w, bias = 0.1 * torch.randn((C, 1, 1, K), device=DEV), torch.randn((C,), device=DEV)
+    plan = _plan(mode, C, K)
+
+    def run(t):
+        out = o1d.fprop(t, w, bias, plan, 1, True, True), o1d.dgrad(t, w, plan, H, W, 1, True)
+        assert o1d.ops.last_route() == "segments"
+        return out
+
+    whole = run(x)
+    for i in (0, 7, 32):
+        assert all(torch.equal(a[i:i + 1], b) for a, b in zip(whole, run(x[i:i + 1].contiguous())))
