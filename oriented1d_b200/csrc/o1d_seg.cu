@@ -33,8 +33,6 @@ Chunk chunk_of(const int8_t *chan, int c0, int c1, int K) {
     return k;
 }
 
-// Cycles of one task on a scheduler with three warps (measured at 56x56x96, batch 128).
-constexpr double kAxis28 = 3600, kAxis14 = 1950, kSlantTask = 4600, kDiagTask = 2050;
 constexpr double kPieceCycles = 2.4;         // TMA, per pixel of a tile
 
 double compute_cycles(const Chunk &k, int imgs, int lenh, int lenw, int LT) {
@@ -46,8 +44,7 @@ double compute_cycles(const Chunk &k, int imgs, int lenh, int lenw, int LT) {
         const int plen = fr == seg::FR_H ? lenw : lenh, llen = fr == seg::FR_H ? lenh : lenw;
         const int lines = kind == KIND_AXIS ? llen : kind == KIND_DIAG ? lenw + seg::kTD - 1 : ceil_div(llen, seg::kSR);
         const int bl = kind == KIND_SLANT ? seg::kST : kind == KIND_AXIS ? LT : seg::kTD;
-        const double cyc = kind == KIND_SLANT ? kSlantTask : kind == KIND_DIAG ? kDiagTask : LT == 28 ? kAxis28 : kAxis14;
-        sum += split * (double)ceil_div(imgs * lines, lpg) * ceil_div(plen, bl) * cyc;
+        sum += split * (double)ceil_div(imgs * lines, lpg) * ceil_div(plen, bl) * seg::task_cycles(kind, LT);
     }
     return sum / 4;                          // schedulers
 }

@@ -11,13 +11,15 @@
 // The line is a stride (pixel, row, or row +- pixel), so the eight orientations are three bodies.
 // Weights sit in registers, one pair of floats per tap.
 //
-// Bound: the FMA pipe.  A packed FMA occupies it for two issue slots, which leaves every other slot for
-// the loads, the bf16 -> fp32 widening and the address arithmetic (1.5-2 instructions per input).
-// That is why the kernels take arbitrary positions inside the tile without special cases: inputs past
-// the end of a line are clamped onto a pixel of zeros (TMA fills coordinates outside the tensor), which
-// costs nothing while the pipe is busy; whole left / right halves of a line's halo are skipped at the
-// borders of the map.  One CTA of twelve warps per SM; the tile after next is loaded while the warps,
-// each at its own pace, walk through the tasks of the current one.
+// Bound: neither memory nor the FMA pipe, but waits that three warps a scheduler do not cover.  56x56x96 bf16, batch 128: issue
+// slots 44 % busy while an SM is active, half of them packed FMAs (which hold the pipe for two slots each); the
+// largest stalls of a warp are instruction fetch (1.3 cycles an issue: the warps of a CTA run the bodies of
+// different line kinds, 10-14 KB of straight code each), fixed latency (1.3) and the busy FMA pipe (0.8); 28 % of
+// the SM cycles wait for the slowest CTA.  Useful operations are 19-22 % of the fp32 rate.
+// Inputs take arbitrary positions inside the tile without special cases: those past the end of a line are
+// clamped onto a pixel of zeros (TMA fills coordinates outside the tensor); whole left / right halves of a
+// line's halo are skipped at the borders of the map.  One CTA of twelve warps per SM; the tile after next is
+// loaded while the warps, each at its own pace, walk through the tasks of the current one.
 //
 // Lanes are ordered pair first, so that the lanes of a load cover whole 32-byte pixels of neighbouring
 // lines (an odd pixel pitch keeps those in different banks) and the lanes of a store whole sectors.
@@ -137,11 +139,12 @@ template <> struct Pair<__nv_bfloat16> {
     }
 };
 
-// Order of a sum: taps ascending, one FMA each on top of the bias, as in the general and the direct kernels,
-// so that a layer's result has the same bits whichever family computes it (a bf16 network amplifies
-// differences of the last bit to the size of its gradients' noise).  The tiled kernels add taps that fall on
-// one pixel first, and walk canonical lines 3 and 4 from the last tap to the first: MERGED does the same, for
-// shapes whose other family they are and wherever the order is free (21 FMAs instead of 31 on a diagonal).
+// Order of a sum: taps ascending, one FMA each on top of the bias, as in the general and the direct kernels.  The
+// tiled kernels add taps that fall on one pixel first, and walk canonical lines 3 and 4 from the last tap to the
+// first: MERGED does the same (21 FMAs instead of 31 on a diagonal).  bf16 outputs and input gradients take the
+// order, and so the bits, of the family that the layer would otherwise have (a bf16 network amplifies
+// differences of the last bit to the size of its gradients' noise); fp32 ones are MERGED always.  The weight
+// gradient has an order of its own: lanes, warps and CTAs, each in a fixed order.
 //
 // Frame of canonical line o: positions run along image columns (H), rows (V) or both (diagonals, from row to
 // row), in the direction in which the taps ascend: base tap m of the line is met m-th.  Lines whose tap k
@@ -406,6 +409,13 @@ __device__ __noinline__ void build_tables(Tables *tab, const SegParams &p, const
     __syncthreads();
 }
 
+// Cycles of one task on a scheduler with three warps, for the division of the work: chunks among CTAs on the host,
+// warps among classes here.  Measured in the forward kernel at 56x56x96, batch 128, one line kind at a time; they
+// know nothing of the instruction fetches of a CTA whose warps run several kinds.
+__host__ __device__ constexpr int task_cycles(int kind, int lt) {
+    return kind == KIND_SLANT ? 4600 : kind == KIND_DIAG ? 2050 : lt == 28 ? 3600 : 1950;
+}
+
 // Weight gradient: the warps are dealt to the classes in proportion to their tasks' cost, so that a warp
 // keeps its accumulators for all items of a segment.  One thread.
 __device__ __noinline__ void deal_warps(Tables *tab, int imgs, int lenh, int lenw, int lt) {
@@ -418,8 +428,7 @@ __device__ __noinline__ void deal_warps(Tables *tab, int imgs, int lenh, int len
         const int plen = fr == FR_H ? lenw : lenh, llen = fr == FR_H ? lenh : lenw;
         const int lines = kind == KIND_AXIS ? llen : kind == KIND_DIAG ? lenw + kTD - 1 : (llen + kSR - 1) / kSR;
         const int bl = kind == KIND_SLANT ? kST : kind == KIND_AXIS ? lt : kTD;
-        const float each = kind == KIND_SLANT ? 4.6f : kind == KIND_DIAG ? 2.05f : lt == 28 ? 3.6f : 1.95f;
-        cost[i] = each * ((imgs * lines + lpg - 1) / lpg) * ((plen + bl - 1) / bl);
+        cost[i] = (float)task_cycles(kind, lt) * ((imgs * lines + lpg - 1) / lpg) * ((plen + bl - 1) / bl);
         total += cost[i];
     }
 #pragma unroll 1

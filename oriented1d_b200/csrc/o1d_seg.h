@@ -8,7 +8,7 @@
 namespace o1d {
 
 constexpr int kSegGeos = 6, kSegRuns = 20;
-// Order of the sums (o1d_seg.cuh): taps ascending, or as in the tiled kernels (the faster one).
+// Order of the sums (o1d_seg.cuh): taps ascending, or as in the tiled kernels.
 enum : int { SEG_UNSET = 0, SEG_ASCENDING, SEG_TILED };
 
 // How the maps of a run of chunks are cut into items: G whole images, or one tile of an image.
