@@ -279,7 +279,7 @@ inline long tiled_window_wavefronts(const int8_t *ids, const TiledParams &p, int
 // pitches most warps straddle two line groups whose origins collide (28x28: 2.0 to 2.6
 // wavefronts per window load).  Shared memory has room at these sizes, so the line pitches are
 // searched for the fewest window-load wavefronts on a few sample chunks (28x28x192: 107 -> 97 us).
-// The result is cached per problem geometry; the search costs about 0.2 ms once.
+// The result is cached per problem geometry; the search costs 0.2 to 4 ms once.
 inline bool tiled_configure(const PlanHeader &ph, const void *plan_host, int N, int H, int W, int C, int K,
                             int stride, int layout, int esize, int smem_limit, int sms, int op, TiledConfig *out) {
     TiledConfig base;
@@ -298,8 +298,9 @@ inline bool tiled_configure(const PlanHeader &ph, const void *plan_host, int N, 
     for (int i = 0; i < ns; i++)
         for (int j = 0; j < CC; j++) sig = (sig ^ (uint8_t)chan[sample[i] * CC + j]) * 1099511628211ull;
     struct Entry { int H, W, CC, BR, NT, esize, op; uint64_t sig; int pn, pt; };
-    static Entry cache[64];
-    static int cached = 0;
+    constexpr int kKept = 256;
+    static Entry cache[kKept];
+    static int cached = 0, oldest = 0;               // a full cache gives up its entries in turn
     static std::mutex mu;
     int pn = 0, pt = 0;
     {
@@ -327,7 +328,9 @@ inline bool tiled_configure(const PlanHeader &ph, const void *plan_host, int N, 
             }
         if (!pn) { pn = base.p.pitch_n; pt = base.p.pitch_t; }
         std::lock_guard<std::mutex> lock(mu);
-        if (cached < 64) cache[cached++] = Entry{H, W, CC, base.p.BR, base.threads, esize, op, sig, pn, pt};
+        const Entry e{H, W, CC, base.p.BR, base.threads, esize, op, sig, pn, pt};
+        if (cached < kKept) cache[cached++] = e;
+        else { cache[oldest] = e; oldest = (oldest + 1) % kKept; }
     }
     if (pn == base.p.pitch_n && pt == base.p.pitch_t) return true;
     TiledConfig tuned;

@@ -287,6 +287,25 @@ def test_nchw_layers_know_every_fast_family(H, W, C, mode, dtype, fast):
     assert not o1d.ops.uses_tiled(plan, 4, H, W, 1, False, dtype)
 
 
+def test_pitch_search_is_kept_for_recent_maps():
+    """The tiled kernels' pitch search takes milliseconds; its result is kept however many geometries a
+    process has seen before."""
+    import time
+
+    def seconds(H, W, C, K, dtype):
+        plan = o1d.Plan(angle_list("model", C), K)
+        t = time.perf_counter()
+        assert o1d.ops.uses_tiled(plan, 2, H, W, 1, True, dtype)
+        return time.perf_counter() - t
+
+    maps = [(7 * a, 7 * b) for a in range(1, 8) for b in range(1, 8) if a % 8 and b % 8]
+    seen = [(h, w, c, 7, dt) for c in (32, 64, 96) for dt in (torch.float32, torch.bfloat16) for h, w in maps]
+    assert len(seen) > 256
+    first = [seconds(*s) for s in seen]
+    again = [seconds(*s) for s in seen[-40:]]
+    assert sorted(again)[20] < 0.2 * sorted(first[-40:])[20], (sorted(first[-40:])[20], sorted(again)[20])
+
+
 def test_last_route_starts_unset():
     import threading
     out = []
