@@ -328,9 +328,33 @@ SegConfig *seg_config(const PlanHeader &ph, const void *plan_host, int N, int H,
     SegConfig *cfg = nullptr;
     return seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, wgrad, &cfg) ? cfg : nullptr;
 }
-// Maps that the automatic route leaves to other families: 7x7 fills half of a segment (7x7x4096, batch 64: 92 us
-// against 35 us for the plane kernels).
-bool seg_route(int H, int W) { return g_prefer == 6 || (g_prefer == 0 && !(H == 7 && W == 7)); }
+// Do the segment kernels come before the other families?  Measured (us, K = 31, batch 128 unless said, forward /
+// weight gradient, segment kernels against the next family with bf16 parameters converted for it):
+//   Maps that fill half of their blocks or less, no:
+//   7x7x768 bf16    46 / 65   plane 23 / 29          8x9x768 bf16   52 / 69   direct 65 / 67
+//   5x5x768 bf16    42 / 58   direct 34 / 36         9x9x768 bf16   56 / 73   direct 85 / 91
+//   6x6x3072 (64)   81 / 116  direct 71 / 77         8x8x3072 (64)  79 / 103  direct 87 / 93
+//   7x8x768 bf16    46 / 65   direct 44 / 46         8x8x768 fp32   42 / 54   direct 44 / 46
+//   (a forward call on few bf16 channel planes does not earn back the conversion: 4x6x6x768 16, direct 19)
+//   Patchy layers (N channels in a row on a line) that fill the tiled kernels' threads, no, once those have eight
+//   items of eight channels for every SM:
+//   56x56x192 (2) bf16  572 / 550   tiled 337 / 437     28x28x192 (2) bf16  155 / 159   tiled 116 / 140
+//   56x56x192 (4) fp32  515 / 468   tiled 382 / 474     14x14x192 (4) bf16   62 / 69    tiled  50 / 65
+//   56x56x40 (5), 512   453 / 324   tiled 289 / 328     56x56x56 (7), 512   513 / 423   tiled 397 / 456
+//   56x56x56 (7), 128   130 / 128   tiled 126 / 159     56x56x32 (4), 1      24 / 36    tiled  32 / 44
+//   56x56x48 (6)         93 / 124   tiled 112 / 140     28x28x56 (7), 512   153 / 130   tiled 213 / 224 (half filled)
+bool seg_first(SegConfig &cfg, const PlanHeader &ph, const void *plan_host, int N, int H, int W, int C, int K, const DeviceInfo &d, bool wgrad) {
+    if (g_prefer != 0) return g_prefer == 6;
+    if (wgrad ? H <= 8 && W <= 8 : H <= 7 && W <= 7 && (H * W == 49 || cfg.esize == 4 || (int64_t)N * C >= 32768)) return false;
+    if (cfg.rank == SEG_UNSET) {
+        TiledConfig t;
+        const bool behind = cfg.patchy && (int64_t)N * C >= 64 * d.sms &&
+                            tiled_configure(ph, plan_host, N, H, W, C, K, 1, O1D_NHWC, cfg.esize, d.smem_optin, d.sms,
+                                            wgrad ? OP_WGRAD : OP_FPROP, &t) && t.util >= kWeakTiled;
+        cfg.rank = behind ? SEG_LAST : SEG_FIRST;
+    }
+    return cfg.rank == SEG_FIRST;
+}
 
 // Tensor maps of `t` for every way the configuration cuts it: the tiles with their halo, or the outputs alone.
 int seg_maps(const SegConfig &cfg, const void *t, bool with_halo, SegMaps *maps, const char *what) {
@@ -365,10 +389,10 @@ int seg_order_bf16(const PlanHeader &ph, const void *plan_host, int H, int W, in
 // channels).  w and bias are bf16 when `wbf16` is set, fp32 otherwise.
 int try_seg(const void *x, const void *w, const void *bias, int wbf16, const PlanHeader &ph, const void *plan_host,
             const void *plan_dev, void *y, int N, int H, int W, int C, int K, int stride, int layout, int dtype,
-            int add_identity, int flip, cudaStream_t st, const DeviceInfo &d) {
+            int add_identity, int flip, cudaStream_t st, const DeviceInfo &d, bool first) {
     const int esize = dtype == O1D_F32 ? 4 : 2;
     SegConfig *cfg = seg_config(ph, plan_host, N, H, W, C, K, stride, layout, esize, d, false);
-    if (!cfg) return kNotTiled;
+    if (!cfg || (first && !seg_first(*cfg, ph, plan_host, N, H, W, C, K, d, false))) return kNotTiled;
     if (((uintptr_t)y & 15) != 0) return kNotTiled;
     int order = SEG_TILED;                       // fp32: the same order everywhere
     if (esize == 2) {
@@ -442,13 +466,14 @@ int try_walk(const void *x, const float *w, const float *bias, const PlanHeader 
 }
 
 // Route of a forward-type call (flip = 1: stride-1 input gradient):
-//   1. segment kernels (NHWC, stride 1, neighbouring channels mostly on one canonical line; not 7x7),
+//   1. segment kernels (NHWC, stride 1, neighbouring channels mostly on one canonical line) where they are first,
 //   2. plane kernels (7x7, canonical lines),
 //   3. walker and whole-line kernels, for the fp32 stage maps where they are the faster ones,
 //   4. direct kernels when one tile holds several whole images, or where the tiled ones would idle,
 //   5. tiled kernels (canonical lines, stride 1, sizes in multiples of 7/8),
 //   6. direct kernels with row/column tiles (stems, large maps, arbitrary angles),
-//   7. general kernels (the caller falls through on kNotTiled).
+//   7. segment kernels where they are not first,
+//   8. general kernels (the caller falls through on kNotTiled).
 int route_forward(const void *x, const float *w, const float *bias, int wbf16, const PlanHeader &ph, const void *plan_host,
                   const void *plan_dev, void *y, int N, int H, int W, int C, int K, int stride, int layout,
                   int dtype, int add_identity, int flip, int act, const void *pre, cudaStream_t st,
@@ -458,9 +483,9 @@ int route_forward(const void *x, const float *w, const float *bias, int wbf16, c
     if (act || pre)       // activation on load / its derivative on store: tiled kernels, else general
         return try_tiled(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity,
                          flip, act, pre, st, d);
-    if (seg_route(H, W)) {     // neighbouring channels on one canonical line: packed-FMA segments
+    if (g_prefer == 0 || g_prefer == 6) {     // neighbouring channels on one canonical line: packed-FMA segments
         rc = try_seg(x, w, bias, wbf16, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip,
-                     st, d);
+                     st, d, /*first=*/true);
         if (rc != kNotTiled) return rc;
     }
     if (g_prefer == 0) {       // 7x7 maps on canonical lines: a channel plane per thread
@@ -496,8 +521,10 @@ int route_forward(const void *x, const float *w, const float *bias, int wbf16, c
     rc = try_tiled(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip,
                    0, nullptr, st, d);
     if (rc != kNotTiled) return rc;
-    return try_direct(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity,
-                      flip, st, d, false);
+    rc = try_direct(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity,
+                    flip, st, d, false);
+    if (rc != kNotTiled || g_prefer != 0) return rc;
+    return try_seg(x, w, bias, 0, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip, st, d, false);
 }
 
 // Weight gradient through the tiled kernels.  `cfg_only`: just report the workspace size.
@@ -594,9 +621,9 @@ int try_direct_wgrad(const void *dy, const void *x, const PlanHeader &ph, const 
 // Weight gradient through the segment kernels; dw and db bf16 when `out_bf16` is set.
 int try_seg_wgrad(const void *dy, const void *x, const PlanHeader &ph, const void *plan_host, const void *plan_dev, void *dw,
                   void *db, int out_bf16, void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K,
-                  int stride, int layout, int dtype, cudaStream_t st, const DeviceInfo &d) {
+                  int stride, int layout, int dtype, cudaStream_t st, const DeviceInfo &d, bool first) {
     SegConfig *cfg = seg_config(ph, plan_host, N, H, W, C, K, stride, layout, dtype == O1D_F32 ? 4 : 2, d, true);
-    if (!cfg) return kNotTiled;
+    if (!cfg || (first && !seg_first(*cfg, ph, plan_host, N, H, W, C, K, d, true))) return kNotTiled;
     if (((uintptr_t)dy & 15) != 0 || ((uintptr_t)workspace & 15) != 0) return kNotTiled;
     if (workspace_bytes < seg_wgrad_bytes(*cfg)) return O1D_ERR_WORKSPACE;
     SegMaps maps, dy_maps;
@@ -683,7 +710,7 @@ int o1d_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int
     const ChunkRange all{0, C / (32 / esize), ph.max_dh, ph.max_dw};
     if (direct_configure(ph, plan_host, all, N, H, W, C, K, stride, layout, esize, 232448, 148, false, false, &dcfg)) return 1;
     // what those two refuse the segment kernels may take: channels that do not fill groups of 32 bytes
-    return seg_route(H, W) && seg_config(ph, plan_host, N, H, W, C, K, stride, layout, esize, {148, 232448}, false) != nullptr;
+    return seg_config(ph, plan_host, N, H, W, C, K, stride, layout, esize, {148, 232448}, false) != nullptr;
 }
 
 int o1d_gelu_uses_tiled(const void *plan_host, int N, int H, int W, int C, int K, int dtype) {
@@ -887,9 +914,9 @@ int wgrad_dispatch(const void *dy, const void *x, const PlanHeader &ph, const vo
                    float *dw, float *db, void *workspace, size_t workspace_bytes, int N, int H, int W, int C, int K,
                    int stride, int layout, int dtype, int act, int out_bf16, cudaStream_t st, const DeviceInfo &d) {
     int rc;
-    if (!act && seg_route(H, W)) {
+    if (!act && (g_prefer == 0 || g_prefer == 6)) {           // see route_forward
         rc = try_seg_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, out_bf16, workspace, workspace_bytes, N, H, W, C, K, stride,
-                           layout, dtype, st, d);
+                           layout, dtype, st, d, /*first=*/true);
         if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
     }
     if (g_prefer == 0 && !act) {       // 7x7 maps on canonical lines: a channel plane per thread
@@ -925,6 +952,11 @@ int wgrad_dispatch(const void *dy, const void *x, const PlanHeader &ph, const vo
     if (!direct_first && !act) {
         rc = try_direct_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, workspace, workspace_bytes, N, H, W, C, K,
                               stride, layout, dtype, st, d, nullptr);
+        if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
+    }
+    if (!act && g_prefer == 0) {
+        rc = try_seg_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, 0, workspace, workspace_bytes, N, H, W, C, K, stride, layout,
+                           dtype, st, d, /*first=*/false);
         if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
     }
     const int P = ceil_div(H, stride), Q = ceil_div(W, stride);

@@ -140,9 +140,15 @@ bool plan_chunks(const int8_t *chan, SegParams &p, int px, int esize, int LT, in
 
 bool make_config(const int8_t *chan, int N, int H, int W, int C, int K, int esize, int smem_optin, int sms, bool wgrad, SegConfig *cfg) {
     if (C % 8 != 0 || K > kMaxTaps) return false;
-    // pairs of channels on different lines are computed twice and stored by halves
-    int mixed = 0;
-    for (int c = 0; c + 1 < C; c += 2) mixed += chan[c] != chan[c + 1];
+    // Pairs of channels on different lines are computed twice and stored by halves: at most one pair in four.
+    // Patchy layers (one pair in eight, or less than six channels in a row on a line) are taken, but behind the
+    // tiled kernels where those are at their best: each line of a chunk is a body of its own.
+    int mixed = 0, lines = 1;
+    for (int c = 0; c + 1 < C; c++) {
+        if (chan[c] == chan[c + 1]) continue;
+        lines++;
+        if (c % 2 == 0) mixed++;
+    }
     if (mixed * 8 > C) return false;
     const int tail = round_up((int)sizeof(seg::Tables), 16) + 12 * seg::kMaxBuf + 128;
     const int room = smem_optin - round_up(seg::kPadBytes, 128) - tail;
@@ -166,6 +172,7 @@ bool make_config(const int8_t *chan, int N, int H, int W, int C, int K, int esiz
     p.off_tile = round_up(seg::kPadBytes, 128);
     p.off_tab = p.off_tile + bytes;
     p.off_bar = p.off_tab + round_up((int)sizeof(seg::Tables), 16);
+    cfg->patchy = lines * 6 > C || mixed * 16 > C;
     cfg->esize = esize;
     cfg->short_reach = K <= 15;
     cfg->smem_bytes = p.off_bar + 12 * seg::kMaxBuf;

@@ -9,7 +9,7 @@ namespace o1d {
 
 constexpr int kSegGeos = 6, kSegRuns = 20;
 // Order of the sums (o1d_seg.cuh): taps ascending, or as in the tiled kernels.
-enum : int { SEG_UNSET = 0, SEG_ASCENDING, SEG_TILED };
+enum : int { SEG_UNSET = 0, SEG_ASCENDING, SEG_TILED, SEG_FIRST, SEG_LAST };
 
 // How the maps of a run of chunks are cut into items: G whole images, or one tile of an image.
 struct SegGeo {
@@ -44,7 +44,9 @@ struct SegMaps { CUtensorMap m[kSegGeos]; };
 struct SegConfig {
     SegParams p;
     int esize, short_reach, line_block, smem_bytes, grid, ngeos;
+    bool patchy;                         // lines change often from channel to channel (see make_config)
     int order;                           // order of the sums, for the caller to keep here: SEG_UNSET at first
+    int rank;                            // place among the kernel families, likewise: SEG_UNSET, SEG_FIRST, SEG_LAST
 };
 
 // Do the segment kernels take this request (NHWC, stride 1, canonical lines)?  `chan`: canonical line of

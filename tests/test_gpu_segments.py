@@ -35,7 +35,31 @@ SHAPES += [(2, 30, 61, 2048, 31, "model"), (3, 28, 100, 1536, 31, "model")]
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
 def test_segments_equal_general(shape, dtype):
-    N, H, W, C, K, mode = shape
+    got = check_against_general(*shape, dtype, route=6)
+    assert got == ("segments", "segments")
+
+
+# where the segment kernels come first, where behind another family, and where before the general kernels only
+# (forward, weight gradient)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("shape,families", [
+    ((3, 9, 9, 64, 31, "model"), ("segments", "segments")), ((3, 8, 9, 64, 31, "model"), ("segments", "segments")),
+    ((3, 8, 8, 128, 31, "model"), ("segments", "direct")), ((1, 7, 8, 128, 31, "model"), ("segments", "direct")),
+    ((513, 6, 6, 64, 31, "model"), ("direct", "direct")), ((256, 5, 5, 128, 15, "model"), ("direct", "direct")),
+    ((511, 6, 6, 64, 31, "model"), ("direct/segments", "direct")),           # fp32 / bf16
+    ((1024, 1, 1, 32, 31, "one2"), ("direct", "direct")), ((3, 7, 7, 64, 31, "model"), ("plane7", "plane7")),
+    ((600, 6, 6, 72, 31, "model"), ("direct/segments", "direct/segments")),  # channels that the bf16 direct kernels refuse
+    ((296, 56, 56, 32, 31, "model"), ("tiled", "tiled")), ((295, 56, 56, 32, 31, "model"), ("segments", "segments")),
+    ((170, 56, 56, 56, 31, "model"), ("tiled", "tiled")), ((200, 56, 56, 48, 31, "model"), ("segments", "segments")),
+    ((240, 28, 28, 40, 31, "model"), ("segments", "segments")), ((300, 40, 60, 32, 31, "model"), ("segments", "segments")),
+], ids=lambda s: "x".join(map(str, s)) if isinstance(s, tuple) and len(s) == 6 else "")
+def test_place_among_the_families(shape, families, dtype):
+    got = check_against_general(*shape, dtype, route=0)
+    assert got == tuple(f.split("/")[-1 if dtype == torch.bfloat16 else 0] for f in families)
+
+
+def check_against_general(N, H, W, C, K, mode, dtype, route):
+    """Forward, input gradient and weight gradient of both; the families that served forward and weight gradient."""
     g = torch.Generator(device=DEV).manual_seed(H * W + C)
     x = torch.randn((N, H, W, C), generator=g, device=DEV).to(dtype)
     dy = torch.randn((N, H, W, C), generator=g, device=DEV).to(dtype)
@@ -46,15 +70,18 @@ def test_segments_equal_general(shape, dtype):
     def run(route):
         try:
             o1d.ops.set_route(route)
-            out = (o1d.fprop(x, w, bias, plan, 1, True, True), o1d.dgrad(dy, w, plan, H, W, 1, True))
-            name = o1d.ops.last_route()
-            return out + o1d.wgrad(dy, x, plan, 1, True, True), name
+            out = (o1d.fprop(x, w, bias, plan, 1, True, True),)
+            names = o1d.ops.last_route()
+            out += (o1d.dgrad(dy, w, plan, H, W, 1, True),)
+            assert o1d.ops.last_route() == names
+            out += o1d.wgrad(dy, x, plan, 1, True, True)
+            return out, (names, o1d.ops.last_route())
         finally:
             o1d.ops.set_route(0)
 
     ref, _ = run(1)
-    got, name = run(0)
-    assert name == "segments" and o1d.ops.device_status() == 0
+    got, names = run(route)
+    assert o1d.ops.device_status() == 0
     for a, b in zip(got[:2], ref[:2]):
         a, b = a.float(), b.float()
         if dtype == torch.float32:
@@ -63,8 +90,9 @@ def test_segments_equal_general(shape, dtype):
             assert float(((a - b).abs() / b.abs().clamp_min(1e-2)).max()) <= 2 ** -7
     for a, b in zip(got[2:], ref[2:]):
         assert float((a - b).abs().max()) <= 1e-4 * float(b.abs().max())
-    again = run(0)[0]
+    again = run(route)[0]
     assert all(torch.equal(a, b) for a, b in zip(got, again))        # same bits again
+    return names
 
 
 def test_nchw_module_of_odd_channel_groups():
