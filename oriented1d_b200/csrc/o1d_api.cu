@@ -328,6 +328,13 @@ SegConfig *seg_config(const PlanHeader &ph, const void *plan_host, int N, int H,
     SegConfig *cfg = nullptr;
     return seg_configure(chan_host, N, H, W, C, K, esize, d.smem_optin, d.sms, wgrad, &cfg) ? cfg : nullptr;
 }
+// Would the tiled kernels take this layer with a segment for most of their threads?  (No search of pitches, which
+// takes milliseconds and changes neither answer; the batch does not either.)
+bool tiled_strong(const PlanHeader &ph, const void *plan_host, int H, int W, int C, int K, int esize, const DeviceInfo &d, int op) {
+    TiledConfig t;
+    return tiled_configure_pitch(ph, plan_host, 1, H, W, C, K, 1, O1D_NHWC, esize, d.smem_optin, d.sms, op, 0, 0, &t) && t.util >= kWeakTiled;
+}
+
 // Do the segment kernels come before the other families?  Measured (us, K = 31, batch 128 unless said, forward /
 // weight gradient, segment kernels against the next family with bf16 parameters converted for it):
 //   Maps that fill half of their blocks or less, no:
@@ -347,10 +354,8 @@ bool seg_first(SegConfig &cfg, const PlanHeader &ph, const void *plan_host, int 
     if (g_prefer != 0) return g_prefer == 6;
     if (wgrad ? H <= 8 && W <= 8 : H <= 7 && W <= 7 && (H * W == 49 || cfg.esize == 4 || (int64_t)N * C >= 32768)) return false;
     if (cfg.rank == SEG_UNSET) {
-        TiledConfig t;
         const bool behind = cfg.patchy && (int64_t)N * C >= 64 * d.sms &&
-                            tiled_configure(ph, plan_host, N, H, W, C, K, 1, O1D_NHWC, cfg.esize, d.smem_optin, d.sms,
-                                            wgrad ? OP_WGRAD : OP_FPROP, &t) && t.util >= kWeakTiled;
+                            tiled_strong(ph, plan_host, H, W, C, K, cfg.esize, d, wgrad ? OP_WGRAD : OP_FPROP);
         cfg.rank = behind ? SEG_LAST : SEG_FIRST;
     }
     return cfg.rank == SEG_FIRST;
@@ -379,10 +384,8 @@ int seg_maps(const SegConfig &cfg, const void *t, bool with_halo, SegMaps *maps,
 // result does not depend on the images beside it.
 int seg_order_bf16(const PlanHeader &ph, const void *plan_host, int H, int W, int C, int K, const DeviceInfo &d) {
     const int N = 16;                            // the direct kernels' tiles hold at most 16 images
-    TiledConfig t;
     DirectLaunchSet ls;
-    const bool tiled = tiled_configure(ph, plan_host, N, H, W, C, K, 1, O1D_NHWC, 2, d.smem_optin, d.sms, OP_FPROP, &t) && t.util >= kWeakTiled;
-    return tiled && !direct_first(ph, plan_host, N, H, W, C, K, 1, O1D_NHWC, 2, d, &ls) ? SEG_TILED : SEG_ASCENDING;
+    return tiled_strong(ph, plan_host, H, W, C, K, 2, d, OP_FPROP) && !direct_first(ph, plan_host, N, H, W, C, K, 1, O1D_NHWC, 2, d, &ls) ? SEG_TILED : SEG_ASCENDING;
 }
 
 // Forward / stride-1 input gradient through the segment kernels (canonical lines shared by neighbouring

@@ -206,35 +206,55 @@ bool make_config(const int8_t *chan, int N, int H, int W, int C, int K, int esiz
     return cfg->smem_bytes <= smem_optin;
 }
 
-// Configurations of the last requests of this thread (they depend on the shape and the lines only).
+// Configurations of the last requests of this thread (they depend on the shape and the lines only).  A
+// classifier has about 20 per image size, so that a loader of two dozen sizes finds its own again; an entry
+// takes 1 KB and a byte per channel.
+struct Key {
+    int N, H, W, C, K, esize, smem, sms, wgrad;
+    bool operator==(const Key &o) const { return memcmp(this, &o, sizeof(Key)) == 0; }
+};
 struct Entry {
-    int N, H, W, C, K, esize, smem, sms;
-    bool wgrad, taken;
+    Key key;
+    bool taken;
     std::vector<int8_t> chan;
     SegConfig cfg;
 };
-constexpr size_t kKept = 64;
+constexpr size_t kKept = 512;
+uint64_t hash_of(const Key &k) {                 // FNV-1a
+    const int v[] = {k.N, k.H, k.W, k.C, k.K, k.esize, k.smem, k.sms, k.wgrad};
+    uint64_t h = 1469598103934665603ull;
+    for (int x : v) h = (h ^ (uint32_t)x) * 1099511628211ull;
+    return h;
+}
 
 }  // namespace
 
 bool seg_configure(const int8_t *chan, int N, int H, int W, int C, int K, int esize, int smem_optin, int sms, bool wgrad,
                    SegConfig **cfg) {
     thread_local std::vector<std::unique_ptr<Entry>> kept;
+    thread_local std::vector<uint64_t> hashes;   // of the entries, side by side
     thread_local size_t oldest = 0;
-    for (const auto &e : kept)
-        if (e->N == N && e->H == H && e->W == W && e->C == C && e->K == K && e->esize == esize && e->smem == smem_optin && e->sms == sms &&
-            e->wgrad == wgrad && memcmp(e->chan.data(), chan, C) == 0) {
-            *cfg = &e->cfg;
-            return e->taken;
+    const Key key{N, H, W, C, K, esize, smem_optin, sms, wgrad};
+    const uint64_t hash = hash_of(key);
+    for (size_t i = 0; i < hashes.size(); i++)
+        if (hashes[i] == hash && kept[i]->key == key && memcmp(kept[i]->chan.data(), chan, C) == 0) {
+            *cfg = &kept[i]->cfg;
+            return kept[i]->taken;
         }
     auto e = std::make_unique<Entry>();
-    e->N = N; e->H = H; e->W = W; e->C = C; e->K = K; e->esize = esize; e->smem = smem_optin; e->sms = sms; e->wgrad = wgrad;
+    e->key = key;
     e->chan.assign(chan, chan + C);
     e->taken = make_config(chan, N, H, W, C, K, esize, smem_optin, sms, wgrad, &e->cfg);
     *cfg = &e->cfg;
     const bool taken = e->taken;
-    if (kept.size() < kKept) kept.push_back(std::move(e));
-    else { kept[oldest] = std::move(e); oldest = (oldest + 1) % kKept; }
+    if (kept.size() < kKept) {
+        kept.push_back(std::move(e));
+        hashes.push_back(hash);
+    } else {                                     // a full cache gives up its entries in turn
+        kept[oldest] = std::move(e);
+        hashes[oldest] = hash;
+        oldest = (oldest + 1) % kKept;
+    }
     return taken;
 }
 

@@ -306,6 +306,22 @@ def test_pitch_search_is_kept_for_recent_maps():
     assert sorted(again)[20] < 0.2 * sorted(first[-40:])[20], (sorted(first[-40:])[20], sorted(again)[20])
 
 
+def test_segment_geometry_is_kept_for_recent_shapes():
+    """Cutting the maps for the segment kernels takes a hundred microseconds; a loader of a few dozen image
+    sizes finds the shapes of its layers again."""
+    import time
+    plan = o1d.Plan(angle_list("model", 40), 31)             # channels that only the segment kernels take
+
+    def seconds(H, W):
+        t = time.perf_counter()
+        assert o1d.ops.uses_tiled(plan, 2, H, W, 1, True, torch.bfloat16)
+        return time.perf_counter() - t
+
+    shapes = [(20 + a, 30 + b) for a in range(20) for b in range(20)]
+    first, again = [seconds(*s) for s in shapes], [seconds(*s) for s in shapes]
+    assert sorted(again)[200] < 0.4 * sorted(first)[200], (sorted(first)[200], sorted(again)[200])
+
+
 def test_last_route_starts_unset():
     import threading
     out = []
