@@ -51,8 +51,7 @@ inline void bind_primary_context() {
 
 // 4-D tiled tensor map, dims/box innermost first, strides in bytes for dims 1..3.
 inline int encode_map4(CUtensorMap *map, const void *base, int esize, const cuuint64_t (&dims)[4],
-                       const cuuint64_t (&strides)[3], const cuuint32_t (&box)[4],
-                       CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
+                       const cuuint64_t (&strides)[3], const cuuint32_t (&box)[4]) {
     if ((uintptr_t)base & 15) return MAP_NA;
     for (int i = 0; i < 4; i++)
         if (box[i] == 0 || box[i] > 256 || dims[i] == 0 || dims[i] > 0xffffffffull) return MAP_NA;
@@ -68,7 +67,7 @@ inline int encode_map4(CUtensorMap *map, const void *base, int esize, const cuui
     for (int attempt = 0; attempt < 2; attempt++) {
         r = enc(map, esize == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
                 const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r == CUDA_SUCCESS) return MAP_OK;
         bind_primary_context();
     }
