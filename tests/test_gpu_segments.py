@@ -95,6 +95,43 @@ def check_against_general(N, H, W, C, K, mode, dtype, route):
     return names
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("shape", [(5, 13, 15, 64, 31, "model"), (2, 29, 27, 40, 15, "model+"), (1, 56, 57, 96, 31, "model"),
+                                   (2, 30, 61, 2048, 31, "model")], ids=lambda s: "x".join(map(str, s)))
+def test_parameters_read_and_written_as_bf16(shape, dtype):
+    """bf16 weights and biases go to the kernels as they are stored: the bits of a call with the same values in
+    fp32, and gradients that are its fp32 ones rounded."""
+    from oriented1d_b200 import _lib
+    N, H, W, C, K, mode = shape
+    g = torch.Generator(device=DEV).manual_seed(C)
+    x, dy = (torch.randn((N, H, W, C), generator=g, device=DEV).to(dtype) for _ in range(2))
+    w = (0.1 * torch.randn((C, 1, 1, K), generator=g, device=DEV)).to(torch.bfloat16)
+    bias = torch.randn((C,), generator=g, device=DEV).to(torch.bfloat16)
+    plan = _plan(mode, C, K)
+    want = (o1d.fprop(x, w.float(), bias.float(), plan, 1, True, True), o1d.dgrad(dy, w.float(), plan, H, W, 1, True))
+    want += tuple(t.to(torch.bfloat16) for t in o1d.wgrad(dy, x, plan, 1, True, True))
+    # through the C ABI, which does not convert: these requests are served as they are
+    y, dx = torch.empty_like(x), torch.empty_like(x)
+    dw, db = torch.empty_like(w), torch.empty_like(bias)
+    host, dev = plan.pointers(x)
+    code, flag, st = (_lib.F32 if dtype == torch.float32 else _lib.BF16), 4, torch.cuda.current_stream().cuda_stream
+    size = _lib.lib.o1d_wgrad_workspace_bytes(N, H, W, C, K, 1, _lib.NHWC, code)
+    ws = torch.empty(size, dtype=torch.uint8, device=DEV)
+    sizes = (N, H, W, C, K, 1, _lib.NHWC, code)
+    calls = (lambda: _lib.lib.o1d_fprop(x.data_ptr(), w.data_ptr(), bias.data_ptr(), host, dev, y.data_ptr(), *sizes, _lib.FLAG_IDENTITY | flag, st),
+             lambda: _lib.lib.o1d_dgrad(dy.data_ptr(), w.data_ptr(), host, dev, dx.data_ptr(), *sizes, flag, st),
+             lambda: _lib.lib.o1d_wgrad_act(dy.data_ptr(), x.data_ptr(), host, dev, dw.data_ptr(), db.data_ptr(), ws.data_ptr(), size, *sizes, flag, st))
+    for call in calls:
+        _lib.check(call(), "segments with bf16 parameters")
+        assert o1d.ops.last_route() == "segments"
+    assert o1d.ops.device_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip((y, dx, dw, db), want))
+    # and through the wrappers
+    got = (o1d.fprop(x, w, bias, plan, 1, True, True), o1d.dgrad(dy, w, plan, H, W, 1, True))
+    got += o1d.wgrad(dy, x, plan, 1, True, True, out_dtype=torch.bfloat16)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def test_nchw_module_of_odd_channel_groups():
     """An NCHW bf16 layer whose channels do not fill groups of 32 bytes: the segment kernels behind two
     layout steps, with the results of the general NCHW kernels."""
