@@ -50,8 +50,10 @@ enum { O1D_NCHW = 0, O1D_NHWC = 1 };
 enum {
     O1D_FLAG_IDENTITY = 1,    /* w' = w + (k == pad): the reference's `resid`                     */
     O1D_FLAG_GELU_INPUT = 2,  /* the input tensor is a pre-activation: exact GELU is applied as it is loaded */
-    O1D_FLAG_PARAMS_BF16 = 4  /* w and bias (o1d_wgrad_act: dw and db) are bf16, not fp32; requests whose kernels
+    O1D_FLAG_PARAMS_BF16 = 4, /* w and bias (o1d_wgrad_act: dw and db) are bf16, not fp32; requests whose kernels
                                  read fp32 parameters only are refused with O1D_ERR_UNSUPPORTED               */
+    O1D_FLAG_MAY_CONVERT = 8  /* with O1D_FLAG_PARAMS_BF16: refuse also where kernels that read fp32 parameters
+                                 are the faster ones, conversion included; the caller then converts           */
 };
 enum { O1D_F32 = 0, O1D_BF16 = 1 };
 

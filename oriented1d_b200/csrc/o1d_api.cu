@@ -54,6 +54,13 @@ int map_fail(const char *what) {
 
 constexpr int kNotTiled = -1;          // "this kernel family does not take the request"
 
+// How a call passes its parameters (or wants their gradients): as fp32, as bf16, or as bf16 by a caller that
+// converts them where kernels of fp32 parameters are the faster ones.
+enum : int { PARAMS_F32 = 0, PARAMS_BF16, BF16_OR_CONVERT };
+int params_of(int flags) {
+    return !(flags & O1D_FLAG_PARAMS_BF16) ? PARAMS_F32 : flags & O1D_FLAG_MAY_CONVERT ? BF16_OR_CONVERT : PARAMS_BF16;
+}
+
 struct DeviceInfo { int sms; int smem_optin; };
 
 // Attributes of the current device, queried once per device.
@@ -495,7 +502,12 @@ int route_forward(const void *x, const float *w, const float *bias, int wbf16, c
         rc = try_small7(x, w, bias, wbf16, ph, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip, st, d);
         if (rc != kNotTiled) return rc;
     }
-    if (wbf16) return O1D_ERR_UNSUPPORTED;       // the other families read fp32 parameters
+    if (wbf16) {                                 // the other families read fp32 parameters
+        rc = wbf16 == BF16_OR_CONVERT || g_prefer != 0 || (H == 7 && W == 7)
+                 ? kNotTiled
+                 : try_seg(x, w, bias, wbf16, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip, st, d, false);
+        return rc == kNotTiled ? O1D_ERR_UNSUPPORTED : rc;
+    }
     if (g_prefer == 0 || g_prefer == 5) {   // items computed in place in their NHWC layout
         rc = try_walk(x, w, bias, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, add_identity, flip,
                       st, d, /*faster_only=*/g_prefer == 0);
@@ -849,7 +861,7 @@ int o1d_fprop(const void *x, const float *w, const float *bias, const void *plan
     if ((rc = device_info(&d))) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     const int identity = add_identity & O1D_FLAG_IDENTITY, act = (add_identity & O1D_FLAG_GELU_INPUT) ? 1 : 0;
-    const int wbf16 = (add_identity & O1D_FLAG_PARAMS_BF16) ? 1 : 0;
+    const int wbf16 = params_of(add_identity);
     rc = route_forward(x, w, bias, wbf16, ph, plan_host, plan_dev, y, N, H, W, C, K, stride, layout, dtype, identity,
                        /*flip=*/0, act, nullptr, st, d);
     if (rc != kNotTiled) return rc;
@@ -877,7 +889,7 @@ int o1d_dgrad_act(const void *dy, const float *w, const void *pre, const void *p
     cudaStream_t st = (cudaStream_t)stream;
     // stride 1: dx = fprop(dy) with the taps mirrored, i.e. (the lines being odd-symmetric)
     // with the weights read in reverse order
-    const int wbf16 = (add_identity & O1D_FLAG_PARAMS_BF16) ? 1 : 0;
+    const int wbf16 = params_of(add_identity);
     add_identity &= O1D_FLAG_IDENTITY;
     if (wbf16 && stride != 1) return O1D_ERR_UNSUPPORTED;
     rc = stride == 1 ? route_forward(dy, w, nullptr, wbf16, ph, plan_host, plan_dev, dx, N, H, W, C, K, stride, layout,
@@ -927,7 +939,13 @@ int wgrad_dispatch(const void *dy, const void *x, const PlanHeader &ph, const vo
                               dtype, st, d);
         if (rc != kNotTiled && rc != O1D_ERR_WORKSPACE) return rc;
     }
-    if (out_bf16) return O1D_ERR_UNSUPPORTED;                 // the other families write fp32 gradients
+    if (out_bf16) {                                           // the other families write fp32 gradients
+        rc = act || out_bf16 == BF16_OR_CONVERT || g_prefer != 0 || (H == 7 && W == 7)
+                 ? kNotTiled
+                 : try_seg_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, out_bf16, workspace, workspace_bytes, N, H, W, C, K, stride,
+                                 layout, dtype, st, d, false);
+        return rc == kNotTiled || rc == O1D_ERR_WORKSPACE ? O1D_ERR_UNSUPPORTED : rc;
+    }
     if (act) {                 // x is GELU(pre), applied on load: tiled kernels, else general
         rc = try_tiled_wgrad(dy, x, ph, plan_host, plan_dev, dw, db, workspace, workspace_bytes, N, H, W, C, K, stride,
                              layout, dtype, act, st, d, nullptr);
@@ -995,7 +1013,7 @@ int o1d_wgrad_act(const void *dy, const void *x, const void *plan_host, const vo
     DeviceInfo d;
     if ((rc = device_info(&d))) return rc;
     return wgrad_dispatch(dy, x, ph, plan_host, plan_dev, dw, db, workspace, workspace_bytes, N, H, W, C, K, stride,
-                          layout, dtype, (flags & O1D_FLAG_GELU_INPUT) ? 1 : 0, (flags & O1D_FLAG_PARAMS_BF16) ? 1 : 0,
+                          layout, dtype, (flags & O1D_FLAG_GELU_INPUT) ? 1 : 0, params_of(flags),
                           (cudaStream_t)stream, d);
 }
 

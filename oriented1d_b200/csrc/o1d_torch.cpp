@@ -101,7 +101,7 @@ Tensor fprop(const Tensor &x_, const Tensor &w, const OptTensor &bias, int64_t p
     void *out = y.data_ptr(), *st = stream();
     call(p, "o1d_fprop", [&](int pf) {
         return o1d_fprop(ptr(x), (const float *)ptr(p.w), (const float *)ptr(p.b), (const void *)host, (const void *)dev, out, (int)d.n,
-                         (int)d.h, (int)d.w, (int)d.c, (int)K, (int)stride, nhwc, code, flags | pf, st);
+                         (int)d.h, (int)d.w, (int)d.c, (int)K, (int)stride, nhwc, code, flags | pf | O1D_FLAG_MAY_CONVERT, st);
     });
     return y;
 }
@@ -128,7 +128,7 @@ Tensor dgrad(const Tensor &dy_, const Tensor &w, int64_t plan_c, int64_t K, int6
     void *out = dx.data_ptr(), *st = stream();
     call(p, "o1d_dgrad", [&](int pf) {
         return o1d_dgrad_act(ptr(dy), (const float *)ptr(p.w), ptr(pre), (const void *)host, (const void *)dev, out, (int)d.n, (int)H,
-                             (int)W, (int)d.c, (int)K, (int)stride, nhwc, code, (identity ? O1D_FLAG_IDENTITY : 0) | pf, st);
+                             (int)W, (int)d.c, (int)K, (int)stride, nhwc, code, (identity ? O1D_FLAG_IDENTITY : 0) | pf | O1D_FLAG_MAY_CONVERT, st);
     });
     return dx;
 }
@@ -159,7 +159,7 @@ std::tuple<Tensor, OptTensor> wgrad(const Tensor &dy_, const Tensor &x_, int64_t
     auto run = [&](int flag) {
         return o1d_wgrad_act(ptr(dy), ptr(x), (const void *)host, (const void *)dev, (float *)dw.data_ptr(),
                              with_bias ? (float *)db.data_ptr() : nullptr, ws.data_ptr(), bytes, (int)d.n, (int)d.h, (int)d.w, (int)d.c,
-                             (int)K, (int)stride, nhwc, code, (gelu ? O1D_FLAG_GELU_INPUT : 0) | flag, st);
+                             (int)K, (int)stride, nhwc, code, (gelu ? O1D_FLAG_GELU_INPUT : 0) | flag | O1D_FLAG_MAY_CONVERT, st);
     };
     int rc = run(bf16 ? O1D_FLAG_PARAMS_BF16 : 0);
     if (rc == O1D_ERR_UNSUPPORTED && bf16) {             // kernels that write fp32 gradients only

@@ -132,6 +132,36 @@ def test_parameters_read_and_written_as_bf16(shape, dtype):
     assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
+@pytest.mark.parametrize("shape,served", [((600, 6, 6, 64, 31, "model"), True), ((3, 8, 8, 64, 31, "model"), True), ((296, 56, 56, 32, 31, "model"), True),
+                                          ((3, 7, 7, 72, 31, "model"), False), ((3, 6, 6, 64, 31, "random"), False)],
+                         ids=lambda s: "x".join(map(str, s)) if isinstance(s, tuple) else "")
+def test_bf16_parameters_where_another_family_comes_first(shape, served):
+    """A caller that cannot convert its parameters is served wherever the segment kernels take the layer; one
+    that can is told where to."""
+    from oriented1d_b200 import _lib
+    N, H, W, C, K, mode = shape
+    torch.manual_seed(C)
+    x, dy = (torch.randn((N, H, W, C), device=DEV).to(torch.bfloat16) for _ in range(2))
+    w = (0.1 * torch.randn((C, 1, 1, K), device=DEV)).to(torch.bfloat16)
+    plan = _plan(mode, C, K)
+    host, dev = plan.pointers(x)
+    sizes, st = (N, H, W, C, K, 1, _lib.NHWC, _lib.BF16), torch.cuda.current_stream().cuda_stream
+    size = _lib.lib.o1d_wgrad_workspace_bytes(*sizes)
+    ws = torch.empty(size, dtype=torch.uint8, device=DEV)
+    y, dw = torch.empty_like(x), torch.empty_like(w)
+
+    def wgrad(flags):
+        return _lib.lib.o1d_wgrad_act(dy.data_ptr(), x.data_ptr(), host, dev, dw.data_ptr(), None, ws.data_ptr(), size, *sizes, flags, st)
+
+    rc = _lib.lib.o1d_fprop(x.data_ptr(), w.data_ptr(), None, host, dev, y.data_ptr(), *sizes, 4, st), wgrad(4)
+    assert rc == ((0, 0) if served else (2, 2)) and wgrad(4 | 8) == 2
+    if served:
+        assert float((y.float() - o1d.fprop(x, w, None, plan, 1, True).float()).abs().max()) <= 2 ** -7 * float(y.float().abs().max())
+        a, b = dw.float(), o1d.wgrad(dy, x, plan, 1, True)[0]
+        assert float((a - b).abs().max()) <= 2 ** -8 * float(b.abs().max())
+        assert o1d.ops.device_status() == 0
+
+
 def test_nchw_module_of_odd_channel_groups():
     """An NCHW bf16 layer whose channels do not fill groups of 32 bytes: the segment kernels behind two
     layout steps, with the results of the general NCHW kernels."""
